@@ -1565,9 +1565,10 @@ extern "C" int l2j_sampler_seed(l2j_ctx *c, int64_t seed)
     if (!c->finalized || !c->is_last)
         return fail(c, L2J_E_STATE, "the sampler belongs to the finalized context that holds the classifier");
     const int n = c->cfg.vocab_size;
-    if (n < 2 || sample_smem_bytes(n) > 220 * 1024)
+    const int n_max = sample_max_vocab(220 * 1024);
+    if (n < 2 || n > n_max)
         return fail(c, L2J_E_INVALID, "the device sampler keeps the probabilities in shared memory: vocabulary of 2..%d tokens",
-                    (int)((220 * 1024 - 65536) / 4));
+                    n_max);
     CK(c, cudaSetDevice(c->device));
     if (!c->samp_state) {
         int rc = dev_alloc(c, &c->samp_state, 1, true);

@@ -286,6 +286,7 @@ void prefill_destroy(Prefill *pf);
 struct SamplerState {
     unsigned long long rng;   // java.util.Random's 48-bit state
     int token;                // the id chosen by the last launch
+    int cur;                  // which of prob[2] / index[2] holds the ProbIndex array
 };
 
 struct SampleParams {
@@ -293,11 +294,12 @@ struct SampleParams {
     int n;
     float temperature, topp;
     SamplerState *st;
-    float *prob[2];           // the Sampler's ProbIndex array (persistent across calls), and the sort's second buffer
+    float *prob[2];           // the Sampler's ProbIndex array (persistent across calls, always sorted), and the next call's
     int *index[2];
 };
 
 size_t sample_smem_bytes(int n);
+int sample_max_vocab(size_t smem_limit);   // largest vocabulary the sampler takes
 cudaError_t prepare_sampler(int n);
 cudaError_t launch_sample(cudaStream_t stream, const SampleParams &sp);
 

@@ -74,6 +74,24 @@ def test_changing_candidate_counts(model, oracle):
     assert got == want
 
 
+@pytest.mark.parametrize("vocab,scale", [(2, 0.02), (9, 1.0), (300, 0.5), (4097, 0.05), (8193, 0.02), (40960, 0.3)])
+def test_vocabulary_sizes(oracle, vocab, scale):
+    """Shares of the cluster's blocks that are empty, ragged or full, flat and peaked distributions, and equal
+    probabilities (pairs of equal classifier rows) in both the candidates and what earlier calls left behind them."""
+    cfg = ModelConfig(64, 176, 1, 4, 4, vocab, 64, False)
+    tensors = syn.synthetic_tensors(cfg, 11)
+    wcls = np.random.default_rng(5).standard_normal((vocab, 64), dtype=np.float32) * np.float32(scale)
+    wcls[1::2] = wcls[0::2][: wcls[1::2].shape[0]]
+    tensors[L.T_WCLS] = wcls.reshape(-1)
+    m = Transformer(cfg, 0, 0, None, 0)
+    m.upload_all(tensors)
+    m.finalize()
+    temps, tops = (0.9, 0.2, 3.0, 1.0), (0.9, 0.5, 0.99, 1.0, 0.7)
+    got, want = _run(m, oracle, vocab, lambda s: (temps[s % 4], tops[s % 5]), steps=40)
+    m.close()
+    assert got == want
+
+
 def test_probabilities_replace_logits(model, oracle):
     """The reference turns the logits into probabilities in place; so does the device (Run.java:645-656)."""
     model.sampler_seed(1)
