@@ -152,7 +152,7 @@ L2J_API int l2j_forward_stage(l2j_ctx *ctx, int token, int pos, const float *x_i
  * that move them with their own device-to-device transport. */
 /* Batched prompt processing (no counterpart in the reference, whose run loop pushes every prompt token through
  * the decode step, Run.java:623-637): positions pos0 .. pos0 + n - 1 with the input tokens given (tokens[i] is
- * the token fed at position pos0 + i, i.e. BOS and then the prompt, Run.java:614,635-637), 64 positions per
+ * the token fed at position pos0 + i, i.e. BOS and then the prompt, Run.java:614,635-637), up to 256 positions per
  * sweep over the weights, dot products on the tensor cores (u8 weights x s8 limbs of the 24-bit fixed-point
  * activations, exact integer sums, group (min, scale) applied in FP32 as in the decode kernels).  Leaves the K/V
  * cache as the decode steps would leave it to FP32 rounding of the row sums (prompt positions are not bitwise

@@ -249,7 +249,7 @@ inline int choose_nsplit(int sm_count, int n_heads, int seq_len)
 }
 
 // ---- batched prompt processing on the tensor cores (l2j_prefill.cu) ---------------------------------------------
-constexpr int kPrefillTokens = 64;   // positions that share one sweep over the weights
+constexpr int kPrefillTokens = 64;   // tokens of one block of the tensor-core operand; entries of one concurrent step
 enum PrefillWeight { PF_WQ = 0, PF_WK, PF_WV, PF_WO, PF_W1, PF_W3, PF_W2, PF_W_COUNT };
 
 struct PrefillLayerDesc {

@@ -1,5 +1,5 @@
-// Batched prompt processing: the positions of a prompt go through every layer 64 at a time, so a weight byte
-// is read from HBM once per 64 tokens instead of once per token, and the dot products run on the tensor cores.
+// Batched prompt processing: the positions of a prompt go through every layer up to 256 at a time, so a weight byte
+// is read from HBM once per 256 tokens instead of once per token, and the dot products run on the tensor cores.
 //
 // The reference has no such path: its run loop pushes every prompt token through the decode step
 // (Run.java:623-637).  What is computed per position is the decode step's arithmetic (Run.java:418-508): the
@@ -10,8 +10,8 @@
 //
 // Kernels:
 //   pf_embed_kernel     rows of the embedding table for the chunk's tokens
-//   pf_limbs_kernel     activations -> limbs [3 x 64 rows][K] (the B operand) + per (group, token) unit and sum;
-//                       input is RMSNorm(x) * w, the attention output, or SwiGLU(h1, h3)
+//   pf_limbs_kernel     activations -> limbs [3 x 64 rows][K] (the B operand) per block of 64 tokens + per (group,
+//                       token) unit and sum; input is RMSNorm(x) * w, the attention output, or SwiGLU(h1, h3)
 //   pf_gemm_kernel      C[64 tokens][rows] (+)= W[rows][K] x limbs: TMA (cp.async.bulk.tensor) feeds 128-byte-
 //                       swizzled tiles to tcgen05.mma kind::i8 (u8 x s8 -> s32, M 128, N 192, K 32), one
 //                       accumulator per quantisation group in tensor memory, double-buffered; four epilogue warps
@@ -38,7 +38,11 @@ namespace l2j {
 
 namespace {
 
-constexpr int kT = kPrefillTokens;          // tokens per chunk
+constexpr int kT = kPrefillTokens;          // tokens per block of the B operand
+constexpr int kTB = 4;                      // token blocks per chunk of a prompt.  A matrix launch costs about 9 us beside its
+                                            // tiles (set-up, first copies, drain) and there are nine launches per layer and
+                                            // chunk: with four blocks instead of one, 3840 tokens through 16 layers of the
+                                            // 7B shape take 144 instead of 214 ms
 constexpr int kN = 3 * kT;                  // columns of the B operand: three limbs per token
 constexpr int kTileM = 128;                 // weight rows per tile
 constexpr int kGemmThreads = 384;          // producer warp, issue warp, two spare, eight epilogue warps
@@ -52,7 +56,7 @@ constexpr int kABytes = kTileM * 128;       // the A part of a stage: 128 rows o
 constexpr int kBBytes = kN * 128;
 constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kMaxParts = 12;               // parts a row sum (or a query's keys) may be dealt into
-constexpr int kWideParts = 3;               // at most this many parts for the wide outputs (QKV, W1/W3): their sums are read back
+constexpr int kWideParts = 3;               // at most this many parts for the wide outputs (W1/W3): their sums are read back
 constexpr int kAccCols = 256;               // column distance of the two accumulators in tensor memory
 constexpr int kTmemCols = 512;
 
@@ -186,13 +190,14 @@ struct PfGemmParams {
     PfGemmSeg seg[3];
     int nseg;
     int groups;          // K / 256
-    const float2 *ux;    // [groups][64]: (value of one unit of the integer sums, sum of the fixed-point activations)
-    const float *ssq;    // [nssq][64] partial sums of squares of the input rows (RMSNorm in front), or nullptr
+    int tblocks;         // blocks of 64 tokens; the grid is a multiple of it, so a block's items are of one token block
+    const float2 *ux;    // [tblocks][groups][64]: (value of one unit of the integer sums, sum of the fixed-point activations)
+    const float *ssq;    // [tblocks][nssq][64] partial sums of squares of the input rows (RMSNorm in front), or nullptr
     int nssq;
     int n;               // elements per input row
-    float *out;          // [ksplit][64][ldc]
+    float *out;          // [ksplit][64 * tblocks][ldc]
     int ldc;
-    int ksplit;          // the groups of a row are dealt to this many blocks; part z goes to out + z * 64 * ldc
+    int ksplit;          // the groups of a row are dealt to this many blocks; part z goes to out + z * 64 * tblocks * ldc
     int nvalid;          // tokens of the chunk that exist
     int timeout_us;
     unsigned int *status;
@@ -220,8 +225,10 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
     int ntiles = 0;
     for (int s = 0; s < p.nseg; ++s)
         ntiles += p.seg[s].rows / kTileM;
-    ntiles *= p.ksplit;                       // work items: (tile, part of the groups)
+    ntiles *= p.ksplit;                       // work items of this token block: (tile, part of the groups)
     const int G = p.groups;
+    // blocks next to each other work on the same weights for different tokens: L2 serves all but the first
+    const int tb = (int)blockIdx.x % p.tblocks, first = (int)blockIdx.x / p.tblocks, stride = (int)gridDim.x / p.tblocks;
     const int gper = (G + p.ksplit - 1) / p.ksplit;
 
     if (tid == 0) {
@@ -247,7 +254,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         if (p.ssq != nullptr) {
             float tot = 0.f;
             for (int y = 0; y < p.nssq; ++y)
-                tot += p.ssq[y * kT + tid];
+                tot += p.ssq[(tb * p.nssq + y) * kT + tid];
             tot = __fdiv_rn(tot, (float)p.n);
             tot = __fadd_rn(tot, 1e-5f);
             ss = __fdiv_rn(1.0f, __fsqrt_rn(tot));
@@ -256,7 +263,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
     }
     __syncthreads();
     for (int i = tid; i < G * kT; i += kGemmThreads) {
-        const float2 u = p.ux[i];
+        const float2 u = p.ux[(size_t)tb * G * kT + i];
         s_ux[i] = make_float2(u.x * s_ss[i & (kT - 1)], u.y);
     }
     tc_fence_before();
@@ -270,7 +277,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         if (lane == 0) {
             const uint64_t pol = policy_evict_first();
             long it = 0;
-            for (int tile = blockIdx.x; tile < ntiles && !*give_up; tile += gridDim.x) {
+            for (int tile = first; tile < ntiles && !*give_up; tile += stride) {
                 int sg = 0, m0 = (tile / p.ksplit) * kTileM;
                 while (m0 >= p.seg[sg].rows) {
                     m0 -= p.seg[sg].rows;
@@ -286,7 +293,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
                     const uint32_t st = base + (uint32_t)s * kStageBytes;
                     mbar_arrive_expect_tx(bar_full + 8 * s, kStageBytes);
                     tma_load_2d_hint(st, ma, hs * 128, m0, bar_full + 8 * s, pol);
-                    tma_load_2d(st + kABytes, &map_b, hs * 128, 0, bar_full + 8 * s);
+                    tma_load_2d(st + kABytes, &map_b, hs * 128, tb * kN, bar_full + 8 * s);
                 }
             }
             if (*give_up) {
@@ -304,7 +311,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         if (lane == 0) {
             long it = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+            for (int tile = first; tile < ntiles && ok; tile += stride) {
                 const int g0 = (tile % p.ksplit) * gper, g1 = min(G, g0 + gper);
                 for (int g = g0; g < g1 && ok; ++g, ++it) {
                     const int b = (int)(it & 1);
@@ -347,7 +354,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(th * kTH);
         long it = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        for (int tile = first; tile < ntiles && ok; tile += stride) {
             int sg = 0, m0 = (tile / p.ksplit) * kTileM;
             while (m0 >= p.seg[sg].rows) {
                 m0 -= p.seg[sg].rows;
@@ -411,11 +418,12 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
                     msq[j] = nxt[j];
             }
             if (ok) {
-                float *o = p.out + (size_t)z * kT * p.ldc + p.seg[sg].col0 + row;
+                const int t0 = tb * kT + th * kTH;
+                float *o = p.out + ((size_t)z * kT * p.tblocks + t0) * p.ldc + p.seg[sg].col0 + row;
 #pragma unroll
                 for (int t = 0; t < kTH; ++t)
-                    if (th * kTH + t < p.nvalid)
-                        o[(size_t)(th * kTH + t) * p.ldc] = acc[t];
+                    if (t0 + t < p.nvalid)
+                        o[(size_t)t * p.ldc] = acc[t];
             }
         }
     }
@@ -435,18 +443,18 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
 enum { PF_IN_NORM = 0, PF_IN_ATTN = 1, PF_IN_SWIGLU = 2 };
 
 struct PfLimbParams {
-    float *a;              // [64][lda]: x (NORM, updated with the parts), h1 (SWIGLU); ATTN: unused
-    const float *b;        // NORM: RMSNorm weights [n]; SWIGLU: h3 [64][lda]
-    const float *parts;    // NORM: [nparts][64][lda] partial row sums of the matrix in front, added to x in this order;
-                           // ATTN: [nparts][64][heads][head + 2] partial attention outputs (o, m, l) of the key ranges
+    float *a;              // [tokens][lda]: x (NORM, updated with the parts), h1 (SWIGLU); ATTN: unused
+    const float *b;        // NORM: RMSNorm weights [n]; SWIGLU: h3 [tokens][lda]
+    const float *parts;    // NORM: [nparts][tokens][lda] partial row sums of the matrix in front, added to x in this order;
+                           // ATTN: [nparts][tokens][heads][head + 2] partial attention outputs (o, m, l) of the key ranges
     int nparts;
     int head;              // ATTN: head size
     int lda;
     int n;                 // elements per token (multiple of 256)
     int nvalid;
-    int8_t *limbs;         // [3 * 64][n]
-    float2 *ux;            // [n / 256][64]: (value of one fixed-point unit, sum of the fixed-point activations)
-    float *ssq;            // NORM: [gridDim.y][64] partial sums of squares of the rows
+    int8_t *limbs;         // [token block][3 * 64][n]
+    float2 *ux;            // [token block][n / 256][64]: (value of one fixed-point unit, sum of the fixed-point activations)
+    float *ssq;            // NORM: [token block][gridDim.y][64] partial sums of squares of the rows
 };
 
 constexpr int kLimbWarps = 4, kLimbThreads = 32 * kLimbWarps;
@@ -458,6 +466,7 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
     // flight at once
     __shared__ float s_ssq[kLimbWarps];
     const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tpad = gridDim.x, tb = t / kT, tl = t % kT;     // tokens of the chunk, whole blocks
     const int G = p.n >> 8;
     const bool live = t < p.nvalid;
     float ssq = 0.f;
@@ -475,10 +484,10 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
                 const int hd = e / p.head, d = e - hd * p.head, heads = p.n / p.head, rec = p.head + 2;
                 float mx = -FLT_MAX;
                 for (int z = 0; z < p.nparts; ++z)
-                    mx = fmaxf(mx, p.parts[((size_t)(z * kT + t) * heads + hd) * rec + p.head]);
+                    mx = fmaxf(mx, p.parts[((size_t)(z * tpad + t) * heads + hd) * rec + p.head]);
                 float lsum = 0.f;
                 for (int z = 0; z < p.nparts; ++z) {
-                    const float *r = p.parts + ((size_t)(z * kT + t) * heads + hd) * rec;
+                    const float *r = p.parts + ((size_t)(z * tpad + t) * heads + hd) * rec;
                     const float w = expf(r[p.head] - mx);
                     lsum = fmaf(w, r[p.head + 1], lsum);
                     x.x = fmaf(w, r[d], x.x); x.y = fmaf(w, r[d + 1], x.y); x.z = fmaf(w, r[d + 2], x.z); x.w = fmaf(w, r[d + 3], x.w);
@@ -487,7 +496,7 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
             }
             if (MODE == PF_IN_NORM && live && p.nparts > 0) {
                 for (int z = 0; z < p.nparts; ++z) {
-                    const float4 d4 = *reinterpret_cast<const float4 *>(p.parts + ((size_t)z * kT + t) * p.lda + e);
+                    const float4 d4 = *reinterpret_cast<const float4 *>(p.parts + ((size_t)z * tpad + t) * p.lda + e);
                     x.x = __fadd_rn(x.x, d4.x); x.y = __fadd_rn(x.y, d4.y); x.z = __fadd_rn(x.z, d4.z); x.w = __fadd_rn(x.w, d4.w);
                 }
                 *reinterpret_cast<float4 *>(p.a + (size_t)t * p.lda + e) = x;   // the residual stream after the matrix in front
@@ -501,8 +510,8 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
                 if (live)
                     y = *reinterpret_cast<const float4 *>(p.b + (size_t)t * p.lda + e);
                 for (int z = 1; z < p.nparts && live; ++z) {   // split-K parts of h1 and h3, in order
-                    const float4 xz = *reinterpret_cast<const float4 *>(p.a + ((size_t)z * kT + t) * p.lda + e);
-                    const float4 yz = *reinterpret_cast<const float4 *>(p.b + ((size_t)z * kT + t) * p.lda + e);
+                    const float4 xz = *reinterpret_cast<const float4 *>(p.a + ((size_t)z * tpad + t) * p.lda + e);
+                    const float4 yz = *reinterpret_cast<const float4 *>(p.b + ((size_t)z * tpad + t) * p.lda + e);
                     x.x = __fadd_rn(x.x, xz.x); x.y = __fadd_rn(x.y, xz.y); x.z = __fadd_rn(x.z, xz.z); x.w = __fadd_rn(x.w, xz.w);
                     y.x = __fadd_rn(y.x, yz.x); y.y = __fadd_rn(y.y, yz.y); y.z = __fadd_rn(y.z, yz.z); y.w = __fadd_rn(y.w, yz.w);
                 }
@@ -538,9 +547,9 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
             const uint32_t t3 = __byte_perm(z[4 * h + 2], z[4 * h + 3], 0x0062);
             const uint32_t l0 = __byte_perm(t0, t2, 0x5410), l1 = __byte_perm(t0, t2, 0x7632), l2 = __byte_perm(t1, t3, 0x5410);
             const size_t e = (size_t)gi * 256 + h * 128 + lane * 4;
-            *reinterpret_cast<uint32_t *>(p.limbs + ((size_t)(0 * kT + t)) * p.n + e) = l0;
-            *reinterpret_cast<uint32_t *>(p.limbs + ((size_t)(1 * kT + t)) * p.n + e) = l1;
-            *reinterpret_cast<uint32_t *>(p.limbs + ((size_t)(2 * kT + t)) * p.n + e) = l2;
+            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)(tb * kN + 0 * kT + tl) * p.n + e) = l0;
+            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)(tb * kN + 1 * kT + tl) * p.n + e) = l1;
+            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)(tb * kN + 2 * kT + tl) * p.n + e) = l2;
             s0 = dp4a_ones(l0, s0);
             s1 = dp4a_ones(l1, s1);
             s2 = dp4a_ones(l2, s2);
@@ -551,7 +560,7 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
         if (lane == 0) {
             const float inv = __int_as_float((127 + ex - 22) << 23);   // value of one fixed-point unit
             const float xs = fmaf((float)s2, 65536.0f, fmaf((float)s1, 256.0f, (float)s0));
-            p.ux[(size_t)gi * kT + t] = live ? make_float2(inv, xs) : make_float2(0.f, 0.f);
+            p.ux[((size_t)tb * G + gi) * kT + tl] = live ? make_float2(inv, xs) : make_float2(0.f, 0.f);
         }
     }
     if (MODE == PF_IN_NORM) {
@@ -564,7 +573,7 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
             float tot = 0.f;
             for (int w = 0; w < kLimbWarps; ++w)
                 tot += s_ssq[w];
-            p.ssq[(size_t)blockIdx.y * kT + t] = tot;
+            p.ssq[((size_t)tb * gridDim.y + blockIdx.y) * kT + tl] = tot;
         }
     }
 }
@@ -585,12 +594,12 @@ __global__ void pf_embed_kernel(const int *tokens, int nvalid, const float *emb,
 }
 
 struct PfRopeParams {
-    const float *qkv;      // [64][dim + 2 kv_dim]
-    float *q;              // [64][dim]
+    const float *qkv;      // [tokens][dim + 2 kv_dim]
+    float *q;              // [tokens][dim]
     float *k_cache, *v_cache;   // layer base, [kv_head][seq][head]
     const float *rope_cos, *rope_sin;   // [seq][head / 2]
     int dim, kv_dim, head, seq_len, pos0, nvalid;
-    int nparts;                         // split-K parts of qkv ([nparts][64][dim + 2 kv_dim]), summed here in order
+    int nparts;                         // split-K parts of qkv ([nparts][tokens][dim + 2 kv_dim]), summed here in order
     const int *pos_of, *seq_of;         // concurrent sequences: position and sequence of every token (else pos0 + t, one cache)
     long long seq_stride;               // floats between the caches of two sequences
 };
@@ -612,7 +621,7 @@ __global__ void pf_rope_kv_kernel(PfRopeParams p)
         const int e = 2 * i;
         float v0 = row[e], v1 = row[e + 1];
         for (int z = 1; z < p.nparts; ++z) {
-            const float *rz = row + (size_t)z * kT * (p.dim + 2 * p.kv_dim);
+            const float *rz = row + (size_t)z * gridDim.x * (p.dim + 2 * p.kv_dim);
             v0 = __fadd_rn(v0, rz[e]);
             v1 = __fadd_rn(v1, rz[e + 1]);
         }
@@ -644,10 +653,11 @@ __global__ void pf_rope_kv_kernel(PfRopeParams p)
 // ---------------------------------------------------------------------------------------------------------------
 
 struct PfAttnParams {
-    const float *q;        // [64][dim] after RoPE
+    const float *q;        // [tokens][dim] after RoPE
     const float *k_cache, *v_cache;
-    float *parts;          // [nsplit][64][heads][head + 2]: unnormalised output, running maximum, sum of the key range
+    float *parts;          // [nsplit][tpad][heads][head + 2]: unnormalised output, running maximum, sum of the key range
     int dim, head, kv_mul, seq_len, pos0, nvalid, nsplit;
+    int tpad;              // tokens of the chunk, whole blocks of 64
 };
 
 constexpr int kAttnQ = 32;       // queries per block
@@ -812,7 +822,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) pf_attention_kernel(const PfA
     for (int i = 0; i < 4; ++i) {
         const int qi = q0 + qa + i;
         if (qi < p.nvalid) {
-            float *rec = p.parts + ((size_t)(z * kT + qi) * heads + h) * (HEAD + 2);
+            float *rec = p.parts + ((size_t)(z * p.tpad + qi) * heads + h) * (HEAD + 2);
 #pragma unroll
             for (int c = 0; c < NV4; ++c) {   // records are 8-byte aligned (HEAD + 2 floats each)
                 *reinterpret_cast<float2 *>(rec + c * 64 + kb * 4) = make_float2(o[i][c].x, o[i][c].y);
@@ -1109,11 +1119,10 @@ struct Prefill {
     CUtensorMap map_b_dim, map_b_hidden;
     int *tokens = nullptr;
     float *x = nullptr, *qkv = nullptr, *q = nullptr, *h13 = nullptr;
-    float *parts = nullptr;      // [kMaxParts][64][dim]: partial row sums of Wo / W2, or the attention's key ranges
-    int ksplit_o = 1, ksplit_2 = 1, ksplit_qkv = 1, ksplit_13 = 1;
+    float *parts = nullptr;      // [kMaxParts][kTB * 64][dim]: partial row sums of Wo / W2, or the attention's key ranges
     int8_t *limbs = nullptr;
     float2 *ux = nullptr;
-    float *ssq = nullptr;         // [groups / 4][64]
+    float *ssq = nullptr;         // [kTB][groups / 4][64]
     int token_cap = 0;
     size_t gemm_smem_dim = 0, gemm_smem_hidden = 0, attn_smem = 0;
     std::vector<void *> owned;
@@ -1178,14 +1187,14 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m)
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&pf->sms, cudaDevAttrMultiProcessorCount, dev);
     const int kmax = m.dim > m.hidden ? m.dim : m.hidden;
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->x, (size_t)kT * m.dim);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->qkv, (size_t)kWideParts * kT * pf->qkv_ld);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->q, (size_t)kT * m.dim);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->h13, (size_t)kWideParts * kT * 2 * m.hidden);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->parts, (size_t)kMaxParts * kT * (m.dim + 2 * m.n_heads));
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->limbs, (size_t)kN * kmax);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->ux, (size_t)(kmax / 256) * kT);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->ssq, (size_t)(kmax / 256) * kT);
+    if (e == cudaSuccess) e = pf_alloc(pf, &pf->x, (size_t)kTB * kT * m.dim);
+    if (e == cudaSuccess) e = pf_alloc(pf, &pf->qkv, (size_t)kTB * kT * pf->qkv_ld);
+    if (e == cudaSuccess) e = pf_alloc(pf, &pf->q, (size_t)kTB * kT * m.dim);
+    if (e == cudaSuccess) e = pf_alloc(pf, &pf->h13, (size_t)kWideParts * kTB * kT * 2 * m.hidden);
+    if (e == cudaSuccess) e = pf_alloc(pf, &pf->parts, (size_t)kMaxParts * kTB * kT * (m.dim + 2 * m.n_heads));
+    if (e == cudaSuccess) e = pf_alloc(pf, &pf->limbs, (size_t)kTB * kN * kmax);
+    if (e == cudaSuccess) e = pf_alloc(pf, &pf->ux, (size_t)kTB * (kmax / 256) * kT);
+    if (e == cudaSuccess) e = pf_alloc(pf, &pf->ssq, (size_t)kTB * (kmax / 256) * kT);
     if (e != cudaSuccess) {
         prefill_destroy(pf);
         return e;
@@ -1197,8 +1206,8 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m)
     for (int l = 0; l < m.n_layers && ok; ++l)
         for (int w = 0; w < PF_W_COUNT && ok; ++w)
             ok = encode_bytes_2d(&pf->maps[(size_t)l * PF_W_COUNT + w], m.layers[(size_t)l].w[w], rows[w], ks[w], kTileM, true);
-    ok = ok && encode_bytes_2d(&pf->map_b_dim, pf->limbs, kN, m.dim, kN, false) &&
-         encode_bytes_2d(&pf->map_b_hidden, pf->limbs, kN, m.hidden, kN, false);
+    ok = ok && encode_bytes_2d(&pf->map_b_dim, pf->limbs, kTB * kN, m.dim, kN, false) &&
+         encode_bytes_2d(&pf->map_b_hidden, pf->limbs, kTB * kN, m.hidden, kN, false);
     if (!ok) {
         prefill_destroy(pf);
         return cudaErrorNotSupported;
@@ -1210,29 +1219,6 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m)
     e = cudaFuncSetAttribute(pf_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gmax);
     const int ld = m.head + 4;
     pf->attn_smem = (size_t)(2 * kAttnKeys * ld + kAttnQ * ld + kAttnQ * kAttnKeys) * sizeof(float);
-    // matrices with few row tiles (Wo, W2: dim / 128) deal the groups of a row to several blocks
-    auto split_for = [&](int rows, int groups) {
-        int ks = 1;
-        while (ks < kMaxParts && (rows / kTileM) * ks * 2 <= pf->sms && groups / (ks * 2) >= 2)
-            ks *= 2;
-        return ks;
-    };
-    pf->ksplit_o = split_for(m.dim, m.dim / 256);
-    pf->ksplit_2 = split_for(m.dim, m.hidden / 256);
-    // the wide matrices have more tiles than SMs or nearly so: the part count that needs the fewest rounds of groups
-    auto rounds_split = [&](int tiles, int groups) {
-        int best = 1, best_cost = 1 << 30;
-        for (int ks = 1; ks <= kWideParts && ks <= groups; ++ks) {
-            const int cost = ((tiles * ks + pf->sms - 1) / pf->sms) * ((groups + ks - 1) / ks);
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = ks;
-            }
-        }
-        return best;
-    };
-    pf->ksplit_qkv = 1;   // measured: three parts for QKV (96 tiles at the 7B shape) gain nothing and cost the RoPE kernel two more reads
-    pf->ksplit_13 = rounds_split(2 * m.hidden / kTileM, m.dim / 256);
     if (e == cudaSuccess)
         e = m.head == 128 ? cudaFuncSetAttribute(pf_attention_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf->attn_smem)
                           : cudaFuncSetAttribute(pf_attention_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf->attn_smem);
@@ -1246,8 +1232,37 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m)
 
 namespace {
 
+// How the groups of a row are dealt to parts, for `tb` blocks of 64 tokens.
+struct Splits {
+    int o, w2, w13;
+};
+
+Splits splits_for(const Prefill *pf, int tb)
+{
+    const PrefillModel &m = pf->m;
+    // matrices with few row tiles (Wo, W2: dim / 128) deal the groups of a row to several blocks
+    auto few = [&](int groups) {
+        int ks = 1;
+        while (ks * 2 <= kMaxParts && (m.dim / kTileM) * tb * ks * 2 <= pf->sms && groups / (ks * 2) >= 2)
+            ks *= 2;
+        return ks;
+    };
+    // W1/W3 have more tiles than SMs or nearly so: the part count that needs the fewest rounds of groups
+    // (QKV stays whole: three parts for its 96 tiles at the 7B shape gain nothing and cost the RoPE kernel two more reads)
+    const int tiles = 2 * m.hidden / kTileM, groups = m.dim / 256, blocks = pf->sms / tb;
+    int best = 1, best_cost = 1 << 30;
+    for (int ks = 1; ks <= kWideParts && ks <= groups; ++ks) {
+        const int cost = ((tiles * ks + blocks - 1) / blocks) * ((groups + ks - 1) / ks);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = ks;
+        }
+    }
+    return Splits{few(m.dim / 256), few(m.hidden / 256), best};
+}
+
 cudaError_t launch_gemm(Prefill *pf, cudaStream_t st, int layer, const int *w, int nw, int k, float *out, int ldc, const int *col0,
-                        int ksplit, int nvalid, bool normed)
+                        int ksplit, int tb, int nvalid, bool normed)
 {
     const PrefillModel &m = pf->m;
     const int rows_of[PF_W_COUNT] = {m.dim, pf->kv_dim, pf->kv_dim, m.dim, m.hidden, m.hidden, m.dim};
@@ -1261,6 +1276,7 @@ cudaError_t launch_gemm(Prefill *pf, cudaStream_t st, int layer, const int *w, i
     }
     p.nseg = nw;
     p.groups = k / 256;
+    p.tblocks = tb;
     p.ux = pf->ux;
     p.out = out;
     p.ldc = ldc;
@@ -1275,14 +1291,15 @@ cudaError_t launch_gemm(Prefill *pf, cudaStream_t st, int layer, const int *w, i
     const CUtensorMap &a0 = base[w[0]], &a1 = base[w[nw > 1 ? 1 : 0]], &a2 = base[w[nw > 2 ? 2 : 0]];
     const CUtensorMap &b = k == m.dim ? pf->map_b_dim : pf->map_b_hidden;
     const size_t smem = k == m.dim ? pf->gemm_smem_dim : pf->gemm_smem_hidden;
-    const int grid = tiles * ksplit < pf->sms ? tiles * ksplit : pf->sms;
+    const int per_block = pf->sms / tb;      // thread blocks per block of tokens
+    const int grid = tb * (tiles * ksplit < per_block ? tiles * ksplit : per_block);
     pf_gemm_kernel<<<grid, kGemmThreads, smem, st>>>(a0, a1, a2, b, p);
     ++pf->launches;
     return cudaGetLastError();
 }
 
 template <int MODE>
-cudaError_t launch_limbs(Prefill *pf, cudaStream_t st, float *a, const float *b, const float *parts, int nparts, int lda, int n, int nvalid)
+cudaError_t launch_limbs(Prefill *pf, cudaStream_t st, float *a, const float *b, const float *parts, int nparts, int lda, int n, int tb, int nvalid)
 {
     PfLimbParams p{};
     p.a = a;
@@ -1296,7 +1313,7 @@ cudaError_t launch_limbs(Prefill *pf, cudaStream_t st, float *a, const float *b,
     p.limbs = pf->limbs;
     p.ux = pf->ux;
     p.ssq = pf->ssq;
-    const dim3 grid((unsigned)kT, (unsigned)((n / 256 + kLimbWarps - 1) / kLimbWarps));
+    const dim3 grid((unsigned)(tb * kT), (unsigned)((n / 256 + kLimbWarps - 1) / kLimbWarps));
     pf_limbs_kernel<MODE><<<grid, kLimbThreads, 0, st>>>(p);
     ++pf->launches;
     return cudaGetLastError();
@@ -1324,28 +1341,28 @@ cudaError_t prefill_run(Prefill *pf, cudaStream_t st, const int *tokens_host, in
     }
     PF_CK(cudaMemcpyAsync(pf->tokens, tokens_host, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st));
     const int dim = m.dim, hidden = m.hidden, kvd = pf->kv_dim;
-    const size_t kv_layer = (size_t)m.n_kv_heads * m.seq_len * m.head;
-    (void)kv_layer;
-    for (int c0 = 0; c0 < n; c0 += kT) {
-        const int nv = n - c0 < kT ? n - c0 : kT;
-        pf_embed_kernel<<<kT, 256, 0, st>>>(pf->tokens + c0, nv, m.emb, dim, m.vocab, pf->x);
+    for (int c0 = 0; c0 < n; c0 += kTB * kT) {
+        const int nv = n - c0 < kTB * kT ? n - c0 : kTB * kT;
+        const int tb = (nv + kT - 1) / kT;
+        const Splits ks = splits_for(pf, tb);
+        pf_embed_kernel<<<tb * kT, 256, 0, st>>>(pf->tokens + c0, nv, m.emb, dim, m.vocab, pf->x);
         ++pf->launches;
         PF_CK(cudaGetLastError());
         int pending = 0;     // partial row sums in `parts` that the next RMSNorm adds to x
         for (int l = 0; l < m.n_layers; ++l) {
             const PrefillLayerDesc &L = m.layers[(size_t)l];
-            PF_CK(launch_limbs<PF_IN_NORM>(pf, st, pf->x, L.rms_att, pf->parts, pending, dim, dim, nv));
+            PF_CK(launch_limbs<PF_IN_NORM>(pf, st, pf->x, L.rms_att, pf->parts, pending, dim, dim, tb, nv));
             {
                 const int w[3] = {PF_WQ, PF_WK, PF_WV}, col0[3] = {0, dim, dim + kvd};
-                PF_CK(launch_gemm(pf, st, l, w, 3, dim, pf->qkv, pf->qkv_ld, col0, pf->ksplit_qkv, nv, true));
+                PF_CK(launch_gemm(pf, st, l, w, 3, dim, pf->qkv, pf->qkv_ld, col0, 1, tb, nv, true));
             }
             {
                 PfRopeParams r{};
                 r.qkv = pf->qkv; r.q = pf->q; r.k_cache = L.kc; r.v_cache = L.vc;
                 r.rope_cos = m.rope_cos; r.rope_sin = m.rope_sin;
                 r.dim = dim; r.kv_dim = kvd; r.head = m.head; r.seq_len = m.seq_len; r.pos0 = pos0 + c0; r.nvalid = nv;
-                r.nparts = pf->ksplit_qkv;
-                const dim3 grid((unsigned)kT, (unsigned)((pf->qkv_ld / 2 + 255) / 256));
+                r.nparts = 1;
+                const dim3 grid((unsigned)(tb * kT), (unsigned)((pf->qkv_ld / 2 + 255) / 256));
                 pf_rope_kv_kernel<<<grid, 256, 0, st>>>(r);
                 ++pf->launches;
                 PF_CK(cudaGetLastError());
@@ -1370,7 +1387,7 @@ cudaError_t prefill_run(Prefill *pf, cudaStream_t st, const int *tokens_host, in
                 PfAttnParams a{};
                 a.q = pf->q; a.k_cache = L.kc; a.v_cache = L.vc; a.parts = pf->parts;
                 a.dim = dim; a.head = m.head; a.kv_mul = m.n_heads / m.n_kv_heads; a.seq_len = m.seq_len; a.pos0 = pos0 + c0; a.nvalid = nv;
-                a.nsplit = nsplit;
+                a.nsplit = nsplit; a.tpad = tb * kT;
                 const dim3 grid((unsigned)m.n_heads, (unsigned)((nv + kAttnQ - 1) / kAttnQ), (unsigned)nsplit);
                 if (m.head == 128)
                     pf_attention_kernel<128><<<grid, kAttnThreads, pf->attn_smem, st>>>(a);
@@ -1379,22 +1396,22 @@ cudaError_t prefill_run(Prefill *pf, cudaStream_t st, const int *tokens_host, in
                 ++pf->launches;
                 PF_CK(cudaGetLastError());
             }
-            PF_CK(launch_limbs<PF_IN_ATTN>(pf, st, nullptr, nullptr, pf->parts, nsplit, dim, dim, nv));
+            PF_CK(launch_limbs<PF_IN_ATTN>(pf, st, nullptr, nullptr, pf->parts, nsplit, dim, dim, tb, nv));
             {
                 const int w[1] = {PF_WO}, col0[1] = {0};
-                PF_CK(launch_gemm(pf, st, l, w, 1, dim, pf->parts, dim, col0, pf->ksplit_o, nv, false));
+                PF_CK(launch_gemm(pf, st, l, w, 1, dim, pf->parts, dim, col0, ks.o, tb, nv, false));
             }
-            PF_CK(launch_limbs<PF_IN_NORM>(pf, st, pf->x, L.rms_ffn, pf->parts, pf->ksplit_o, dim, dim, nv));
+            PF_CK(launch_limbs<PF_IN_NORM>(pf, st, pf->x, L.rms_ffn, pf->parts, ks.o, dim, dim, tb, nv));
             {
                 const int w[2] = {PF_W1, PF_W3}, col0[2] = {0, hidden};
-                PF_CK(launch_gemm(pf, st, l, w, 2, dim, pf->h13, 2 * hidden, col0, pf->ksplit_13, nv, true));
+                PF_CK(launch_gemm(pf, st, l, w, 2, dim, pf->h13, 2 * hidden, col0, ks.w13, tb, nv, true));
             }
-            PF_CK(launch_limbs<PF_IN_SWIGLU>(pf, st, pf->h13, pf->h13 + hidden, nullptr, pf->ksplit_13, 2 * hidden, hidden, nv));
+            PF_CK(launch_limbs<PF_IN_SWIGLU>(pf, st, pf->h13, pf->h13 + hidden, nullptr, ks.w13, 2 * hidden, hidden, tb, nv));
             {
                 const int w[1] = {PF_W2}, col0[1] = {0};
-                PF_CK(launch_gemm(pf, st, l, w, 1, hidden, pf->parts, dim, col0, pf->ksplit_2, nv, false));
+                PF_CK(launch_gemm(pf, st, l, w, 1, hidden, pf->parts, dim, col0, ks.w2, tb, nv, false));
             }
-            pending = pf->ksplit_2;
+            pending = ks.w2;
         }
     }
     return cudaSuccess;
@@ -1457,19 +1474,20 @@ static cudaError_t batch_enqueue(Prefill *pf, cudaStream_t st, int nv)
     ++pf->launches;
     PF_CK(cudaGetLastError());
     int pending = 0;
+    const Splits ks = splits_for(pf, 1);
     for (int l = 0; l < m.n_layers; ++l) {
         const PrefillLayerDesc &L = m.layers[(size_t)l];
-        PF_CK(launch_limbs<PF_IN_NORM>(pf, st, pf->x, L.rms_att, pf->parts, pending, dim, dim, nv));
+        PF_CK(launch_limbs<PF_IN_NORM>(pf, st, pf->x, L.rms_att, pf->parts, pending, dim, dim, 1, nv));
         {
             const int w[3] = {PF_WQ, PF_WK, PF_WV}, col0[3] = {0, dim, dim + kvd};
-            PF_CK(launch_gemm(pf, st, l, w, 3, dim, pf->qkv, pf->qkv_ld, col0, pf->ksplit_qkv, nv, true));
+            PF_CK(launch_gemm(pf, st, l, w, 3, dim, pf->qkv, pf->qkv_ld, col0, 1, 1, nv, true));
         }
         {
             PfRopeParams r{};
             r.qkv = pf->qkv; r.q = pf->q; r.k_cache = pf->bkc + l * layer_stride; r.v_cache = pf->bvc + l * layer_stride;
             r.rope_cos = m.rope_cos; r.rope_sin = m.rope_sin;
             r.dim = dim; r.kv_dim = kvd; r.head = m.head; r.seq_len = pf->seq_len_b; r.pos0 = 0; r.nvalid = nv;
-            r.nparts = pf->ksplit_qkv;
+            r.nparts = 1;
             r.pos_of = d_pos; r.seq_of = d_seq; r.seq_stride = seq_stride;
             const dim3 grid((unsigned)kT, (unsigned)((pf->qkv_ld / 2 + 255) / 256));
             pf_rope_kv_kernel<<<grid, 256, 0, st>>>(r);
@@ -1489,22 +1507,22 @@ static cudaError_t batch_enqueue(Prefill *pf, cudaStream_t st, int nv)
             ++pf->launches;
             PF_CK(cudaGetLastError());
         }
-        PF_CK(launch_limbs<PF_IN_ATTN>(pf, st, nullptr, nullptr, pf->parts, 1, dim, dim, nv));
+        PF_CK(launch_limbs<PF_IN_ATTN>(pf, st, nullptr, nullptr, pf->parts, 1, dim, dim, 1, nv));
         {
             const int w[1] = {PF_WO}, col0[1] = {0};
-            PF_CK(launch_gemm(pf, st, l, w, 1, dim, pf->parts, dim, col0, pf->ksplit_o, nv, false));
+            PF_CK(launch_gemm(pf, st, l, w, 1, dim, pf->parts, dim, col0, ks.o, 1, nv, false));
         }
-        PF_CK(launch_limbs<PF_IN_NORM>(pf, st, pf->x, L.rms_ffn, pf->parts, pf->ksplit_o, dim, dim, nv));
+        PF_CK(launch_limbs<PF_IN_NORM>(pf, st, pf->x, L.rms_ffn, pf->parts, ks.o, dim, dim, 1, nv));
         {
             const int w[2] = {PF_W1, PF_W3}, col0[2] = {0, hidden};
-            PF_CK(launch_gemm(pf, st, l, w, 2, dim, pf->h13, 2 * hidden, col0, pf->ksplit_13, nv, true));
+            PF_CK(launch_gemm(pf, st, l, w, 2, dim, pf->h13, 2 * hidden, col0, ks.w13, 1, nv, true));
         }
-        PF_CK(launch_limbs<PF_IN_SWIGLU>(pf, st, pf->h13, pf->h13 + hidden, nullptr, pf->ksplit_13, 2 * hidden, hidden, nv));
+        PF_CK(launch_limbs<PF_IN_SWIGLU>(pf, st, pf->h13, pf->h13 + hidden, nullptr, ks.w13, 2 * hidden, hidden, 1, nv));
         {
             const int w[1] = {PF_W2}, col0[1] = {0};
-            PF_CK(launch_gemm(pf, st, l, w, 1, hidden, pf->parts, dim, col0, pf->ksplit_2, nv, false));
+            PF_CK(launch_gemm(pf, st, l, w, 1, hidden, pf->parts, dim, col0, ks.w2, 1, nv, false));
         }
-        pending = pf->ksplit_2;
+        pending = ks.w2;
     }
     bd_final_norm_kernel<<<kT, 256, 0, st>>>(pf->x, pf->parts, pending, m.rms_final, dim, nv, pf->xn);
     PF_CK(cudaGetLastError());

@@ -1,7 +1,7 @@
 """Batched prompt processing (l2j_prefill) against the decode path it replaces and against the CPU checker.
 
-The reference pushes every prompt token through the decode step (Run.java:623-637); l2j_prefill runs 64
-positions per sweep over the weights on the tensor cores.  Per position it computes the decode step's
+The reference pushes every prompt token through the decode step (Run.java:623-637); l2j_prefill runs up to
+256 positions per sweep over the weights on the tensor cores.  Per position it computes the decode step's
 arithmetic with the row sums added in another order, so the gates are tolerances, written here: the K/V
 cache rows the prompt leaves behind within 1e-4 of the row's largest magnitude, and the logits of the decode
 step after the prompt within 1e-4 of the logit range of the decode-only path (and within the 1e-3 of the
@@ -101,6 +101,15 @@ def test_prefill_ragged_lengths_and_continuation():
         pre.close()
         assert float(np.abs(got - ref).max()) / float(ref.max() - ref.min()) < LOGIT_TOL, first
     dec.close()
+
+
+@pytest.mark.parametrize("heads", [4, 8])                       # head sizes 128 and 64
+@pytest.mark.parametrize("n", [1, 63, 129, 192, 256, 257, 321])
+def test_prefill_lengths_around_the_blocks_of_a_chunk(n, heads):
+    """Blocks of 64 tokens, chunks of 256: one token, one short of a block, two, three and four blocks, a second chunk."""
+    cfg = ModelConfig(512, 1280, 2, heads, heads // 2, 1000, 512, True)
+    positions = sorted({0, n // 2, n - 1} | {p for p in (63, 64, 128, 191, 255, 256) if p < n})
+    _compare_with_decode(cfg, _tensors(cfg, 8), n, positions, (0, 1))
 
 
 def test_prefill_then_decode_against_the_checker(oracle):
