@@ -17,7 +17,8 @@
 //                       accumulator per quantisation group in tensor memory, double-buffered; four epilogue warps
 //                       read it back (tcgen05.ld), scale in FP32 and keep the row sums in registers
 //   pf_rope_kv_kernel   RoPE on q and k, rows of the K/V cache (ApplyRope.java:61-92, Run.java:443-455)
-//   pf_attention_kernel causal attention of the chunk's queries over the cache, FP32, online softmax
+//   pf_attention_kernel causal attention of the chunk's queries over the cache: FP32 operands in three bf16 pieces on
+//                       the tensor cores, online softmax in FP32
 
 #include "l2j_device.cuh"
 #include "l2j_internal.h"
@@ -652,188 +653,424 @@ __global__ void pf_rope_kv_kernel(PfRopeParams p)
 // causal attention of the chunk's queries
 // ---------------------------------------------------------------------------------------------------------------
 
-struct PfAttnParams {
-    const float *q;        // [tokens][dim] after RoPE
-    const float *k_cache, *v_cache;
-    float *parts;          // [nsplit][tpad][heads][head + 2]: unnormalised output, running maximum, sum of the key range
-    int dim, head, kv_mul, seq_len, pos0, nvalid, nsplit;
-    int tpad;              // tokens of the chunk, whole blocks of 64
-};
-
-constexpr int kAttnQ = 32;       // queries per block
-constexpr int kAttnKeys = 64;    // keys per tile
-constexpr int kAttnThreads = 128;
-
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-__device__ __forceinline__ void cp_async_wait_all()
+struct PfAttnParams {
+    const float *q;        // [tokens][dim] after RoPE
+    const float *k_cache, *v_cache;
+    float *parts;          // [nsplit][tpad][heads][head + 2]: unnormalised output, running maximum, sum of the key range
+    int dim, kv_mul, seq_len, pos0, nvalid, nsplit;
+    int tpad;              // tokens of the chunk, whole blocks of 64
+    int timeout_us;
+    unsigned int *status;
+};
+
+// Block = (head, 128 queries, one range of key tiles), on the tensor cores without giving up FP32: every operand is
+// the sum of three bf16 numbers of 8 significant bits (24 in all, exact), and the six products of pieces that reach
+// 2^-24 of the result are added, the smallest first, into a fresh FP32 accumulator per tile; the running output is
+// kept and rescaled in FP32 registers, so no sum is longer than one tile in the tensor cores' accumulator.
+//
+//   warps 0-3    softmax: thread = query row; S from tensor memory, online maximum and sum, the three pieces of P back
+//                into tensor memory (the A operand of the second product)
+//   warps 4-11   K and V of the tile from global memory through registers into their pieces in shared memory (V
+//                transposed: both operands K-major, 128-byte swizzle); the output row of the query in registers
+//   warp 12      issue: S(j + 1) = Q K' while the softmax works on tile j, then O(j) = P V
+//
+// Six bf16 products of 128 x 64 x HEAD, twice per tile, are 3072 tensor-core cycles at head size 128; on the FP32 units
+// the same tile takes 16384 cycles at best.  3840 tokens through 16 layers of the 7B shape: 144 ms with the FP32 kernel
+// before this one (4 x 4 scores per thread), 88 ms with it.  Error against float64 the same or lower (3.4e-6 against 3.6e-6
+// of a row of V behind it, mean over head sizes 64 and 128 and peaked softmaxes).
+constexpr int kAttnQ = 128;      // queries per block: the rows of one accumulator
+constexpr int kAttnKeys = 64;    // keys per tile
+constexpr int kAttnSoft = 4, kAttnCvt = 8;              // warps by role
+constexpr int kAttnThreads = 32 * (kAttnSoft + kAttnCvt + 1);
+constexpr int kAttnColO = 128, kAttnColP = 256;         // tensor memory: S 2 x 64 columns, O, P 3 x 32 columns
+
+template <int HEAD>
+constexpr size_t attn_smem_bytes()
 {
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    return (size_t)3 * (kAttnQ + 2 * kAttnKeys) * HEAD * 2 + 1024;      // pieces of Q, K and V, alignment
 }
 
-// Block = (head, 32 queries, one range of key tiles); thread = 4 queries x 4 keys of a tile for the scores and
-// 4 queries x HEAD / 16 elements for the output.  The K and V rows of a tile come into shared memory with
-// asynchronous 16-byte copies (no registers, no load-to-store dependency per row); two blocks share an SM.
-template <int HEAD>
-__global__ void __launch_bounds__(kAttnThreads, 2) pf_attention_kernel(const PfAttnParams p)
+// c f32, a and b bf16, both K-major, M 128
+__host__ __device__ constexpr uint32_t attn_idesc(int n)
 {
-    constexpr int LD = HEAD + 4;             // row pitch in floats: consecutive rows start 4 banks apart
-    constexpr int NV4 = HEAD / 64;           // float4 chunks of the output per thread and query
-    extern __shared__ __align__(16) float pf_att_smem[];
-    float *sK = pf_att_smem;                 // [64][LD]
-    float *sV = sK + kAttnKeys * LD;
-    float *sQ = sV + kAttnKeys * LD;         // [32][LD]
-    float *sP = sQ + kAttnQ * LD;            // [32][64]
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kAttnQ >> 4) << 24);
+}
 
-    const int h = blockIdx.x, q0 = blockIdx.y * kAttnQ, z = blockIdx.z, tid = threadIdx.x;
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// A from tensor memory: two consecutive K elements per 32-bit column
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *r)
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]),
+        "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_wait()
+{
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// A pair of floats as three pairs of bf16 that add up to them: each difference is exact, and what the third piece has to
+// hold fits its 8 bits.
+__device__ __forceinline__ void split_bf16(float a, float b, uint32_t (&piece)[3])
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(piece[i]) : "f"(b), "f"(a));
+        a -= __uint_as_float(piece[i] << 16);
+        b -= __uint_as_float(piece[i] & 0xffff0000u);
+    }
+}
+
+// Eight floats to the 16-byte chunk `chunk` of row `row` of a swizzled K-major tile, one tile per piece.
+__device__ __forceinline__ void store_pieces(unsigned char *tile, uint32_t piece_bytes, int row, int chunk, const float *v)
+{
+    uint32_t w[4][3];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        split_bf16(v[2 * i], v[2 * i + 1], w[i]);
+    unsigned char *dst = tile + row * 128 + ((chunk ^ (row & 7)) << 4);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        *reinterpret_cast<uint4 *>(dst + i * piece_bytes) = make_uint4(w[0][i], w[1][i], w[2][i], w[3][i]);
+}
+
+// The pairs of pieces whose product is added, the smallest first (0: the leading eight bits).
+__device__ __constant__ const int kPairA[6] = {2, 1, 0, 1, 0, 0}, kPairB[6] = {0, 1, 2, 0, 1, 0};
+
+template <int HEAD>
+__global__ void __launch_bounds__(kAttnThreads, 1) pf_attention_kernel(const PfAttnParams p)
+{
+    constexpr int HB = HEAD / 64;                            // 64-column blocks of a row of Q and K
+    constexpr uint32_t kQBlock = kAttnQ * 128, kKBlock = kAttnKeys * 128, kVPiece = HEAD * 128;
+    constexpr uint32_t kQPiece = HB * kQBlock, kKPiece = HB * kKBlock;
+    constexpr int NU = HEAD / 32;                            // units of eight elements per converting thread and tile
+    constexpr int NO = HEAD / 2;                             // output elements per converting thread
+    extern __shared__ unsigned char pf_att_smem[];
+    __shared__ __align__(8) unsigned long long s_bar[11];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_give_up;
+    __shared__ float s_alpha[2][kAttnQ];
+
+    const int h = blockIdx.x, q0 = blockIdx.y * kAttnQ, z = blockIdx.z;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (q0 >= p.nvalid)
         return;
+    const uint32_t base = (smem_u32(pf_att_smem) + 1023u) & ~1023u;
+    unsigned char *gen = pf_att_smem + (base - smem_u32(pf_att_smem));
+    unsigned char *gQ = gen, *gK = gQ + 3 * kQPiece, *gV = gK + 3 * kKPiece;
+    const uint32_t aQ = base, aK = aQ + 3 * kQPiece, aV = aK + 3 * kKPiece;
+    const uint32_t bar = smem_u32(&s_bar[0]);
+    const uint32_t b_k = bar, b_v = bar + 8, b_p = bar + 16, b_pv = bar + 24, b_qk = bar + 32, b_s = bar + 48, b_a = bar + 64,
+                   b_fin = bar + 80;                         // b_qk, b_s, b_a: two each, by the tile's parity
+    const long long limit = 2000ll * (long long)p.timeout_us;
+    volatile int *give_up = &s_give_up;
+
     const int kvh = h / p.kv_mul;
     const float *kbase = p.k_cache + (size_t)kvh * p.seq_len * HEAD;
     const float *vbase = p.v_cache + (size_t)kvh * p.seq_len * HEAD;
-    const int qa = (tid >> 4) * 4;           // this thread's four queries
-    const int kb = tid & 15;                 // its keys are kb, kb + 16, kb + 32, kb + 48 of a tile
-    const float root = sqrtf((float)HEAD);   // AttentionLoop: score / sqrt(head_size)
-
-    const int last_q = min(q0 + kAttnQ, p.nvalid) - 1;
-    const int nkeys = p.pos0 + last_q + 1;                      // keys 0 .. position of the block's last query
+    const int nkeys = p.pos0 + min(q0 + kAttnQ, p.nvalid);  // keys 0 .. position of the block's last query
     const int tiles = (nkeys + kAttnKeys - 1) / kAttnKeys;
     const int tper = (tiles + p.nsplit - 1) / p.nsplit;
-    const int t_lo = z * tper, t_hi = min(tiles, t_lo + tper);
+    const int t_lo = z * tper, n = max(0, min(tiles, t_lo + tper) - t_lo);
 
-    for (int i = tid; i < kAttnQ * (HEAD / 4); i += kAttnThreads) {
-        const int r = i / (HEAD / 4), c = i % (HEAD / 4);
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (q0 + r < p.nvalid)
-            v = *reinterpret_cast<const float4 *>(p.q + (size_t)(q0 + r) * p.dim + h * HEAD + c * 4);
-        *reinterpret_cast<float4 *>(sQ + r * LD + c * 4) = v;
+    if (tid == 0) {
+        mbar_init(b_k, kAttnCvt);
+        mbar_init(b_v, kAttnCvt);
+        mbar_init(b_p, kAttnSoft);
+        mbar_init(b_pv, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(b_qk + 8 * i, 1);
+            mbar_init(b_s + 8 * i, kAttnSoft);
+            mbar_init(b_a + 8 * i, kAttnSoft);
+        }
+        mbar_init(b_fin, 1);
+        mbar_fence_init();
+        s_give_up = 0;
     }
-    float m[4], l[4];
-    float4 o[4][NV4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        m[i] = -FLT_MAX;
-        l[i] = 0.f;
-#pragma unroll
-        for (int c = 0; c < NV4; ++c)
-            o[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (warp == kAttnSoft + kAttnCvt) {
+        tmem_alloc(smem_u32(&s_tmem), kTmemCols);
+        tmem_relinquish();
     }
-
-    for (int tile = t_lo; tile < t_hi; ++tile) {
-        const int k0 = tile * kAttnKeys;
-        __syncthreads();
-        for (int i = tid; i < kAttnKeys * (HEAD / 4); i += kAttnThreads) {
-            const int r = i / (HEAD / 4), c = i % (HEAD / 4);
-            if (k0 + r < nkeys) {
-                cp_async16(smem_u32(sK + r * LD + c * 4), kbase + (size_t)(k0 + r) * HEAD + c * 4);
-                cp_async16(smem_u32(sV + r * LD + c * 4), vbase + (size_t)(k0 + r) * HEAD + c * 4);
-            } else {
-                *reinterpret_cast<float4 *>(sK + r * LD + c * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<float4 *>(sV + r * LD + c * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+    for (int u = tid; u < kAttnQ * HEAD / 8; u += kAttnThreads) {
+        const int r = u / (HEAD / 8), c8 = u % (HEAD / 8);
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (q0 + r < p.nvalid) {
+            const float4 *src = reinterpret_cast<const float4 *>(p.q + (size_t)(q0 + r) * p.dim + h * HEAD + c8 * 8);
+            const float4 x = src[0], y = src[1];
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
         }
-        cp_async_wait_all();
-        __syncthreads();
-        // scores of 4 queries x 4 keys
-        float s[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                s[i][j] = 0.f;
-#pragma unroll 2
-        for (int d = 0; d < HEAD; d += 4) {
-            float4 qv[4], kv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                qv[i] = *reinterpret_cast<const float4 *>(sQ + (qa + i) * LD + d);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                kv[j] = *reinterpret_cast<const float4 *>(sK + (kb + 16 * j) * LD + d);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    s[i][j] = fmaf(qv[i].x, kv[j].x, s[i][j]);
-                    s[i][j] = fmaf(qv[i].y, kv[j].y, s[i][j]);
-                    s[i][j] = fmaf(qv[i].z, kv[j].z, s[i][j]);
-                    s[i][j] = fmaf(qv[i].w, kv[j].w, s[i][j]);
-                }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int qpos = p.pos0 + q0 + qa + i;
-            float mx = -FLT_MAX;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int key = k0 + kb + 16 * j;
-                s[i][j] = key <= qpos ? __fdiv_rn(s[i][j], root) : -FLT_MAX;
-                mx = fmaxf(mx, s[i][j]);
-            }
-#pragma unroll
-            for (int o2 = 1; o2 < 16; o2 <<= 1)
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o2));
-            const float mn = fmaxf(m[i], mx);
-            const float alpha = expf(m[i] - mn);
-            float sum = 0.f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float pv = s[i][j] > -FLT_MAX ? expf(s[i][j] - mn) : 0.f;
-                sP[(qa + i) * kAttnKeys + kb + 16 * j] = pv;
-                sum += pv;
-            }
-#pragma unroll
-            for (int o2 = 1; o2 < 16; o2 <<= 1)
-                sum += __shfl_xor_sync(0xffffffffu, sum, o2);
-            l[i] = l[i] * alpha + sum;
-            m[i] = mn;
-#pragma unroll
-            for (int c = 0; c < NV4; ++c) {
-                o[i][c].x *= alpha; o[i][c].y *= alpha; o[i][c].z *= alpha; o[i][c].w *= alpha;
-            }
-        }
-        __syncthreads();
-        const int kmax = (min(kAttnKeys, nkeys - k0) + 3) & ~3;   // rows past the last key hold zeros and weigh zero
-        for (int j = 0; j < kmax; j += 4) {
-            float4 pj[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                pj[i] = *reinterpret_cast<const float4 *>(sP + (qa + i) * kAttnKeys + j);
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-#pragma unroll
-                for (int c = 0; c < NV4; ++c) {
-                    const float4 vv = *reinterpret_cast<const float4 *>(sV + (j + jj) * LD + c * 64 + kb * 4);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float w = jj == 0 ? pj[i].x : (jj == 1 ? pj[i].y : (jj == 2 ? pj[i].z : pj[i].w));
-                        o[i][c].x = fmaf(w, vv.x, o[i][c].x); o[i][c].y = fmaf(w, vv.y, o[i][c].y);
-                        o[i][c].z = fmaf(w, vv.z, o[i][c].z); o[i][c].w = fmaf(w, vv.w, o[i][c].w);
-                    }
-                }
-            }
-        }
+        store_pieces(gQ + (c8 >> 3) * kQBlock, kQPiece, r, c8 & 7, v);
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
     const int heads = p.dim / HEAD;
+
+    if (warp < kAttnSoft) {
+        // ---- softmax: thread = query row
+        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+        const int row = warp * 32 + lane, qpos = p.pos0 + q0 + row;
+        const float root = sqrtf((float)HEAD), inv_root = __fdiv_rn(1.0f, root);   // AttentionLoop: score / sqrt(head_size)
+        float m = -FLT_MAX, l = 0.f;
+        for (int j = 0; j < n; ++j) {
+            const int k0 = (t_lo + j) * kAttnKeys;
+            if (!__all_sync(0xffffffffu, pf_wait(b_qk + 8 * (j & 1), (uint32_t)((j >> 1) & 1), give_up, limit)))
+                break;
+            tc_fence_after();
+            uint32_t raw[64];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int qi = q0 + qa + i;
-        if (qi < p.nvalid) {
-            float *rec = p.parts + ((size_t)(z * p.tpad + qi) * heads + h) * (HEAD + 2);
+            for (int c = 0; c < 4; ++c)
+                tmem_ld16(trow + (uint32_t)((j & 1) * kAttnKeys + 16 * c), raw + 16 * c);
+            tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(b_s + 8 * (j & 1));
+            float mx = -FLT_MAX;
+            const int last = qpos - k0;                      // keys past it are masked
 #pragma unroll
-            for (int c = 0; c < NV4; ++c) {   // records are 8-byte aligned (HEAD + 2 floats each)
-                *reinterpret_cast<float2 *>(rec + c * 64 + kb * 4) = make_float2(o[i][c].x, o[i][c].y);
-                *reinterpret_cast<float2 *>(rec + c * 64 + kb * 4 + 2) = make_float2(o[i][c].z, o[i][c].w);
+            for (int c = 0; c < 64; ++c) {
+                // s / root: the product with the reciprocal and one correction of its remainder
+                const float s = __uint_as_float(raw[c]);
+                const float q = __fmul_rn(s, inv_root);
+                const float r = fmaf(-q, root, s);
+                float v = r == r ? fmaf(r, inv_root, q) : q;
+                v = c <= last ? v : -FLT_MAX;
+                raw[c] = __float_as_uint(v);
+                mx = fmaxf(mx, v);
             }
-            if (kb == 0) {
-                rec[HEAD] = m[i];
-                rec[HEAD + 1] = l[i];
+            const float mn = fmaxf(m, mx);
+            const float alpha = expf(m - mn);
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 64; ++c) {
+                const float v = __uint_as_float(raw[c]);
+                const float pv = v > -FLT_MAX ? expf(v - mn) : 0.f;
+                raw[c] = __float_as_uint(pv);
+                sum[c & 3] += pv;
+            }
+            l = l * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+            m = mn;
+            if (j > 0 && !__all_sync(0xffffffffu, pf_wait(b_pv, (uint32_t)((j - 1) & 1), give_up, limit)))
+                break;
+            tc_fence_after();
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t w[3][16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    uint32_t pc[3];
+                    split_bf16(__uint_as_float(raw[32 * half + 2 * i]), __uint_as_float(raw[32 * half + 2 * i + 1]), pc);
+                    w[0][i] = pc[0]; w[1][i] = pc[1]; w[2][i] = pc[2];
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    tmem_st16(trow + (uint32_t)(kAttnColP + 32 * i + 16 * half), w[i]);
+            }
+            tmem_st_wait();
+            s_alpha[j & 1][row] = alpha;
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(b_p);
+                mbar_arrive(b_a + 8 * (j & 1));
+            }
+        }
+        if (q0 + row < p.nvalid && !*give_up) {
+            float *rec = p.parts + ((size_t)(z * p.tpad + q0 + row) * heads + h) * (HEAD + 2);
+            rec[HEAD] = m;
+            rec[HEAD + 1] = l;
+        }
+    } else if (warp < kAttnSoft + kAttnCvt) {
+        // ---- operands and output: K and V unit by unit, output row q, half of its elements
+        const int ct = tid - 32 * kAttnSoft, quarter = warp & 3, part = (warp - kAttnSoft) >> 2;
+        const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(kAttnColO + part * NO);
+        const int row = quarter * 32 + lane;
+        float o[NO];
+#pragma unroll
+        for (int i = 0; i < NO; ++i)
+            o[i] = 0.f;
+        float x[NU][8];
+        auto load_k = [&](int j) {
+            const int k0 = (t_lo + j) * kAttnKeys;
+#pragma unroll
+            for (int i = 0; i < NU; ++i) {
+                const int u = ct + 256 * i, key = u / (HEAD / 8), c8 = u % (HEAD / 8);
+                float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+                if (k0 + key < nkeys) {
+                    const float4 *src = reinterpret_cast<const float4 *>(kbase + (size_t)(k0 + key) * HEAD + c8 * 8);
+                    a = src[0];
+                    b = src[1];
+                }
+                x[i][0] = a.x; x[i][1] = a.y; x[i][2] = a.z; x[i][3] = a.w; x[i][4] = b.x; x[i][5] = b.y; x[i][6] = b.z; x[i][7] = b.w;
+            }
+        };
+        auto load_v = [&](int j) {
+            const int k0 = (t_lo + j) * kAttnKeys;
+#pragma unroll
+            for (int i = 0; i < NU; ++i) {
+                const int u = ct + 256 * i, d = u % HEAD, key = 8 * (u / HEAD);
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    x[i][e] = k0 + key + e < nkeys ? vbase[(size_t)(k0 + key + e) * HEAD + d] : 0.f;
+            }
+        };
+        auto publish = [&](uint32_t b) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(b);
+        };
+        auto store_k = [&]() {
+#pragma unroll
+            for (int i = 0; i < NU; ++i) {
+                const int u = ct + 256 * i, key = u / (HEAD / 8), c8 = u % (HEAD / 8);
+                store_pieces(gK + (c8 >> 3) * kKBlock, kKPiece, key, c8 & 7, x[i]);
+            }
+            publish(b_k);
+        };
+        auto add_output = [&](int j) -> bool {               // O(j) of the tensor cores into the running output
+            if (!__all_sync(0xffffffffu, pf_wait(b_a + 8 * (j & 1), (uint32_t)((j >> 1) & 1), give_up, limit)) ||
+                !__all_sync(0xffffffffu, pf_wait(b_pv, (uint32_t)(j & 1), give_up, limit)))
+                return false;
+            tc_fence_after();
+            const float alpha = s_alpha[j & 1][row];
+#pragma unroll
+            for (int c = 0; c < NO; c += 16) {
+                uint32_t t[16];
+                tmem_ld16(trow + (uint32_t)c, t);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    o[c + i] = fmaf(o[c + i], alpha, __uint_as_float(t[i]));
+            }
+            tc_fence_before();
+            return true;
+        };
+        if (n > 0) {
+            load_k(0);
+            store_k();
+        }
+        if (n > 1)
+            load_k(1);
+        bool ok = true;
+        for (int j = 0; j < n; ++j) {
+            if (j + 1 < n) {
+                ok = __all_sync(0xffffffffu, pf_wait(b_qk + 8 * (j & 1), (uint32_t)((j >> 1) & 1), give_up, limit));
+                if (!ok)
+                    break;
+                store_k();
+            }
+            load_v(j);
+            if (j > 0) {
+                ok = add_output(j - 1);
+                if (!ok)
+                    break;
+            }
+#pragma unroll
+            for (int i = 0; i < NU; ++i) {
+                const int u = ct + 256 * i;
+                store_pieces(gV, kVPiece, u % HEAD, u / HEAD, x[i]);
+            }
+            publish(b_v);
+            if (j + 2 < n)
+                load_k(j + 2);
+        }
+        if (ok && n > 0)
+            ok = add_output(n - 1);
+        if (ok && q0 + row < p.nvalid) {
+            float *rec = p.parts + ((size_t)(z * p.tpad + q0 + row) * heads + h) * (HEAD + 2) + part * NO;
+#pragma unroll
+            for (int i = 0; i < NO; i += 2)                  // records are 8-byte aligned (HEAD + 2 floats each)
+                *reinterpret_cast<float2 *>(rec + i) = make_float2(o[i], o[i + 1]);
+        }
+    } else if (lane == 0) {
+        // ---- tensor-core issue: one lane
+        bool ok = true;
+        for (int j = 0; j <= n && n > 0; ++j) {
+            if (j < n) {
+                ok = pf_wait(b_k, (uint32_t)(j & 1), give_up, limit) &&
+                     (j < 2 || pf_wait(b_s + 8 * (j & 1), (uint32_t)(((j >> 1) - 1) & 1), give_up, limit));
+                if (!ok)
+                    break;
+                tc_fence_after();
+                const uint32_t d = tmem + (uint32_t)((j & 1) * kAttnKeys);
+#pragma unroll 1
+                for (int i = 0; i < 6; ++i) {
+                    const uint32_t ta = aQ + (uint32_t)kPairA[i] * kQPiece, tb = aK + (uint32_t)kPairB[i] * kKPiece;
+#pragma unroll
+                    for (int kk = 0; kk < HEAD / 16; ++kk)
+                        umma_bf16(d, smem_desc_sw128(ta + (kk >> 2) * kQBlock + (kk & 3) * 32u),
+                                  smem_desc_sw128(tb + (kk >> 2) * kKBlock + (kk & 3) * 32u), attn_idesc(kAttnKeys), (i | kk) ? 1u : 0u);
+                }
+                umma_commit(b_qk + 8 * (j & 1));
+            }
+            if (j > 0) {
+                ok = pf_wait(b_p, (uint32_t)((j - 1) & 1), give_up, limit) && pf_wait(b_v, (uint32_t)((j - 1) & 1), give_up, limit);
+                if (!ok)
+                    break;
+                tc_fence_after();
+#pragma unroll 1
+                for (int i = 0; i < 6; ++i) {
+                    const uint32_t ta = tmem + kAttnColP + 32u * (uint32_t)kPairA[i], tb = aV + (uint32_t)kPairB[i] * kVPiece;
+#pragma unroll
+                    for (int kk = 0; kk < kAttnKeys / 16; ++kk)
+                        umma_bf16_ts(tmem + kAttnColO, ta + 8u * kk, smem_desc_sw128(tb + kk * 32u), attn_idesc(HEAD), (i | kk) ? 1u : 0u);
+                }
+                umma_commit(b_pv);
+            }
+        }
+        if (!ok || *give_up) {
+            umma_commit(b_fin);
+            const long long c0 = sm_clock();
+            while (!mbar_try_wait(b_fin, 0) && sm_clock() - c0 < limit) {
             }
         }
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == kAttnSoft + kAttnCvt)
+        tmem_dealloc(tmem, kTmemCols);
+    if (tid == 0 && s_give_up)
+        atomicOr(p.status, PF_DS_WAIT_TIMEOUT);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1217,8 +1454,7 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m)
     pf->gemm_smem_hidden = (size_t)kStages * kStageBytes + (size_t)(m.hidden / 256) * kT * sizeof(float2) + 1024;
     const size_t gmax = pf->gemm_smem_dim > pf->gemm_smem_hidden ? pf->gemm_smem_dim : pf->gemm_smem_hidden;
     e = cudaFuncSetAttribute(pf_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gmax);
-    const int ld = m.head + 4;
-    pf->attn_smem = (size_t)(2 * kAttnKeys * ld + kAttnQ * ld + kAttnQ * kAttnKeys) * sizeof(float);
+    pf->attn_smem = m.head == 128 ? attn_smem_bytes<128>() : attn_smem_bytes<64>();
     if (e == cudaSuccess)
         e = m.head == 128 ? cudaFuncSetAttribute(pf_attention_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf->attn_smem)
                           : cudaFuncSetAttribute(pf_attention_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf->attn_smem);
@@ -1369,25 +1605,23 @@ cudaError_t prefill_run(Prefill *pf, cudaStream_t st, const int *tokens_host, in
             }
             int nsplit = 1;
             {
+                // Key ranges per (head, 128 queries): the count that needs the fewest rounds of key tiles with one block per
+                // SM; a block's set-up (the pieces of Q, the first tile through every role) and the merge of its part cost
+                // about three tiles.
                 const int tiles = (pos0 + c0 + nv + kAttnKeys - 1) / kAttnKeys;
-                // key ranges per (head, 32 queries): the count that needs the fewest rounds of key tiles, with two
-                // blocks resident per SM (each block pays about half a tile for its set-up and the merge of a part)
-                {
-                    const int base = m.n_heads * ((nv + kAttnQ - 1) / kAttnQ), places = 2 * pf->sms;
-                    float best = 0.f;
-                    for (int ns = 1; ns <= kMaxParts && ns <= tiles; ++ns) {
-                        const int waves = (base * ns + places - 1) / places;
-                        const float cost = (float)waves * ((float)((tiles + ns - 1) / ns) + 0.5f);
-                        if (ns == 1 || cost < best) {
-                            best = cost;
-                            nsplit = ns;
-                        }
+                const int base = m.n_heads * ((nv + kAttnQ - 1) / kAttnQ);
+                int best = 0;
+                for (int ns = 1; ns <= kMaxParts && ns <= tiles; ++ns) {
+                    const int cost = ((base * ns + pf->sms - 1) / pf->sms) * ((tiles + ns - 1) / ns + 3);
+                    if (ns == 1 || cost < best) {
+                        best = cost;
+                        nsplit = ns;
                     }
                 }
                 PfAttnParams a{};
                 a.q = pf->q; a.k_cache = L.kc; a.v_cache = L.vc; a.parts = pf->parts;
-                a.dim = dim; a.head = m.head; a.kv_mul = m.n_heads / m.n_kv_heads; a.seq_len = m.seq_len; a.pos0 = pos0 + c0; a.nvalid = nv;
-                a.nsplit = nsplit; a.tpad = tb * kT;
+                a.dim = dim; a.kv_mul = m.n_heads / m.n_kv_heads; a.seq_len = m.seq_len; a.pos0 = pos0 + c0; a.nvalid = nv;
+                a.nsplit = nsplit; a.tpad = tb * kT; a.timeout_us = m.timeout_us; a.status = m.status;
                 const dim3 grid((unsigned)m.n_heads, (unsigned)((nv + kAttnQ - 1) / kAttnQ), (unsigned)nsplit);
                 if (m.head == 128)
                     pf_attention_kernel<128><<<grid, kAttnThreads, pf->attn_smem, st>>>(a);

@@ -112,6 +112,29 @@ def test_prefill_lengths_around_the_blocks_of_a_chunk(n, heads):
     _compare_with_decode(cfg, _tensors(cfg, 8), n, positions, (0, 1))
 
 
+@pytest.mark.parametrize("heads, kv_heads", [(4, 2), (8, 8), (8, 2)])
+@pytest.mark.parametrize("first, more", [(1, 1), (63, 2), (64, 64), (65, 127), (190, 131), (320, 180)])
+def test_prefill_attention_around_its_tiles(heads, kv_heads, first, more):
+    """Key tiles of 64, query blocks of 128, key ranges: a second call whose queries start and end beside their edges."""
+    cfg = ModelConfig(512, 1280, 2, heads, kv_heads, 1000, 512, True)
+    tensors = _tensors(cfg, 9)
+    n = first + more
+    toks = _inputs(cfg, n)
+    dec = _build(cfg, tensors)
+    for i in range(n):
+        dec.forward(int(toks[i]), i, want_logits=False)
+    pre = _build(cfg, tensors)
+    pre.prefill(toks[:first], 0)
+    pre.prefill(toks[first:], first)
+    for pos in sorted({first, (first + n) // 2, n - 1}):
+        for which in (5, 6):
+            a, b = dec.read_buffer(which, cfg.kv_dim, 1, pos), pre.read_buffer(which, cfg.kv_dim, 1, pos)
+            assert float(np.abs(a - b).max()) / float(np.abs(a).max()) < CACHE_TOL, (pos, which)
+    assert pre.stats().device_status == 0
+    dec.close()
+    pre.close()
+
+
 def test_prefill_then_decode_against_the_checker(oracle):
     """A 100-token prompt through l2j_prefill, then greedy decoding: logits of every decoded position within
     the north star's 1e-3 of range of the CPU checker that ran the whole sequence token by token."""
