@@ -72,6 +72,29 @@ def test_sequences_of_different_lengths_step_together(cfg):
     m.close()
 
 
+@pytest.mark.parametrize("cfg", [ModelConfig(512, 1280, 2, 4, 2, 1000, 320, True),
+                                 ModelConfig(512, 1280, 2, 8, 8, 1029, 320, False)], ids=["heads128", "heads64"])
+def test_lengths_around_the_key_ranges(cfg):
+    """Rounds of 32 keys per block, ranges of whole rounds, more ranges than a short sequence fills; alone and together."""
+    lengths = [1, 7, 8, 31, 32, 33, 64, 96, 257, 300]
+    tensors = _tensors(cfg, 21)
+    stream = np.concatenate([[1], np.random.default_rng(22).integers(3, cfg.vocab_size, 300)]).astype(np.int32)
+    refs = _alone(cfg, tensors, stream)
+    m = _build(cfg, tensors)
+    m.batch_create(len(lengths), 310)
+    entries = [(s, p) for s, n in enumerate(lengths) for p in range(n)]
+    for i in range(0, len(entries), 64):
+        part = entries[i: i + 64]
+        m.batch_forward([s for s, _ in part], [p for _, p in part], [int(stream[p]) for _, p in part], want_logits=False)
+    for some in (list(range(len(lengths))), [8], [0], [5, 9], [3, 4, 8]):
+        logits, am = m.batch_forward(some, [lengths[s] for s in some], [int(stream[lengths[s]]) for s in some])
+        for i, s in enumerate(some):
+            _check(logits[i], refs[lengths[s]])
+            assert int(am[i]) == int(logits[i].argmax())
+    assert m.stats().device_status == 0
+    m.close()
+
+
 def test_full_batch_of_64_at_the_110m_shape():
     cfg = syn.SHAPES["stories110M"]
     tensors = _tensors(cfg, 13)
