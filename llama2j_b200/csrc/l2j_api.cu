@@ -1425,6 +1425,7 @@ static PrefillModel prefill_model(l2j_ctx *c)
     m.rms_final = c->rms_final;
     m.status = reinterpret_cast<unsigned int *>(&c->state->status);
     m.timeout_us = c->wait_limit_us;
+    m.pdl = !(c->flags & L2J_F_NO_PDL);
     auto payload = [](const MvSeg &s) { return s.payload + s.flat0; };
     auto hdr = [](const MvSeg &s) { return s.hdr + s.flat0 / kGroup; };
     for (int li = 0; li < c->nl; ++li) {

@@ -267,6 +267,7 @@ struct PrefillModel {
     const float *rope_cos, *rope_sin;
     unsigned int *status;            // device status word of the context
     int timeout_us;
+    bool pdl;                        // programmatic dependent launch between the kernels (not with L2J_F_NO_PDL)
     std::vector<PrefillLayerDesc> layers;
 };
 

@@ -27,8 +27,8 @@ def _tensors(cfg, seed):
     return tensors
 
 
-def _build(cfg, tensors):
-    m = Transformer(cfg, 0, 0, None, 0)
+def _build(cfg, tensors, flags=0):
+    m = Transformer(cfg, 0, 0, None, flags)
     m.upload_all(tensors)
     m.finalize()
     return m
@@ -93,6 +93,27 @@ def test_lengths_around_the_key_ranges(cfg):
             assert int(am[i]) == int(logits[i].argmax())
     assert m.stats().device_status == 0
     m.close()
+
+
+@pytest.mark.parametrize("heads", [4, 8])
+def test_overlapped_launches_change_nothing(heads):
+    """A prompt of two chunks and a step of three sequences with programmatic dependent launch and without: same bits."""
+    cfg = ModelConfig(512, 1280, 3, heads, heads // 2, 1000, 512, True)
+    tensors = _tensors(cfg, 23)
+    toks = np.random.default_rng(24).integers(3, cfg.vocab_size, 300).astype(np.int32)
+    got = []
+    for flags in (0, L.F_NO_PDL):
+        m = _build(cfg, tensors, flags)
+        m.prefill(toks, 0)
+        out = [m.read_buffer(which, cfg.kv_dim, 2, p) for which in (5, 6) for p in (0, 130, 299)]
+        m.batch_create(3, 64)
+        for p in range(3):
+            out.append(m.batch_forward([0, 1, 2], [p] * 3, [int(t) for t in toks[3 * p: 3 * p + 3]])[0])
+        assert m.stats().device_status == 0
+        m.close()
+        got.append(out)
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
 
 
 def test_full_batch_of_64_at_the_110m_shape():
