@@ -691,11 +691,6 @@ __global__ void pf_rope_kv_kernel(PfRopeParams p)
 // causal attention of the chunk's queries
 // ---------------------------------------------------------------------------------------------------------------
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-
 struct PfAttnParams {
     const float *q;        // [tokens][dim] after RoPE
     const float *k_cache, *v_cache;
@@ -1249,21 +1244,28 @@ int bd_splits(int heads, int nv, int sms)
 }
 
 // x after the last layer (with the partial row sums of its W2), RMSNorm with the final weights
-// (RootMeanSquare.java:25-35, WeightNormalizeAndScale.java:71-74): [64][dim] FP32 for the classifier.
-__global__ void __launch_bounds__(256) bd_final_norm_kernel(const float *x, const float *parts, int nparts, const float *w, int dim, int nvalid,
-                                                            float *out)
+// (RootMeanSquare.java:25-35, WeightNormalizeAndScale.java:71-74), written as three bf16 pieces [3][64][dim]: the
+// classifier's B operand.
+__global__ void __launch_bounds__(256) bd_final_norm_kernel(float *x, const float *parts, int nparts, const float *w, int dim, int nvalid,
+                                                            uint32_t *pieces)
 {
     __shared__ float s_red[8];
     const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_launch_dependents();
     pdl_wait();
     float ssq = 0.f;
-    for (int i = tid; i < dim; i += 256) {
-        float v = t < nvalid ? x[(size_t)t * dim + i] : 0.f;
-        for (int z = 0; z < nparts && t < nvalid; ++z)
-            v = __fadd_rn(v, parts[((size_t)z * kT + t) * dim + i]);
-        out[(size_t)t * dim + i] = v;
-        ssq = fmaf(v, v, ssq);
+    for (int i = tid; i < dim / 2; i += 256) {
+        float2 v = make_float2(0.f, 0.f);
+        if (t < nvalid)
+            v = reinterpret_cast<const float2 *>(x + (size_t)t * dim)[i];
+        for (int z = 0; z < nparts && t < nvalid; ++z) {
+            const float2 d = reinterpret_cast<const float2 *>(parts + ((size_t)z * kT + t) * dim)[i];
+            v.x = __fadd_rn(v.x, d.x);
+            v.y = __fadd_rn(v.y, d.y);
+        }
+        reinterpret_cast<float2 *>(x + (size_t)t * dim)[i] = v;
+        ssq = fmaf(v.x, v.x, ssq);
+        ssq = fmaf(v.y, v.y, ssq);
     }
     ssq = warp_sum(ssq);
     if (lane == 0)
@@ -1275,82 +1277,231 @@ __global__ void __launch_bounds__(256) bd_final_norm_kernel(const float *x, cons
     tot = __fdiv_rn(tot, (float)dim);
     tot = __fadd_rn(tot, 1e-5f);
     const float ss = __fdiv_rn(1.0f, __fsqrt_rn(tot));
-    for (int i = tid; i < dim; i += 256)
-        out[(size_t)t * dim + i] = __fmul_rn(w[i], __fmul_rn(ss, out[(size_t)t * dim + i]));
+    for (int i = tid; i < dim / 2; i += 256) {
+        const float2 v = reinterpret_cast<const float2 *>(x + (size_t)t * dim)[i], g = reinterpret_cast<const float2 *>(w)[i];
+        uint32_t pc[3];
+        split_bf16(__fmul_rn(g.x, __fmul_rn(ss, v.x)), __fmul_rn(g.y, __fmul_rn(ss, v.y)), pc);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            pieces[((size_t)k * kT + t) * (dim / 2) + i] = pc[k];
+    }
 }
 
-// logits[t][v] = sum_k wcls[v][k] * xn[t][k] for 64 tokens: FP32 on the CUDA cores (the classifier is not
-// quantised, TransformerWeights.java:25,41,122), 128 vocabulary rows x 64 tokens per block, K in chunks of 32
-// double-buffered with asynchronous copies, 8 rows x 4 tokens per thread.
-constexpr int kClsRows = 128, kClsK = 32, kClsLd = kClsK + 4, kClsThreads = 256;
-constexpr int kClsStage = (kClsRows + kT) * kClsLd;      // floats per stage
+// logits[t][v] = sum_k wcls[v][k] * xn[t][k] for 64 tokens (the classifier is not quantised,
+// TransformerWeights.java:25,41,122) on the tensor cores, FP32 operands in three bf16 pieces as in the attention above:
+// per 64 columns of K, W's leading pieces times all three of x (N 192), the second times two (N 128), the third times one
+// (N 64), into one accumulator per piece of x.  The accumulator starts anew every 64 columns and is added to the row sums
+// in FP32 registers, so that no long sum runs in the tensor cores.  Bound by the 4 bytes per weight from HBM (80 us at
+// 32000 x 4096); the FMA kernel before it was bound by its 16.8 GFLOP and made a step 0.29 to 0.38 ms longer.
+//
+//   warps 0-7    W from HBM through registers (two blocks of 64 columns ahead) into its pieces in shared memory
+//   warps 8-15   row sums: thread = vocabulary row, half of the tokens
+//   warp 16      tensor-core issue;  warp 17: copies of x's pieces (TMA)
+constexpr int kClsRows = 128, kClsCols = 64, kClsStages = 3, kClsCvt = 8, kClsEpi = 8;
+constexpr int kClsThreads = 32 * (kClsCvt + kClsEpi + 2);
+constexpr int kClsAPiece = kClsRows * 128, kClsABytes = 3 * kClsAPiece, kClsBBytes = kN * 128, kClsStage = kClsABytes + kClsBBytes;
 
-__global__ void __launch_bounds__(kClsThreads) bd_classifier_kernel(const float *wcls, const float *xn, int vocab, int dim, float *logits)
+struct BdClsParams {
+    const float *wcls;
+    int vocab, dim, nvalid;
+    float *logits;         // [64][vocab]
+    int timeout_us;
+    unsigned int *status;
+};
+
+__global__ void __launch_bounds__(kClsThreads, 1) bd_classifier_kernel(const __grid_constant__ CUtensorMap map_x, const BdClsParams p)
 {
-    extern __shared__ __align__(16) float cls_smem[];
-    const int tid = threadIdx.x, v0 = blockIdx.x * kClsRows;
+    extern __shared__ unsigned char cls_smem[];
+    __shared__ __align__(8) unsigned long long s_bar[3 * kClsStages + 5];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_give_up;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t base = (smem_u32(cls_smem) + 1023u) & ~1023u;
+    unsigned char *gen = cls_smem + (base - smem_u32(cls_smem));
+    const uint32_t b_full = smem_u32(&s_bar[0]), b_empty = smem_u32(&s_bar[kClsStages]), b_x = smem_u32(&s_bar[2 * kClsStages]),
+                   b_acc = smem_u32(&s_bar[3 * kClsStages]), b_free = b_acc + 16, b_fin = b_acc + 32;
+    const long long limit = 2000ll * (long long)p.timeout_us;
+    volatile int *give_up = &s_give_up;
+    const int tiles = (p.vocab + kClsRows - 1) / kClsRows, nk = p.dim / kClsCols;
+    const int total = ((tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * nk;   // blocks of columns of all the tiles
+
+    if (tid == 0) {
+        for (int s = 0; s < kClsStages; ++s) {
+            mbar_init(b_full + 8 * s, kClsCvt);
+            mbar_init(b_x + 8 * s, 1);
+            mbar_init(b_empty + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(b_acc + 8 * b, 1);
+            mbar_init(b_free + 8 * b, kClsEpi);
+        }
+        mbar_init(b_fin, 1);
+        mbar_fence_init();
+        s_give_up = 0;
+    }
     pdl_launch_dependents();
-    pdl_wait();
-    const int rg = tid >> 4, tg = tid & 15;          // rows rg + 16 i (i < 8), tokens tg + 16 j (j < 4)
-    float acc[8][4];
+    __syncthreads();
+
+    if (warp < kClsCvt) {
+        // unit: eight columns of a row; a row's 64 columns are 256 contiguous bytes
+        float4 x[2][4][2];
+        auto load = [&](int it, float4 (&d)[4][2]) {
+            const int tile = (int)blockIdx.x + it / nk * (int)gridDim.x, k0 = it % nk * kClsCols;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < 4; ++i) {
+                const int u = tid + 256 * i, v = tile * kClsRows + (u >> 3);
+                d[i][0] = d[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (v < p.vocab) {
+                    const float4 *src = reinterpret_cast<const float4 *>(p.wcls + (size_t)v * p.dim + k0 + 8 * (u & 7));
+                    d[i][0] = __ldcs(src);
+                    d[i][1] = __ldcs(src + 1);
+                }
+            }
+        };
+        auto store = [&](int it, const float4 (&d)[4][2]) -> bool {
+            const int s = it % kClsStages;
+            if (!__all_sync(0xffffffffu, pf_wait(b_empty + 8 * s, (uint32_t)((it / kClsStages) & 1) ^ 1u, give_up, limit)))
+                return false;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            acc[i][j] = 0.f;
-    auto load_stage = [&](int st, int k0) {
-        float *sw = cls_smem + st * kClsStage, *sx = sw + kClsRows * kClsLd;
-        for (int i = tid; i < (kClsRows + kT) * (kClsK / 4); i += kClsThreads) {
-            const int r = i / (kClsK / 4), c = i % (kClsK / 4);
-            if (r < kClsRows) {
-                const int v = min(v0 + r, vocab - 1);
-                cp_async16(smem_u32(sw + r * kClsLd + c * 4), wcls + (size_t)v * dim + k0 + c * 4);
-            } else {
-                cp_async16(smem_u32(sx + (r - kClsRows) * kClsLd + c * 4), xn + (size_t)(r - kClsRows) * dim + k0 + c * 4);
+            for (int i = 0; i < 4; ++i) {
+                const int u = tid + 256 * i;
+                const float v[8] = {d[i][0].x, d[i][0].y, d[i][0].z, d[i][0].w, d[i][1].x, d[i][1].y, d[i][1].z, d[i][1].w};
+                store_pieces(gen + (size_t)s * kClsStage, kClsAPiece, u >> 3, u & 7, v);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(b_full + 8 * s);
+            return true;
+        };
+        // the weights do not depend on the kernel in front: no wait for it here
+        if (total > 0)
+            load(0, x[0]);
+        if (total > 1)
+            load(1, x[1]);
+        for (int it = 0; it < total; it += 2) {
+            if (!store(it, x[0]))
+                break;
+            if (it + 2 < total)
+                load(it + 2, x[0]);
+            if (it + 1 < total) {
+                if (!store(it + 1, x[1]))
+                    break;
+                if (it + 3 < total)
+                    load(it + 3, x[1]);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    const int nk = dim / kClsK;
-    load_stage(0, 0);
-    for (int kc = 0; kc < nk; ++kc) {
-        if (kc + 1 < nk) {
-            load_stage((kc + 1) & 1, (kc + 1) * kClsK);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const float *sw = cls_smem + (kc & 1) * kClsStage, *sx = sw + kClsRows * kClsLd;
-#pragma unroll
-        for (int k = 0; k < kClsK; k += 4) {
-            float4 wv[8], xv[4];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                wv[i] = *reinterpret_cast<const float4 *>(sw + (rg + 16 * i) * kClsLd + k);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                xv[j] = *reinterpret_cast<const float4 *>(sx + (tg + 16 * j) * kClsLd + k);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc[i][j] = fmaf(wv[i].x, xv[j].x, acc[i][j]);
-                    acc[i][j] = fmaf(wv[i].y, xv[j].y, acc[i][j]);
-                    acc[i][j] = fmaf(wv[i].z, xv[j].z, acc[i][j]);
-                    acc[i][j] = fmaf(wv[i].w, xv[j].w, acc[i][j]);
+        pdl_wait();
+    } else if (warp == kClsCvt + kClsEpi + 1) {
+        pdl_wait();
+        if (lane == 0) {
+            int it = 0;
+            for (; it < total; ++it) {
+                const int s = it % kClsStages;
+                if (!pf_wait(b_empty + 8 * s, (uint32_t)((it / kClsStages) & 1) ^ 1u, give_up, limit))
+                    break;
+                mbar_arrive_expect_tx(b_x + 8 * s, kClsBBytes);
+                tma_load_2d(base + (uint32_t)(s * kClsStage + kClsABytes), &map_x, it % nk * 128, 0, b_x + 8 * s);
+            }
+            if (*give_up) {
+                // copies that nobody consumed must land before the block's shared memory goes away
+                for (int i = max(0, it - kClsStages); i < it; ++i) {
+                    const long long c0 = sm_clock();
+                    while (!mbar_try_wait(b_x + 8 * (i % kClsStages), (uint32_t)((i / kClsStages) & 1)) && sm_clock() - c0 < limit) {
+                    }
                 }
+            }
         }
-        __syncthreads();
-    }
+    } else if (warp == kClsCvt + kClsEpi) {
+        pdl_wait();
+        tmem_alloc(smem_u32(&s_tmem), kTmemCols);
+        tmem_relinquish();
+        tc_fence_before();
+        named_barrier_sync(1, 32 * (kClsEpi + 1));
+        tc_fence_after();
+        const uint32_t tmem = s_tmem;
+        if (lane == 0) {
+            bool ok = true;
+            for (int it = 0; it < total; ++it) {
+                const int s = it % kClsStages, b = it & 1;
+                ok = pf_wait(b_free + 8 * b, (uint32_t)((it >> 1) & 1) ^ 1u, give_up, limit) &&
+                     pf_wait(b_full + 8 * s, (uint32_t)((it / kClsStages) & 1), give_up, limit) &&
+                     pf_wait(b_x + 8 * s, (uint32_t)((it / kClsStages) & 1), give_up, limit);
+                if (!ok)
+                    break;
+                tc_fence_after();
+                const uint32_t ta = base + (uint32_t)(s * kClsStage), tb = ta + kClsABytes, d = tmem + (uint32_t)b * kAccCols;
+                // columns 64 i .. 64 i + 63 of the accumulator belong to piece i of x; the first instruction starts all of them
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int v = v0 + rg + 16 * i;
-        if (v < vocab)
+                for (int kk = 0; kk < kClsCols / 16; ++kk)
+                    umma_bf16(d, smem_desc_sw128(ta + kk * 32u), smem_desc_sw128(tb + kk * 32u), attn_idesc(kN), kk ? 1u : 0u);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                logits[(size_t)(tg + 16 * j) * vocab + v] = acc[i][j];
+                for (int kk = 0; kk < kClsCols / 16; ++kk) {
+                    umma_bf16(d, smem_desc_sw128(ta + kClsAPiece + kk * 32u), smem_desc_sw128(tb + kk * 32u), attn_idesc(2 * kT), 1u);
+                    umma_bf16(d, smem_desc_sw128(ta + 2 * kClsAPiece + kk * 32u), smem_desc_sw128(tb + kk * 32u), attn_idesc(kT), 1u);
+                }
+                umma_commit(b_empty + 8 * s);
+                umma_commit(b_acc + 8 * b);
+            }
+            if (!ok || *give_up) {
+                umma_commit(b_fin);
+                const long long c0 = sm_clock();
+                while (!mbar_try_wait(b_fin, 0) && sm_clock() - c0 < limit) {
+                }
+            }
+        }
+    } else {
+        pdl_wait();
+        named_barrier_sync(1, 32 * (kClsEpi + 1));
+        tc_fence_after();
+        const int quarter = warp & 3, th = (warp - kClsCvt) >> 2;
+        const uint32_t trow = s_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(th * kTH);
+        float acc[kTH];
+#pragma unroll
+        for (int t = 0; t < kTH; ++t)
+            acc[t] = 0.f;
+        for (int it = 0; it < total; ++it) {
+            const int b = it & 1;
+            if (!__all_sync(0xffffffffu, pf_wait(b_acc + 8 * b, (uint32_t)((it >> 1) & 1), give_up, limit)))
+                break;
+            tc_fence_after();
+            const uint32_t tacc = trow + (uint32_t)b * kAccCols;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t s0[16], s1[16], s2[16];
+                tmem_ld16(tacc + 16 * half, s0);
+                tmem_ld16(tacc + kT + 16 * half, s1);
+                tmem_ld16(tacc + 2 * kT + 16 * half, s2);
+                tmem_ld_wait();
+                if (half == 1) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(b_free + 8 * b);
+                }
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                    acc[16 * half + k] += __uint_as_float(s0[k]) + (__uint_as_float(s1[k]) + __uint_as_float(s2[k]));
+            }
+            if (it % nk == nk - 1) {
+                const int v = ((int)blockIdx.x + it / nk * (int)gridDim.x) * kClsRows + quarter * 32 + lane;
+                float *o = p.logits + (size_t)th * kTH * p.vocab + v;
+#pragma unroll
+                for (int t = 0; t < kTH; ++t) {
+                    if (v < p.vocab && th * kTH + t < p.nvalid)
+                        o[(size_t)t * p.vocab] = acc[t];
+                    acc[t] = 0.f;
+                }
+            }
+        }
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == kClsCvt + kClsEpi)
+        tmem_dealloc(s_tmem, kTmemCols);
+    if (tid == 0 && s_give_up)
+        atomicOr(p.status, PF_DS_WAIT_TIMEOUT);
 }
 
 // First maximum of every token's logits (Sampler.java:46-57).
@@ -1451,7 +1602,9 @@ struct Prefill {
     int n_seq = 0, seq_len_b = 0;
     float *bkc = nullptr, *bvc = nullptr;      // [sequence][layer][kv_head][seq_len_b][head]
     int *meta = nullptr;                       // device: tokens[64], positions[64], sequences[64], arg-max[64]
-    float *xn = nullptr, *logits = nullptr;    // [64][dim], [64][vocab]
+    uint32_t *xn = nullptr;                    // [3][64][dim] bf16: the classifier's input in three pieces
+    CUtensorMap map_xn;
+    float *logits = nullptr;                   // [64][vocab]
     int *meta_host = nullptr;                  // pinned, 4 x 64
     float *logits_host = nullptr;              // pinned, [64][vocab]
     std::map<int, cudaGraphExec_t> step_graphs; // captured step per entry count
@@ -1773,11 +1926,13 @@ cudaError_t prefill_batch_create(Prefill *pf, int n_seq, int seq_len)
     PF_CK(pf_alloc(pf, &pf->bvc, per_seq * n_seq));
     if (!pf->meta) {
         PF_CK(pf_alloc(pf, &pf->meta, (size_t)4 * kT));
-        PF_CK(pf_alloc(pf, &pf->xn, (size_t)kT * m.dim));
+        PF_CK(pf_alloc(pf, &pf->xn, (size_t)kN * m.dim / 2));
+        if (!encode_bytes_2d(&pf->map_xn, pf->xn, kN, 2 * m.dim, kN, false))
+            return cudaErrorNotSupported;
         PF_CK(pf_alloc(pf, &pf->logits, (size_t)kT * m.vocab));
         PF_CK(cudaHostAlloc(reinterpret_cast<void **>(&pf->meta_host), sizeof(int) * 4 * kT, cudaHostAllocDefault));
         PF_CK(cudaHostAlloc(reinterpret_cast<void **>(&pf->logits_host), sizeof(float) * (size_t)kT * m.vocab, cudaHostAllocDefault));
-        PF_CK(cudaFuncSetAttribute(bd_classifier_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * kClsStage * sizeof(float))));
+        PF_CK(cudaFuncSetAttribute(bd_classifier_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClsStages * kClsStage + 1024));
     }
     pf->n_seq = n_seq;
     pf->seq_len_b = seq_len;
@@ -1848,8 +2003,14 @@ static cudaError_t batch_enqueue(Prefill *pf, cudaStream_t st, int nv)
         pending = ks.w2;
     }
     PF_CK(launch(pf, st, bd_final_norm_kernel, dim3((unsigned)kT), 256, 0, pf->x, pf->parts, pending, m.rms_final, dim, nv, pf->xn));
-    PF_CK(launch(pf, st, bd_classifier_kernel, dim3((unsigned)((m.vocab + kClsRows - 1) / kClsRows)), kClsThreads, 2 * kClsStage * sizeof(float),
-                 m.wcls, pf->xn, m.vocab, dim, pf->logits));
+    {
+        BdClsParams c{};
+        c.wcls = m.wcls; c.vocab = m.vocab; c.dim = dim; c.nvalid = nv; c.logits = pf->logits;
+        c.timeout_us = m.timeout_us; c.status = m.status;
+        const int tiles = (m.vocab + kClsRows - 1) / kClsRows;
+        PF_CK(launch(pf, st, bd_classifier_kernel, dim3((unsigned)(tiles < pf->sms ? tiles : pf->sms)), kClsThreads,
+                     (size_t)(kClsStages * kClsStage + 1024), pf->map_xn, c));
+    }
     PF_CK(launch(pf, st, bd_argmax_kernel, dim3((unsigned)nv), 256, 0, pf->logits, m.vocab, nv, d_arg));
     PF_CK(cudaMemcpyAsync(pf->meta_host + 3 * kT, d_arg, sizeof(int) * kT, cudaMemcpyDeviceToHost, st));
     return cudaSuccess;

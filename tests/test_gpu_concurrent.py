@@ -116,6 +116,23 @@ def test_overlapped_launches_change_nothing(heads):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("vocab, entries", [(127, 1), (128, 2), (129, 33), (1000, 64), (19200, 31)])
+def test_classifier_of_a_step(vocab, entries):
+    """Vocabularies beside the 128-row tiles, one tile and more tiles than SMs, token counts beside the 32-token halves,
+    against the decode path's classifier."""
+    cfg = ModelConfig(512, 1280, 1, 8, 8, vocab, 64, False)
+    tensors = _tensors(cfg, 25)
+    toks = np.random.default_rng(26).integers(0, vocab, entries).astype(np.int32)
+    m = _build(cfg, tensors)
+    m.batch_create(entries, 8)
+    logits, am = m.batch_forward(np.arange(entries), np.zeros(entries, dtype=np.int32), toks)
+    assert np.array_equal(am, logits.argmax(axis=1))
+    for i, t in enumerate(toks):
+        _check(logits[i], m.forward(int(t), 0)[0])
+    assert m.stats().device_status == 0
+    m.close()
+
+
 def test_full_batch_of_64_at_the_110m_shape():
     cfg = syn.SHAPES["stories110M"]
     tensors = _tensors(cfg, 13)
