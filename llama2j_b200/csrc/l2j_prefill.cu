@@ -46,7 +46,7 @@ constexpr int kTB = 4;                      // token blocks per chunk of a promp
                                             // 7B shape take 144 instead of 214 ms
 constexpr int kN = 3 * kT;                  // columns of the B operand: three limbs per token
 constexpr int kTileM = 128;                 // weight rows per tile
-constexpr int kGemmThreads = 384;          // producer warp, issue warp, two spare, eight epilogue warps
+constexpr int kGemmThreads = 384;          // A producer, two issue warps, B producer, eight epilogue warps
 constexpr int kEpiWarps = 8;                // warps 4..11: quarter of tensor memory = warp % 4, half of the tokens = (warp - 4) / 4
 constexpr int kTH = kT / 2;                 // tokens per epilogue thread
 constexpr int kStages = 4;                  // ring depth, a power of two known at compile time: the two single-lane issue
@@ -207,7 +207,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
                const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b, const PfGemmParams p)
 {
     extern __shared__ unsigned char pf_smem_raw[];
-    __shared__ __align__(8) unsigned long long s_bar[2 * kMaxStages + 4 + 1];
+    __shared__ __align__(8) unsigned long long s_bar[2 * kMaxStages + 4 + 2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_give_up;
     __shared__ float s_ss[kT];
@@ -232,7 +232,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_full + 8 * s, 2);            // both producers
             mbar_init(bar_empty + 8 * s, 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -240,6 +240,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
             mbar_init(bar_acc_empty + 8 * b, kEpiWarps);
         }
         mbar_init(bar_fin, 1);
+        mbar_init(bar_fin + 8, 1);
         mbar_fence_init();
         s_give_up = 0;
     }
@@ -262,7 +263,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         const int g0 = (first % p.ksplit) * gper, g1 = min(G, g0 + gper);
         primed = max(0, min(kStages, 2 * (g1 - g0)));
         for (int s = 0; s < primed; ++s) {
-            mbar_arrive_expect_tx(bar_full + 8 * s, kStageBytes);
+            mbar_arrive_expect_tx(bar_full + 8 * s, kABytes);
             tma_load_2d_hint(base + (uint32_t)s * kStageBytes, ma, (2 * g0 + s) * 128, m0, bar_full + 8 * s, policy_evict_first());
         }
     }
@@ -295,76 +296,84 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
     const uint32_t tmem = s_tmem;
     volatile int *give_up = &s_give_up;
 
-    if (warp == 0) {
-        // ---- producer: one lane feeds the ring
+    if (warp == 0 || warp == 3) {
+        // ---- producers: one lane feeds the weights to the ring, one the activations.  A wait and the issue of a copy take a
+        // few hundred cycles, and a stage is used up in 500: one lane for both was as slow as everything else together.
+        const bool weights = warp == 0;
         if (lane == 0) {
             const uint64_t pol = policy_evict_first();
-            long it = 0;
+            int it = 0, s = 0;
+            uint32_t ph = 1;
             for (int tile = first; tile < ntiles && !*give_up; tile += stride) {
                 int m0;
                 const CUtensorMap *ma = tile_map(tile, m0);
                 const int g0 = (tile % p.ksplit) * gper, g1 = min(G, g0 + gper);
                 for (int hs = 2 * g0; hs < 2 * g1; ++hs, ++it) {   // half groups
-                    const int s = (int)(it % kStages);
                     const uint32_t st = base + (uint32_t)s * kStageBytes;
-                    if (it >= primed) {
-                        const uint32_t ph = (uint32_t)((it / kStages) & 1);
-                        if (!pf_wait(bar_empty + 8 * s, ph ^ 1u, give_up, limit))
+                    if (!weights || it >= primed) {
+                        if (!pf_wait(bar_empty + 8 * s, ph, give_up, limit))
                             break;
-                        mbar_arrive_expect_tx(bar_full + 8 * s, kStageBytes);
-                        tma_load_2d_hint(st, ma, hs * 128, m0, bar_full + 8 * s, pol);
+                        mbar_arrive_expect_tx(bar_full + 8 * s, weights ? kABytes : kBBytes);
+                        if (weights)
+                            tma_load_2d_hint(st, ma, hs * 128, m0, bar_full + 8 * s, pol);
+                        else
+                            tma_load_2d(st + kABytes, &map_b, hs * 128, tb * kN, bar_full + 8 * s);
                     }
-                    tma_load_2d(st + kABytes, &map_b, hs * 128, tb * kN, bar_full + 8 * s);
+                    if (++s == kStages) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
             }
             if (*give_up) {
                 // copies that nobody consumed must land before the block's shared memory goes away
-                for (int s = 0; s < kStages; ++s)
-                    for (uint32_t ph = 0; ph < 2; ++ph) {
+                for (int i = 0; i < kStages; ++i)
+                    for (uint32_t q = 0; q < 2; ++q) {
                         const long long c0 = sm_clock();
-                        while (!mbar_try_wait(bar_full + 8 * s, ph) && sm_clock() - c0 < limit) {
+                        while (!mbar_try_wait(bar_full + 8 * i, q) && sm_clock() - c0 < limit) {
                         }
                     }
             }
         }
-    } else if (warp == 1) {
-        // ---- tensor-core issue: one lane
+    } else if (warp <= 2) {
+        // ---- tensor-core issue: one lane of each of two warps, which take the groups (and the accumulators) in turn.  The
+        // issue of a group's eight instructions takes as long as the tensor cores need for them (900 cycles), and the waits,
+        // fences and commits around it as long again: with one lane the tensor cores idled through the latter.  With this
+        // and two producer lanes 256 tokens through 16 layers of the 7B shape take 3.83 instead of 4.17 ms.
         if (lane == 0) {
-            long it = 0;
-            bool ok = true;
-            for (int tile = first; tile < ntiles && ok; tile += stride) {
-                const int g0 = (tile % p.ksplit) * gper, g1 = min(G, g0 + gper);
-                for (int g = g0; g < g1 && ok; ++g, ++it) {
-                    const int b = (int)(it & 1);
-                    const uint32_t pha = (uint32_t)((it >> 1) & 1);
-                    if (!pf_wait(bar_acc_empty + 8 * b, pha ^ 1u, give_up, limit)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t d = tmem + (uint32_t)b * kAccCols;
-                    for (int half = 0; half < 2; ++half) {
-                        const long hit = 2 * it + half;
-                        const int s = (int)(hit % kStages);
-                        if (!pf_wait(bar_full + 8 * s, (uint32_t)((hit / kStages) & 1), give_up, limit)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t ta = base + (uint32_t)s * kStageBytes, tb = ta + kABytes;
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            umma_i8(d, smem_desc_sw128(ta + (uint32_t)kk * 32u), smem_desc_sw128(tb + (uint32_t)kk * 32u), kIdesc,
-                                    (half | kk) ? 1u : 0u);
-                        umma_commit(bar_empty + 8 * s);        // the stage may be refilled when these have read it
-                    }
-                    if (ok)
-                        umma_commit(bar_acc_full + 8 * b);     // the group's sums are complete
-                }
+            const int b = warp - 1;
+            static_assert(kStages == 4, "a group's two stages are 2 b and 2 b + 1");
+            int mine = 0;                        // groups of the block that are this lane's: every second one
+            for (int tile = first; tile < ntiles; tile += stride) {
+                const int g0 = (tile % p.ksplit) * gper;
+                mine += max(0, min(G, g0 + gper) - g0);
             }
-            if (!ok) {
-                umma_commit(bar_fin);
+            mine = (mine + 1 - b) / 2;
+            bool ok = true;
+            uint32_t ph = 0;
+            const uint32_t d = tmem + (uint32_t)b * kAccCols, ta = base + (uint32_t)(2 * b) * kStageBytes;
+            for (; mine > 0 && ok; --mine, ph ^= 1u) {
+                ok = pf_wait(bar_acc_empty + 8 * b, ph ^ 1u, give_up, limit);
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    ok = ok && pf_wait(bar_full + 8 * (2 * b + half), ph, give_up, limit);
+                    if (!ok)
+                        break;
+                    tc_fence_after();
+                    const uint32_t t = ta + (uint32_t)half * kStageBytes;
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_i8(d, smem_desc_sw128(t + (uint32_t)kk * 32u), smem_desc_sw128(t + kABytes + (uint32_t)kk * 32u), kIdesc,
+                                (half | kk) ? 1u : 0u);
+                    umma_commit(bar_empty + 8 * (2 * b + half));     // the stage may be refilled when these have read it
+                }
+                if (ok)
+                    umma_commit(bar_acc_full + 8 * b);               // the group's sums are complete
+            }
+            if (!ok || *give_up) {
+                umma_commit(bar_fin + 8 * b);
                 const long long c0 = sm_clock();
-                while (!mbar_try_wait(bar_fin, 0) && sm_clock() - c0 < limit) {
+                while (!mbar_try_wait(bar_fin + 8 * b, 0) && sm_clock() - c0 < limit) {
                 }
             }
         }
