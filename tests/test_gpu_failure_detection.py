@@ -129,3 +129,25 @@ def test_duplicate_part_cannot_stand_in_for_a_missing_one():
     lg, _ = m.forward(1, 0)
     assert np.isfinite(lg).all()
     m.close()
+
+
+def test_small_shapes_wait_for_whole_kernels_until_a_failure_is_injected():
+    """A small shape without flags takes dependency waits instead of the hand-over counters: the same bits as with them, and
+    l2j_debug_desync puts it on the counters first, so that the injected failure is reported and a reset recovers."""
+    cfg = ModelConfig(dim=768, hidden_dim=2048, n_layers=2, n_heads=12, n_kv_heads=4, vocab_size=1000, seq_len=64,
+                      shared_classifier=True)
+    tensors = syn.synthetic_tensors(cfg, 5)
+    counters = _build(cfg, tensors, L.F_STEP_KERNELS)
+    plain = _build(cfg, tensors, limit_us=500)
+    good = [counters.forward(t, p)[0].copy() for p, t in enumerate((1, 17, 400))]
+    for p, t in enumerate((1, 17, 400)):
+        assert np.array_equal(plain.forward(t, p)[0], good[p])
+    plain.debug_desync()
+    with pytest.raises(L.L2jError) as e:
+        plain.forward(1, 0)
+    assert e.value.code == L.E_DEVICE
+    plain.reset()
+    for p, t in enumerate((1, 17, 400)):
+        assert np.array_equal(plain.forward(t, p)[0], good[p])
+    counters.close()
+    plain.close()
