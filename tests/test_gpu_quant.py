@@ -56,3 +56,15 @@ def test_synthetic_checkpoint_equals_oracle_checkpoint(oracle, l2j):
     assert sorted(a) == sorted(b)
     for t in a:
         assert np.array_equal(a[t].view(np.uint8), b[t].view(np.uint8)), t
+
+
+@pytest.mark.parametrize("extra", [0, 1, 257, 262144, 262145 + 256])
+def test_large_arrays_through_the_staging_buffers(extra, l2j):
+    """4 Mi floats and more go through pinned buffers on several threads: the bytes of the same floats sent in parts that
+    are too short for that, around the ends of the pieces (262144 floats) and groups (256)."""
+    n = (1 << 22) + extra
+    values = np.random.default_rng(extra).normal(0, 0.02, n).astype(np.float32)
+    whole = syn.quant_encode(values)
+    part = 1 << 20
+    pieces = [syn.quant_encode(values[i: i + part]) for i in range(0, n, part)]
+    assert np.array_equal(whole, np.concatenate(pieces))
