@@ -44,7 +44,8 @@ namespace cg = cooperative_groups;
 constexpr int kSampThreads = 1024, kSampWarps = kSampThreads / 32;
 constexpr int kSampCtas = 8;                       // blocks of the cluster (the portable maximum)
 constexpr int kSampRows = 5;                       // elements per thread of a block's share of the vocabulary
-constexpr int kSampMaxVocab = kSampCtas * kSampRows * kSampThreads;
+constexpr int kSampMaxVocab = 39936;               // what the entry point takes
+static_assert(kSampMaxVocab <= kSampCtas * kSampRows * kSampThreads, "every element has a thread");
 constexpr int kDigitBits = 8, kDigits = 1 << kDigitBits;
 constexpr int kHistBytes = kDigits * kSampWarps * 2;
 constexpr int kSegRows = kSampRows;                // rows of 32 elements per warp in the local sort

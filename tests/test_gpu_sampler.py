@@ -165,3 +165,20 @@ def test_command_line_loop_with_temperature(oracle, tmp_path, monkeypatch, capsy
     m.close()
     assert got == want
     assert len(set(want)) > 4
+
+
+@pytest.mark.parametrize("vocab, taken", [(39936, True), (39937, False)])
+def test_largest_vocabulary(vocab, taken):
+    """The bound of the entry point: probabilities of at most 39936 tokens."""
+    cfg = ModelConfig(256, 768, 1, 4, 4, vocab, 16, True)
+    m = Transformer(cfg)
+    m.upload_all(syn.synthetic_tensors(cfg, 3))
+    m.finalize()
+    m.forward(1, 0, want_logits=False)
+    if taken:
+        m.sampler_seed(7)
+        assert 0 <= m.sample(0.9, 0.9) < vocab
+    else:
+        with pytest.raises(L.L2jError):
+            m.sampler_seed(7)
+    m.close()
