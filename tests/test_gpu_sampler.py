@@ -74,7 +74,7 @@ def test_changing_candidate_counts(model, oracle):
     assert got == want
 
 
-@pytest.mark.parametrize("vocab,scale", [(2, 0.02), (9, 1.0), (300, 0.5), (4097, 0.05), (8193, 0.02), (40960, 0.3)])
+@pytest.mark.parametrize("vocab,scale", [(2, 0.02), (9, 1.0), (300, 0.5), (4097, 0.05), (8193, 0.02), (39936, 0.3)])
 def test_vocabulary_sizes(oracle, vocab, scale):
     """Shares of the cluster's blocks that are empty, ragged or full, flat and peaked distributions, and equal
     probabilities (pairs of equal classifier rows) in both the candidates and what earlier calls left behind them."""
