@@ -14,7 +14,7 @@
 //                       token) unit and sum; input is RMSNorm(x) * w, the attention output, or SwiGLU(h1, h3)
 //   pf_gemm_kernel      C[64 tokens][rows] (+)= W[rows][K] x limbs: TMA (cp.async.bulk.tensor) feeds 128-byte-
 //                       swizzled tiles to tcgen05.mma kind::i8 (u8 x s8 -> s32, M 128, N 192, K 32), one
-//                       accumulator per quantisation group in tensor memory, double-buffered; four epilogue warps
+//                       accumulator per quantisation group in tensor memory, double-buffered; eight epilogue warps
 //                       read it back (tcgen05.ld), scale in FP32 and keep the row sums in registers
 //   pf_rope_kv_kernel   RoPE on q and k, rows of the K/V cache (ApplyRope.java:61-92, Run.java:443-455)
 //   pf_attention_kernel causal attention of the chunk's queries over the cache: FP32 operands in three bf16 pieces on
@@ -723,7 +723,8 @@ struct PfAttnParams {
 //   warp 12      issue: S(j + 1) = Q K' while the softmax works on tile j, then O(j) = P V
 //
 // Six bf16 products of 128 x 64 x HEAD, twice per tile, are 3072 tensor-core cycles at head size 128; on the FP32 units
-// the same tile takes 16384 cycles at best.  3840 tokens through 16 layers of the 7B shape: 144 ms with the FP32 kernel
+// the same tile takes 16384 cycles at best.  A tile takes 8000, 6900 of them the issue of its 72 instructions (48 wider
+// ones took as long).  3840 tokens through 16 layers of the 7B shape: 144 ms with the FP32 kernel
 // before this one (4 x 4 scores per thread), 88 ms with it.  Error against float64 the same or lower (3.4e-6 against 3.6e-6
 // of a row of V behind it, mean over head sizes 64 and 128 and peaked softmaxes).
 constexpr int kAttnQ = 128;      // queries per block: the rows of one accumulator
@@ -1304,8 +1305,8 @@ __global__ void __launch_bounds__(256) bd_final_norm_kernel(float *x, const floa
 // TransformerWeights.java:25,41,122) on the tensor cores, FP32 operands in three bf16 pieces as in the attention above:
 // per 64 columns of K, W's leading pieces times all three of x (N 192), the second times two (N 128), the third times one
 // (N 64), into one accumulator per piece of x.  The accumulator starts anew every 64 columns and is added to the row sums
-// in FP32 registers, so that no long sum runs in the tensor cores.  Bound by the 4 bytes per weight from HBM (80 us at
-// 32000 x 4096); the FMA kernel before it was bound by its 16.8 GFLOP and made a step 0.29 to 0.38 ms longer.
+// in FP32 registers, so that no long sum runs in the tensor cores.  The floor is the 4 bytes per weight from HBM (80 us at
+// 32000 x 4096; 167 us with cold caches: two tiles on two thirds of the SMs, one on the others); the FMA kernel before it was bound by its 16.8 GFLOP and made a step 0.29 to 0.38 ms longer.
 //
 //   warps 0-7    W from HBM through registers (two blocks of 64 columns ahead) into its pieces in shared memory
 //   warps 8-15   row sums: thread = vocabulary row, half of the tokens
