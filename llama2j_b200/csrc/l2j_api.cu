@@ -83,6 +83,7 @@ struct l2j_ctx {
     unsigned int *work = nullptr;   // two counters per ring-kernel launch of a forward
     unsigned int *chain = nullptr;  // hand-over counters, one per kernel of a forward, each on its own 128-byte line
     bool chain_on = true;
+    bool whole_waits = false;       // a small shape whose kernels wait for the whole kernel in front instead of its counter
     bool kv_prefetch = true;
     bool attn_cluster = true;       // one thread-block cluster per head in the attention kernel
     unsigned long long *trace = nullptr;   // per-launch timelines, only when L2J_TRACE is set
@@ -1063,8 +1064,10 @@ static int create_impl(const l2j_config *cfg, int device, int first_layer, int l
     // at 15M.  Where blocks end apart the counters win (7B shape 1862 -> 1853, 20 layers of 13B 1566 -> 1549).
     if (tp_size == 1 && c->use_ring && !c->use_fused && !(flags & (L2J_F_STEP_KERNELS | L2J_F_NO_PDL)) && !getenv("L2J_CHAIN")) {
         const int64_t layer = 2 * (int64_t)c->dim * (c->dim + c->kv_dim) + 3 * (int64_t)c->dim * c->hidden;
-        if (layer / 4 <= (int64_t)65536 * c->sm_count)
+        if (layer / 4 <= (int64_t)65536 * c->sm_count) {
             c->chain_on = false;
+            c->whole_waits = true;
+        }
     }
     CREATE_CUDA(cudaStreamSynchronize(c->stream));
     CREATE_CUDA(cudaDeviceSynchronize());
@@ -1969,7 +1972,8 @@ int check_tp_group(l2j_ctx *const *ranks, int n, bool need_link)
             return fail(c0, L2J_E_INVALID, "rank %d was created for another model", i);
         if (c->tp_size != n || c->tp_rank != i || !(c->is_first && c->is_last))
             return fail(c0, L2J_E_INVALID, "context %d is rank %d of %d, expected rank %d of %d", i, c->tp_rank, c->tp_size, i, n);
-        if (!c->use_ring || !c->chain_on)
+        // (a group of one hands nothing over, so a small shape may wait for whole kernels there)
+        if (!c->use_ring || !(c->chain_on || (n == 1 && c->whole_waits)))
             return fail(c0, L2J_E_STATE, "a tensor-parallel group needs the ring kernels and the hand-over counters");
         for (int j = 0; j < i; ++j)
             if (ranks[j]->device == c->device)
@@ -2201,7 +2205,7 @@ extern "C" int l2j_debug_desync(l2j_ctx *c)
     if (!c)
         return L2J_E_INVALID;
     std::lock_guard<std::mutex> lock(c->mu);
-    if (!c->finalized || !c->use_ring)
+    if (!c->finalized || !c->use_ring || !(c->chain_on || c->whole_waits))
         return fail(c, L2J_E_STATE, "needs a finalized context that runs the hand-over counters");
     CK(c, cudaSetDevice(c->device));
     CK(c, cudaStreamSynchronize(c->stream));

@@ -3,6 +3,8 @@ order of the single device's per-step kernels, so logits and greedy tokens must 
 running those kernels (the persistent kernel sums the attention partials in another order: close, not bitwise).  Ranks wait for each
 other inside their kernels (with a time limit) and therefore need a GPU each: the tests with more than
 one rank are skipped on a single GPU."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -50,6 +52,32 @@ def test_group_of_one_is_the_plain_context():
     cfg = syn.SHAPES["stories15M"]
     tensors = syn.synthetic_tensors(cfg, 0)
     _check_group(cfg, tensors, 1, steps=48, n_prompt=8)
+
+
+@pytest.mark.parametrize("flags", [0, L.F_STEP_KERNELS, L.F_NO_PDL, L.F_PERSISTENT])
+@pytest.mark.parametrize("dim, hidden", [(768, 2048), (2048, 5632)])     # whole-kernel waits without flags, persistent kernel without flags
+def test_any_whole_context_is_a_group_of_one(dim, hidden, flags):
+    """A group of one hands nothing over between ranks: whatever way its context takes through the layers, linked after
+    l2j_create as after l2j_create_tp, it is accepted and computes the context's own bits."""
+    cfg = ModelConfig(dim=dim, hidden_dim=hidden, n_layers=2, n_heads=dim // 64, n_kv_heads=dim // 64, vocab_size=1000,
+                      seq_len=64, shared_classifier=True)
+    tensors = syn.synthetic_tensors(cfg, 6)
+    prompt = syn.synthetic_prompt(6, 2, cfg.vocab_size)
+    plain, made = Transformer(cfg, flags=flags), Transformer(cfg, flags=flags)
+    made.close()
+    c = cfg.to_c()
+    L.check(L.load().l2j_create_tp(C.byref(c), 0, 0, 1, flags, C.byref(made._ctx)), None)
+    for m in (plain, made):
+        m.upload_all(tensors)
+        m.finalize()
+    want = [plain.forward(t, p)[0].copy() for p, t in enumerate((1, 17, 400))]
+    tokens = plain.generate_greedy(prompt, 24)
+    for m in (plain, made):
+        group = TensorParallel([m])
+        for p, t in enumerate((1, 17, 400)):
+            assert np.array_equal(group.forward(t, p)[0].view(np.uint32), want[p].view(np.uint32))
+        assert np.array_equal(group.generate_greedy(prompt, 24), tokens)
+        group.close()
 
 
 def test_two_ranks_stories15m_unaligned_rows():
