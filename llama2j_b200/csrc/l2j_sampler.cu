@@ -80,10 +80,11 @@ __device__ __forceinline__ Step step_then(const Step &f, const Step &g)
     return h;
 }
 
-// x: the element in ulps (exact: a power of two times the element)
+// x: the element in ulps (exact: a power of two times the element).  A NaN leaves the binade too: the element is then
+// added with an ordinary addition.
 __device__ __forceinline__ Step step_of(float x)
 {
-    if (x >= 33554432.0f)
+    if (!(x < 33554432.0f))
         return Step{1 << 25, 1 << 25};
     const int a = (int)x;
     const float f = x - (float)a;
@@ -100,21 +101,32 @@ struct ScanShared {
     int hit;         // element at which the sum exceeded the threshold, or -1
 };
 
+// The first of the four sums behind elements i .. i + 3 that exceeds the limit (-1: none), and that sum (else the last).
+// A later element that is NaN does not hide an earlier sum.
+__device__ __forceinline__ int first_above(const float4 &c, int i, float limit, float &sum)
+{
+    sum = c.x > limit ? c.x : (c.y > limit ? c.y : (c.z > limit ? c.z : c.w));
+    return c.x > limit ? i : (c.y > limit ? i + 1 : (c.z > limit ? i + 2 : (c.w > limit ? i + 3 : -1)));
+}
+
 // Adds v[0 .. n) in order to `sum` (block-wide; v in shared memory, 16-byte aligned, readable up to the next multiple
 // of four) and returns the first i with (sum after element i) > limit, or -1; `sum` becomes the sum behind that element
-// or behind all of them.  keep: the running sums replace the elements (up to the stop).
+// or behind all of them.  keep: the running sums replace the elements (up to the stop).  A sum that is NaN stays NaN and
+// exceeds nothing, so it ends the walk (nobody asks for the running sums then).
 __device__ int sequential_sum(float *v, int n, float &sum, float limit, bool keep, ScanShared &sh)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int i0 = 0, serial = kFirstSerial;
     while (i0 < n) {
-        if (i0 < serial || sum < 1e-30f) {
-            // the first elements (many binades in few steps), and sums so small that an element in ulps could overflow
+        if (sum != sum)
+            return -1;
+        if (i0 < serial || !(sum >= 1e-30f && sum < INFINITY)) {
+            // the first elements (many binades in few steps), sums so small that an element in ulps could overflow, infinity
             const int end = min(n, i0 + kFirstSerial);
             if (tid == 0) {
                 float s = sum;
                 int hit = -1;
-                for (int i = i0; i < end && hit < 0; i += 4) {
+                for (int i = i0; i < end && hit < 0 && s == s; i += 4) {
                     float4 x = *reinterpret_cast<const float4 *>(v + i);
                     x.x = __fadd_rn(s, x.x);
                     x.y = i + 1 < n ? __fadd_rn(x.x, x.y) : x.x;
@@ -123,10 +135,8 @@ __device__ int sequential_sum(float *v, int n, float &sum, float limit, bool kee
                     s = x.w;
                     if (keep)
                         *reinterpret_cast<float4 *>(v + i) = x;
-                    if (s > limit) {
-                        hit = x.x > limit ? i : (x.y > limit ? i + 1 : (x.z > limit ? i + 2 : i + 3));
-                        s = x.x > limit ? x.x : (x.y > limit ? x.y : (x.z > limit ? x.z : x.w));
-                    }
+                    if (!(s <= limit))
+                        hit = first_above(x, i, limit, s);
                 }
                 sh.sum = s;
                 sh.hit = hit;
@@ -207,11 +217,9 @@ __device__ int sequential_sum(float *v, int n, float &sum, float limit, bool kee
         __syncthreads();
         const int first = sh.first;
         if (tid == min(first, kSampThreads - 1)) {
-            int hit = -1;
-            if (c.w > limit)
-                hit = c.x > limit ? i : (c.y > limit ? i + 1 : (c.z > limit ? i + 2 : i + 3));
-            sh.sum = hit < 0 ? c.w : (c.x > limit ? c.x : (c.y > limit ? c.y : (c.z > limit ? c.z : c.w)));
-            sh.hit = hit;
+            float s;
+            sh.hit = first_above(c, i, limit, s);
+            sh.sum = s;
         }
         __syncthreads();
         sum = sh.sum;

@@ -182,3 +182,47 @@ def test_largest_vocabulary(vocab, taken):
         with pytest.raises(L.L2jError):
             m.sampler_seed(7)
     m.close()
+
+
+@pytest.mark.parametrize("topp", [1.0, 0.9])
+@pytest.mark.parametrize("bad", [[0], [255], [256], [3001], [31999], [5, 700], "all"])
+def test_logits_that_are_not_numbers(oracle, bad, topp):
+    """One NaN makes the reference's sum and with it every probability NaN: the plain walk ends at the last token, the
+    nucleus has no candidate (the reference leaves its array there; the device answers token 0).  NaN among the elements
+    added one by one (the first 256), in a scanned window, last, and everywhere."""
+    cfg = ModelConfig(64, 176, 1, 4, 4, 32000, 64, False)
+    tensors = syn.synthetic_tensors(cfg, 11)
+    wcls = np.random.default_rng(5).standard_normal((cfg.vocab_size, 64), dtype=np.float32)
+    wcls[slice(None) if bad == "all" else bad] = np.nan
+    tensors[L.T_WCLS] = wcls.reshape(-1)
+    m = Transformer(cfg)
+    m.upload_all(tensors)
+    m.finalize()
+    _not_a_number(m, oracle, 0.9, topp)
+    m.close()
+
+
+@pytest.mark.parametrize("topp", [1.0, 0.9])
+def test_temperature_that_overflows_the_logits(oracle, topp):
+    """logits / 1e-40 are infinite: infinity - infinity among the arguments of exp is NaN, as above."""
+    cfg = ModelConfig(64, 176, 1, 4, 4, 4097, 64, False)
+    m = Transformer(cfg)
+    m.upload_all(syn.synthetic_tensors(cfg, 11))
+    m.finalize()
+    _not_a_number(m, oracle, 1e-40, topp)
+    m.close()
+
+
+def _not_a_number(m, oracle, temperature, topp):
+    vocab = m.cfg.vocab_size
+    m.sampler_seed(3)
+    ref = oracle.Sampler(3, vocab)
+    for pos in range(3):
+        logits = m.forward(1 + pos, pos)[0].copy()
+        token = m.sample(temperature, topp)
+        assert np.isnan(m.read_buffer(4, vocab)).all()
+        # (the checker's nucleus walk has no answer without candidates)
+        assert token == (ref.sample(logits, temperature, topp) if topp > 0.999 else 0)
+        if topp > 0.999:
+            assert token == vocab - 1
+    ref.close()
