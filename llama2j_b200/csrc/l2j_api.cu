@@ -1594,7 +1594,7 @@ extern "C" int l2j_sampler_seed(l2j_ctx *c, int64_t seed)
         if (rc != L2J_OK)
             return rc;
         CK(c, cudaHostAlloc((void **)&c->samp_host, sizeof(SamplerState), cudaHostAllocDefault));
-        CK(c, prepare_sampler(n));
+        CK(c, prepare_sampler());
     }
     CK(c, cudaStreamSynchronize(c->stream));
     // new Sampler(seed, vocab): every ProbIndex is (0, 0), Random(seed) scrambles the seed (java.util.Random)

@@ -301,7 +301,7 @@ struct SampleParams {
 
 size_t sample_smem_bytes(int n);
 int sample_max_vocab(size_t smem_limit);   // largest vocabulary the sampler takes
-cudaError_t prepare_sampler(int n);
+cudaError_t prepare_sampler();
 cudaError_t launch_sample(cudaStream_t stream, const SampleParams &sp);
 
 struct MvPlan {

@@ -60,6 +60,7 @@ constexpr int kMaxParts = 12;               // parts a row sum (or a query's key
 constexpr int kWideParts = 3;               // at most this many parts for the wide outputs (W1/W3): their sums are read back
 constexpr int kAccCols = 256;               // column distance of the two accumulators in tensor memory
 constexpr int kTmemCols = 512;
+constexpr int kMaxDim = 16384;              // longest row of a matrix
 
 // ---- tcgen05 / TMA wrappers ----------------------------------------------------------------------------------
 
@@ -1629,7 +1630,7 @@ struct Prefill {
 bool prefill_supported(const PrefillModel &m)
 {
     const int kv_dim = m.n_kv_heads * m.head;
-    return m.dim % 256 == 0 && m.hidden % 256 == 0 && kv_dim % kTileM == 0 && m.dim <= 16384 && m.hidden <= 16384 &&
+    return m.dim % 256 == 0 && m.hidden % 256 == 0 && kv_dim % kTileM == 0 && m.dim <= kMaxDim && m.hidden <= kMaxDim &&
            (m.head == 64 || m.head == 128) && m.n_heads * m.head == m.dim && m.n_layers > 0;
 }
 
@@ -1702,7 +1703,9 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m)
     // ring, unit table (at most 64 groups: 32 KB), alignment slack: below the 227 KB a block may have
     pf->gemm_smem_dim = (size_t)kStages * kStageBytes + (size_t)(m.dim / 256) * kT * sizeof(float2) + 1024;
     pf->gemm_smem_hidden = (size_t)kStages * kStageBytes + (size_t)(m.hidden / 256) * kT * sizeof(float2) + 1024;
-    const size_t gmax = pf->gemm_smem_dim > pf->gemm_smem_hidden ? pf->gemm_smem_dim : pf->gemm_smem_hidden;
+    // (the limit belongs to the kernel on the device, not to this context: it covers every shape)
+    constexpr size_t gmax = (size_t)kStages * kStageBytes + (size_t)(kMaxDim / 256) * kT * sizeof(float2) + 1024;
+    static_assert(gmax <= 227 * 1024, "what a block may have");
     e = cudaFuncSetAttribute(pf_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gmax);
     pf->attn_smem = m.head == 128 ? attn_smem_bytes<128>() : attn_smem_bytes<64>();
     if (e == cudaSuccess)

@@ -575,9 +575,10 @@ int sample_max_vocab(size_t smem_limit)
     return n;
 }
 
-cudaError_t prepare_sampler(int n)
+// The limit belongs to the kernel on the device, whichever context asks for it: it is the same for all of them.
+cudaError_t prepare_sampler()
 {
-    return cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sample_smem_bytes(n));
+    return cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sample_smem_bytes(kSampMaxVocab));
 }
 
 cudaError_t launch_sample(cudaStream_t stream, const SampleParams &sp)

@@ -135,6 +135,32 @@ def test_prefill_attention_around_its_tiles(heads, kv_heads, first, more):
     pre.close()
 
 
+def test_a_smaller_shape_does_not_take_the_larger_ones_shared_memory():
+    """Two contexts of one device in turn: a long row and a large vocabulary, then short ones, then the first again."""
+    toks = np.random.default_rng(4).integers(3, 300, 70).astype(np.int32)
+    models = []
+    for hidden, vocab in ((5120, 30000), (512, 300)):
+        cfg = ModelConfig(512, hidden, 1, 4, 4, vocab, 128, True)
+        models.append(_build(cfg, _tensors(cfg, 10)))
+    rounds = []
+    for _ in range(2):
+        got = []
+        for m in models:
+            m.reset()
+            m.prefill(toks, 0)
+            got.append(m.forward(7, toks.size)[0].copy())
+            m.batch_create(2, 8)
+            got.append(m.batch_forward([0, 1], [0, 0], [5, 6])[0])
+            m.sampler_seed(1)
+            got.append(m.sample(0.9, 0.9))
+        rounds.append(got)
+    for a, b in zip(*rounds):
+        assert np.array_equal(a, b)
+    for m in models:
+        assert m.stats().device_status == 0
+        m.close()
+
+
 def test_prefill_then_decode_against_the_checker(oracle):
     """A 100-token prompt through l2j_prefill, then greedy decoding: logits of every decoded position within
     the north star's 1e-3 of range of the CPU checker that ran the whole sequence token by token."""
