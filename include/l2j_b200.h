@@ -269,6 +269,11 @@ L2J_API int l2j_set_wait_limit_us(l2j_ctx *ctx, int limit_us);
  * usable again.  Nothing faults: every wait gives up and the kernels return. */
 L2J_API int l2j_debug_desync(l2j_ctx *ctx);
 
+/* The same for allocations: the nth device or pinned allocation that the context makes from now on (prompt
+ * workspaces, caches of concurrent sequences, sampler: whatever is made on first use) fails as if memory had run
+ * out; 0 takes the injection back.  The call answers with an error and may be made again. */
+L2J_API int l2j_debug_fail_alloc(l2j_ctx *ctx, int nth);
+
 L2J_API int l2j_get_stats(l2j_ctx *ctx, l2j_stats *out);
 
 /* How the per-token work is issued: bit 0 CUDA graph replay, bit 1 programmatic dependent launch

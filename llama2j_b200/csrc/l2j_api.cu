@@ -61,6 +61,7 @@ struct l2j_ctx {
     std::vector<std::pair<int64_t, int64_t>> got[L2J_T_COUNT];
     Prefill *prefill = nullptr;            // batched prompt path, built on first use where the shape allows it
     bool prefill_tried = false;
+    int fail_alloc = 0;             // l2j_debug_fail_alloc: allocations until the one that fails
     SamplerState *samp_state = nullptr;   // device sampler (l2j_sampler_seed / l2j_sample), allocated on first use
     float *samp_prob[2] = {nullptr, nullptr};
     int *samp_index[2] = {nullptr, nullptr};
@@ -157,9 +158,11 @@ int dev_alloc(l2j_ctx *ctx, T **out, int64_t count, bool zero)
 {
     void *p = nullptr;
     const size_t bytes = (size_t)(count > 0 ? count : 1) * sizeof(T);
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess)
+    cudaError_t e = alloc_fails(&ctx->fail_alloc) ? cudaErrorMemoryAllocation : cudaMalloc(&p, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
         return fail(ctx, L2J_E_NOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+    }
     if (zero) {
         e = cudaMemset(p, 0, bytes);
         if (e != cudaSuccess) {
@@ -1438,6 +1441,7 @@ static PrefillModel prefill_model(l2j_ctx *c)
     m.rms_final = c->rms_final;
     m.status = reinterpret_cast<unsigned int *>(&c->state->status);
     m.timeout_us = c->wait_limit_us;
+    m.fail_alloc = &c->fail_alloc;
     m.pdl = !(c->flags & L2J_F_NO_PDL);
     auto payload = [](const MvSeg &s) { return s.payload + s.flat0; };
     auto hdr = [](const MvSeg &s) { return s.hdr + s.flat0 / kGroup; };
@@ -1460,14 +1464,22 @@ static PrefillModel prefill_model(l2j_ctx *c)
     return m;
 }
 
-// Builds the batched path of a whole-model context on first use; L2J_E_INVALID where the shape is outside it.
+// Builds the batched path of a whole-model context on first use; L2J_E_INVALID where the shape is outside it,
+// L2J_E_NOMEM (this call's, the next one tries again) where its workspaces do not fit.
 static int ensure_prefill(l2j_ctx *c, bool required)
 {
     if (!c->prefill_tried) {
-        c->prefill_tried = true;
         const PrefillModel m = prefill_model(c);
-        if (prefill_supported(m) && !(c->flags & L2J_F_NO_TENSOR_PREFILL))
-            CK(c, prefill_create(&c->prefill, m));
+        if (prefill_supported(m) && !(c->flags & L2J_F_NO_TENSOR_PREFILL)) {
+            const cudaError_t e = prefill_create(&c->prefill, m);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                return fail(c, L2J_E_NOMEM, "no device memory for the workspaces of the batched path");
+            }
+            c->prefill_tried = true;
+            CK(c, e);
+        }
+        c->prefill_tried = true;
     }
     if (required && !c->prefill)
         return fail(c, L2J_E_INVALID, "the batched path needs rows of whole quantisation groups and a head size of 64 or 128");
@@ -1493,10 +1505,15 @@ extern "C" int l2j_prefill(l2j_ctx *c, const int32_t *tokens, int n, int pos0)
             return L2J_OK;
         CK(c, cudaSetDevice(c->device));
         const int rc = ensure_prefill(c, false);
-        if (rc != L2J_OK)
+        if (rc != L2J_OK && rc != L2J_E_NOMEM)       // without workspaces: through the decode step, this time
             return rc;
         if (c->prefill) {
-            CK(c, prefill_run(c->prefill, c->stream, tokens, n, pos0));
+            const cudaError_t e = prefill_run(c->prefill, c->stream, tokens, n, pos0);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                return fail(c, L2J_E_NOMEM, "no device memory for %d prompt tokens", n);
+            }
+            CK(c, e);
             CK(c, cudaMemcpyAsync(c->state_host, c->state, sizeof(SeqState), cudaMemcpyDeviceToHost, c->stream));
             CK(c, cudaStreamSynchronize(c->stream));
             return finish_status(c);
@@ -1584,17 +1601,29 @@ extern "C" int l2j_sampler_seed(l2j_ctx *c, int64_t seed)
         return fail(c, L2J_E_INVALID, "the device sampler keeps the probabilities in shared memory: vocabulary of 2..%d tokens",
                     n_max);
     CK(c, cudaSetDevice(c->device));
-    if (!c->samp_state) {
-        int rc = dev_alloc(c, &c->samp_state, 1, true);
+    if (!c->samp_state) {           // made last: everything else is there then
+        int rc = L2J_OK;
         for (int b = 0; b < 2 && rc == L2J_OK; ++b) {
-            rc = dev_alloc(c, &c->samp_prob[b], n, true);
-            if (rc == L2J_OK)
+            if (!c->samp_prob[b])
+                rc = dev_alloc(c, &c->samp_prob[b], n, true);
+            if (rc == L2J_OK && !c->samp_index[b])
                 rc = dev_alloc(c, &c->samp_index[b], n, true);
         }
         if (rc != L2J_OK)
             return rc;
-        CK(c, cudaHostAlloc((void **)&c->samp_host, sizeof(SamplerState), cudaHostAllocDefault));
+        if (!c->samp_host) {
+            const cudaError_t e = alloc_fails(&c->fail_alloc)
+                                      ? cudaErrorMemoryAllocation
+                                      : cudaHostAlloc((void **)&c->samp_host, sizeof(SamplerState), cudaHostAllocDefault);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                return fail(c, L2J_E_NOMEM, "no pinned memory for the sampler: %s", cudaGetErrorString(e));
+            }
+        }
         CK(c, prepare_sampler());
+        rc = dev_alloc(c, &c->samp_state, 1, true);
+        if (rc != L2J_OK)
+            return rc;
     }
     CK(c, cudaStreamSynchronize(c->stream));
     // new Sampler(seed, vocab): every ProbIndex is (0, 0), Random(seed) scrambles the seed (java.util.Random)
@@ -2238,6 +2267,15 @@ extern "C" int l2j_debug_desync(l2j_ctx *c)
     CK(c, cudaMemcpy(&v, epoch, sizeof(v), cudaMemcpyDeviceToHost));
     ++v;
     CK(c, cudaMemcpy(epoch, &v, sizeof(v), cudaMemcpyHostToDevice));
+    return L2J_OK;
+}
+
+extern "C" int l2j_debug_fail_alloc(l2j_ctx *c, int nth)
+{
+    if (!c || nth < 0)
+        return L2J_E_INVALID;
+    std::lock_guard<std::mutex> lock(c->mu);
+    c->fail_alloc = nth;
     return L2J_OK;
 }
 

@@ -267,9 +267,16 @@ struct PrefillModel {
     const float *rope_cos, *rope_sin;
     unsigned int *status;            // device status word of the context
     int timeout_us;
+    int *fail_alloc;                 // host-side failure injection: the allocation that counts it down to zero fails
     bool pdl;                        // programmatic dependent launch between the kernels (not with L2J_F_NO_PDL)
     std::vector<PrefillLayerDesc> layers;
 };
+
+// True for the allocation that l2j_debug_fail_alloc chose.
+inline bool alloc_fails(int *countdown)
+{
+    return countdown && *countdown > 0 && --*countdown == 0;
+}
 
 struct Prefill;
 bool prefill_supported(const PrefillModel &m);

@@ -1624,6 +1624,7 @@ struct Prefill {
     float *logits_host = nullptr;              // pinned, [64][vocab]
     std::map<int, cudaGraphExec_t> step_graphs; // captured step per entry count
     unsigned long long step_launches = 0;
+    bool step_ready = false;                    // all of the buffers of a step exist
     bool no_graph = false;
 };
 
@@ -1653,12 +1654,19 @@ template <typename T>
 static cudaError_t pf_alloc(Prefill *pf, T **out, size_t count)
 {
     void *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    cudaError_t e = alloc_fails(pf->m.fail_alloc) ? cudaErrorMemoryAllocation : cudaMalloc(&p, count * sizeof(T));
     if (e != cudaSuccess)
         return e;
     pf->owned.push_back(p);
     *out = static_cast<T *>(p);
     return cudaMemset(p, 0, count * sizeof(T));
+}
+
+template <typename T>
+static cudaError_t pf_host_alloc(Prefill *pf, T **out, size_t count)
+{
+    return alloc_fails(pf->m.fail_alloc) ? cudaErrorMemoryAllocation
+                                         : cudaHostAlloc(reinterpret_cast<void **>(out), count * sizeof(T), cudaHostAllocDefault);
 }
 
 cudaError_t prefill_create(Prefill **out, const PrefillModel &m)
@@ -1841,7 +1849,8 @@ cudaError_t prefill_run(Prefill *pf, cudaStream_t st, const int *tokens_host, in
     const PrefillModel &m = pf->m;
     if (n > pf->token_cap) {
         int *t = nullptr;
-        PF_CK(cudaMalloc(reinterpret_cast<void **>(&t), sizeof(int) * (size_t)(n + kT)));
+        PF_CK(alloc_fails(m.fail_alloc) ? cudaErrorMemoryAllocation
+                                        : cudaMalloc(reinterpret_cast<void **>(&t), sizeof(int) * (size_t)(n + kT)));
         pf->owned.push_back(t);
         pf->tokens = t;
         pf->token_cap = n;
@@ -1941,15 +1950,21 @@ cudaError_t prefill_batch_create(Prefill *pf, int n_seq, int seq_len)
     }
     PF_CK(pf_alloc(pf, &pf->bkc, per_seq * n_seq));
     PF_CK(pf_alloc(pf, &pf->bvc, per_seq * n_seq));
-    if (!pf->meta) {
-        PF_CK(pf_alloc(pf, &pf->meta, (size_t)4 * kT));
-        PF_CK(pf_alloc(pf, &pf->xn, (size_t)kN * m.dim / 2));
+    if (!pf->step_ready) {      // what an earlier call that failed half-way made is there already
+        if (!pf->meta)
+            PF_CK(pf_alloc(pf, &pf->meta, (size_t)4 * kT));
+        if (!pf->xn)
+            PF_CK(pf_alloc(pf, &pf->xn, (size_t)kN * m.dim / 2));
         if (!encode_bytes_2d(&pf->map_xn, pf->xn, kN, 2 * m.dim, kN, false))
             return cudaErrorNotSupported;
-        PF_CK(pf_alloc(pf, &pf->logits, (size_t)kT * m.vocab));
-        PF_CK(cudaHostAlloc(reinterpret_cast<void **>(&pf->meta_host), sizeof(int) * 4 * kT, cudaHostAllocDefault));
-        PF_CK(cudaHostAlloc(reinterpret_cast<void **>(&pf->logits_host), sizeof(float) * (size_t)kT * m.vocab, cudaHostAllocDefault));
+        if (!pf->logits)
+            PF_CK(pf_alloc(pf, &pf->logits, (size_t)kT * m.vocab));
+        if (!pf->meta_host)
+            PF_CK(pf_host_alloc(pf, &pf->meta_host, (size_t)4 * kT));
+        if (!pf->logits_host)
+            PF_CK(pf_host_alloc(pf, &pf->logits_host, (size_t)kT * m.vocab));
         PF_CK(cudaFuncSetAttribute(bd_classifier_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClsStages * kClsStage + 1024));
+        pf->step_ready = true;
     }
     pf->n_seq = n_seq;
     pf->seq_len_b = seq_len;

@@ -79,6 +79,7 @@ _SIGNATURES = {
     "l2j_pipeline_reset": (C.c_int, [C.POINTER(_P), C.c_int]),
     "l2j_set_wait_limit_us": (C.c_int, [_P, C.c_int]),
     "l2j_debug_desync": (C.c_int, [_P]),
+    "l2j_debug_fail_alloc": (C.c_int, [_P, C.c_int]),
     "l2j_get_stats": (C.c_int, [_P, C.POINTER(Stats)]),
     "l2j_launch_mode": (C.c_int, [_P]),
     "l2j_read_buffer": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, _P, C.c_int]),

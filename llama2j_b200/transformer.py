@@ -227,6 +227,10 @@ class Transformer:
         """Host-side failure injection: the next forward waits for hand-overs that never come."""
         _lib.check(self._lib.l2j_debug_desync(self._ctx), self._ctx)
 
+    def debug_fail_alloc(self, nth: int) -> None:
+        """Host-side failure injection: the nth allocation from now on fails (0: none)."""
+        _lib.check(self._lib.l2j_debug_fail_alloc(self._ctx, int(nth)), self._ctx)
+
     def stats(self) -> _lib.Stats:
         st = _lib.Stats()
         _lib.check(self._lib.l2j_get_stats(self._ctx, C.byref(st)), self._ctx)

@@ -151,3 +151,51 @@ def test_small_shapes_wait_for_whole_kernels_until_a_failure_is_injected():
         assert np.array_equal(plain.forward(t, p)[0], good[p])
     counters.close()
     plain.close()
+
+
+@pytest.mark.parametrize("what", ["batch", "prefill", "sampler"])
+def test_allocation_that_fails_half_way_can_be_made_again(what):
+    """Each allocation of a call that builds its buffers on first use fails in turn (injected on the host, no memory is
+    exhausted): the call reports it, nothing may be used half made, and the same call afterwards works."""
+    cfg = ModelConfig(dim=512, hidden_dim=1280, n_layers=2, n_heads=4, n_kv_heads=4, vocab_size=1000, seq_len=320,
+                      shared_classifier=True)
+    tensors = syn.synthetic_tensors(cfg, 6)
+    toks = np.random.default_rng(7).integers(3, cfg.vocab_size, 300).astype(np.int32)
+
+    def call(m):
+        if what == "batch":
+            m.batch_create(3, 16)
+            return m.batch_forward([0, 1, 2], [0, 0, 0], [5, 6, 7])[0]
+        if what == "prefill":
+            m.prefill(toks, 0)
+            return m.forward(7, toks.size)[0].copy()
+        m.sampler_seed(3)
+        m.forward(7, 0, want_logits=False)
+        return np.array([m.sample(0.9, 0.9)])
+
+    clean = _build(cfg, tensors)
+    want = call(clean)
+    clean.close()
+    failures = 0
+    for nth in range(1, 20):
+        m = _build(cfg, tensors)
+        m.debug_fail_alloc(nth)
+        try:
+            got = call(m)
+        except L.L2jError as e:
+            failures += 1
+            assert e.code == L.E_NOMEM
+            if what == "batch":
+                with pytest.raises(L.L2jError) as e2:        # not by way of buffers that are not there
+                    m.batch_forward([0], [0], [5])
+                assert e2.value.code == L.E_STATE
+            if what == "sampler":
+                with pytest.raises(L.L2jError) as e2:
+                    m.sample(0.9, 0.9)
+                assert e2.value.code == L.E_STATE
+            got = call(m)
+        # (a prompt whose workspaces did not fit has gone through the decode step: 1e-4 as in the tests of the prompt path)
+        assert float(np.abs(got - want).max()) <= (1e-4 * float(want.max() - want.min()) if what == "prefill" else 0.0), nth
+        assert m.stats().device_status == 0
+        m.close()
+    assert failures >= {"batch": 15, "prefill": 1, "sampler": 6}[what]
