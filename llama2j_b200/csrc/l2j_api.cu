@@ -1328,6 +1328,7 @@ extern "C" int l2j_finalize(l2j_ctx *c)
         if (c->exec && c->use_ring && !c->use_fused && c->cfg.seq_len > kLongContextPos)
             try_capture(c, c->pdl_on, true);   // without it the long regime is enqueued kernel by kernel
     }
+    CK(c, cudaStreamSynchronize(nullptr));     // the copies above: the context's stream does not wait for the default stream
     c->finalized = true;
     return L2J_OK;
 }
@@ -1471,7 +1472,7 @@ static int ensure_prefill(l2j_ctx *c, bool required)
     if (!c->prefill_tried) {
         const PrefillModel m = prefill_model(c);
         if (prefill_supported(m) && !(c->flags & L2J_F_NO_TENSOR_PREFILL)) {
-            const cudaError_t e = prefill_create(&c->prefill, m);
+            const cudaError_t e = prefill_create(&c->prefill, m, c->stream);
             if (e == cudaErrorMemoryAllocation) {
                 cudaGetLastError();
                 return fail(c, L2J_E_NOMEM, "no device memory for the workspaces of the batched path");
@@ -1605,9 +1606,9 @@ extern "C" int l2j_sampler_seed(l2j_ctx *c, int64_t seed)
         int rc = L2J_OK;
         for (int b = 0; b < 2 && rc == L2J_OK; ++b) {
             if (!c->samp_prob[b])
-                rc = dev_alloc(c, &c->samp_prob[b], n, true);
+                rc = dev_alloc(c, &c->samp_prob[b], n, false);
             if (rc == L2J_OK && !c->samp_index[b])
-                rc = dev_alloc(c, &c->samp_index[b], n, true);
+                rc = dev_alloc(c, &c->samp_index[b], n, false);
         }
         if (rc != L2J_OK)
             return rc;
@@ -1621,20 +1622,22 @@ extern "C" int l2j_sampler_seed(l2j_ctx *c, int64_t seed)
             }
         }
         CK(c, prepare_sampler());
-        rc = dev_alloc(c, &c->samp_state, 1, true);
+        rc = dev_alloc(c, &c->samp_state, 1, false);
         if (rc != L2J_OK)
             return rc;
     }
     CK(c, cudaStreamSynchronize(c->stream));
     // new Sampler(seed, vocab): every ProbIndex is (0, 0), Random(seed) scrambles the seed (java.util.Random)
     for (int b = 0; b < 2; ++b) {
-        CK(c, cudaMemset(c->samp_prob[b], 0, sizeof(float) * (size_t)n));
-        CK(c, cudaMemset(c->samp_index[b], 0, sizeof(int) * (size_t)n));
+        CK(c, cudaMemsetAsync(c->samp_prob[b], 0, sizeof(float) * (size_t)n, c->stream));
+        CK(c, cudaMemsetAsync(c->samp_index[b], 0, sizeof(int) * (size_t)n, c->stream));
     }
     SamplerState init{};
     init.rng = ((unsigned long long)seed ^ 0x5DEECE66DULL) & ((1ULL << 48) - 1ULL);
     init.token = 0;
-    CK(c, cudaMemcpy(c->samp_state, &init, sizeof(init), cudaMemcpyHostToDevice));
+    *c->samp_host = init;
+    CK(c, cudaMemcpyAsync(c->samp_state, c->samp_host, sizeof(init), cudaMemcpyHostToDevice, c->stream));
+    CK(c, cudaStreamSynchronize(c->stream));   // samp_host belongs to the next sample
     return L2J_OK;
 }
 

@@ -1600,6 +1600,7 @@ bool encode_bytes_2d(CUtensorMap *map, const void *base, int rows, int k, int bo
 
 struct Prefill {
     PrefillModel m;
+    cudaStream_t stream = nullptr;   // where all work on the buffers goes, their clearing included
     int kv_dim = 0, qkv_ld = 0, sms = 0;
     std::vector<CUtensorMap> maps;   // [layer][PF_W_COUNT]
     CUtensorMap map_b_dim, map_b_hidden;
@@ -1650,6 +1651,7 @@ void prefill_destroy(Prefill *pf)
     delete pf;
 }
 
+// Cleared on the stream of the kernels that use it: that stream does not wait for the default stream.
 template <typename T>
 static cudaError_t pf_alloc(Prefill *pf, T **out, size_t count)
 {
@@ -1659,7 +1661,7 @@ static cudaError_t pf_alloc(Prefill *pf, T **out, size_t count)
         return e;
     pf->owned.push_back(p);
     *out = static_cast<T *>(p);
-    return cudaMemset(p, 0, count * sizeof(T));
+    return cudaMemsetAsync(p, 0, count * sizeof(T), pf->stream);
 }
 
 template <typename T>
@@ -1669,13 +1671,14 @@ static cudaError_t pf_host_alloc(Prefill *pf, T **out, size_t count)
                                          : cudaHostAlloc(reinterpret_cast<void **>(out), count * sizeof(T), cudaHostAllocDefault);
 }
 
-cudaError_t prefill_create(Prefill **out, const PrefillModel &m)
+cudaError_t prefill_create(Prefill **out, const PrefillModel &m, cudaStream_t st)
 {
     *out = nullptr;
     if (!prefill_supported(m) || (int)m.layers.size() != m.n_layers)
         return cudaErrorInvalidValue;
     Prefill *pf = new Prefill();
     pf->m = m;
+    pf->stream = st;
     pf->kv_dim = m.n_kv_heads * m.head;
     pf->qkv_ld = m.dim + 2 * pf->kv_dim;
     int dev = 0;
@@ -1849,9 +1852,7 @@ cudaError_t prefill_run(Prefill *pf, cudaStream_t st, const int *tokens_host, in
     const PrefillModel &m = pf->m;
     if (n > pf->token_cap) {
         int *t = nullptr;
-        PF_CK(alloc_fails(m.fail_alloc) ? cudaErrorMemoryAllocation
-                                        : cudaMalloc(reinterpret_cast<void **>(&t), sizeof(int) * (size_t)(n + kT)));
-        pf->owned.push_back(t);
+        PF_CK(pf_alloc(pf, &t, (size_t)(n + kT)));
         pf->tokens = t;
         pf->token_cap = n;
     }

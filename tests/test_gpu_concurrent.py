@@ -133,6 +133,27 @@ def test_classifier_of_a_step(vocab, entries):
     m.close()
 
 
+def test_steps_right_behind_large_new_caches():
+    """Caches of several GB are still being cleared when the first step is enqueued: it comes behind the clearing, so the
+    rows it writes are there for the second step."""
+    import torch
+    cfg = ModelConfig(1024, 1280, 1, 8, 8, 300, 4096, True)
+    m = _build(cfg, _tensors(cfg, 31))
+    seqs = list(range(64))
+    toks = np.random.default_rng(32).integers(3, cfg.vocab_size, (3, 64)).astype(np.int32)
+    got = []
+    for wait, n_seq in ((True, 64), (False, 256), (False, 384)):      # 8.6 GB per 256 sequences
+        m.batch_create(n_seq, 4096)
+        if wait:
+            torch.cuda.synchronize()
+        got.append([m.batch_forward(seqs, [p] * 64, toks[p])[0] for p in range(3)])
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert np.array_equal(a, b)
+    assert m.stats().device_status == 0
+    m.close()
+
+
 def test_full_batch_of_64_at_the_110m_shape():
     cfg = syn.SHAPES["stories110M"]
     tensors = _tensors(cfg, 13)
