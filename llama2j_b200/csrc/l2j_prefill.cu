@@ -1375,6 +1375,8 @@ __global__ void __launch_bounds__(kClsThreads, 1) bd_classifier_kernel(const __g
         };
         auto store = [&](int it, const float4 (&d)[4][2]) -> bool {
             const int s = it % kClsStages;
+            if (it == kClsStages)
+                pdl_wait();
             if (!__all_sync(0xffffffffu, pf_wait(b_empty + 8 * s, (uint32_t)((it / kClsStages) & 1) ^ 1u, give_up, limit)))
                 return false;
 #pragma unroll
@@ -1389,7 +1391,8 @@ __global__ void __launch_bounds__(kClsThreads, 1) bd_classifier_kernel(const __g
                 mbar_arrive(b_full + 8 * s);
             return true;
         };
-        // the weights do not depend on the kernel in front: no wait for it here
+        // The weights do not depend on the kernel in front: no wait for it before the ring is full.  The stage after that is
+        // freed by the roles that do wait; the time limit of waiting for it must not run while the kernel in front still does.
         if (total > 0)
             load(0, x[0]);
         if (total > 1)
@@ -1406,7 +1409,7 @@ __global__ void __launch_bounds__(kClsThreads, 1) bd_classifier_kernel(const __g
                     load(it + 3, x[1]);
             }
         }
-        pdl_wait();
+        pdl_wait();                                          // (a ring that was never full)
     } else if (warp == kClsCvt + kClsEpi + 1) {
         pdl_wait();
         if (lane == 0) {

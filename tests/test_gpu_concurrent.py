@@ -154,6 +154,29 @@ def test_steps_right_behind_large_new_caches():
     m.close()
 
 
+def test_short_wait_limit_does_not_count_the_kernels_in_front():
+    """The classifier's blocks start while W2 (32 groups per block here, well over the limit of 20 us) still runs; their
+    time limits start when it has ended."""
+    cfg = ModelConfig(8192, 16384, 1, 64, 8, 1024, 16, False)
+    m = Transformer(cfg)
+    m.set_wait_limit_us(20)
+    for t in L.QUANT_TENSORS:
+        n = cfg.tensor_floats(t)
+        m.upload_quant(t, syn.quant_encode(np.ones(n, dtype=np.float32)) if t in (L.T_RMS_ATT, L.T_RMS_FFN, L.T_RMS_FINAL)
+                       else syn.synth_quant(n, 41, t))
+    for t in (L.T_TOKEN_EMBEDDING, L.T_WCLS):
+        m.upload_f32(t, syn.synth_f32(cfg.tensor_floats(t), 41, t))
+    m.finalize()
+    m.batch_create(64, 4)
+    first = None
+    for _ in range(5):
+        logits, _ = m.batch_forward(list(range(64)), [0] * 64, list(range(64)))
+        assert m.stats().device_status == 0
+        first = logits if first is None else first
+        assert np.array_equal(logits, first)
+    m.close()
+
+
 def test_full_batch_of_64_at_the_110m_shape():
     cfg = syn.SHAPES["stories110M"]
     tensors = _tensors(cfg, 13)
