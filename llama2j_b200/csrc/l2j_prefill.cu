@@ -418,7 +418,8 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
                     const float2 ms = msq[j];
                     const int b = (int)(it & 1);
                     const uint32_t pha = (uint32_t)((it >> 1) & 1);
-                    if (!pf_wait(bar_acc_full + 8 * b, pha, give_up, limit)) {
+                    // one answer for the warp: the loads below are the whole warp's
+                    if (!__all_sync(0xffffffffu, pf_wait(bar_acc_full + 8 * b, pha, give_up, limit))) {
                         ok = false;
                         continue;
                     }
