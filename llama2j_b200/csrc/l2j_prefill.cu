@@ -781,12 +781,17 @@ __device__ __forceinline__ void tmem_st_wait()
 }
 
 // A pair of floats as three pairs of bf16 that add up to them: each difference is exact, and what the third piece has to
-// hold fits its 8 bits.
+// hold fits its 8 bits.  The first two pieces saturate: a float above the largest bf16 is then the sum of finite pieces,
+// and of an infinite one only the third piece is infinite, which meets nothing but the other operand's first piece, so that
+// the product is the infinity of the right sign and not infinity - infinity.
 __device__ __forceinline__ void split_bf16(float a, float b, uint32_t (&piece)[3])
 {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(piece[i]) : "f"(b), "f"(a));
+        if (i < 2)
+            asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(piece[i]) : "f"(b), "f"(a));
+        else
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(piece[i]) : "f"(b), "f"(a));
         a -= __uint_as_float(piece[i] << 16);
         b -= __uint_as_float(piece[i] & 0xffff0000u);
     }

@@ -133,6 +133,33 @@ def test_classifier_of_a_step(vocab, entries):
     m.close()
 
 
+def test_classifier_weights_at_the_end_of_the_range():
+    """Weights that are infinite, NaN, or finite but above the largest bf16 number (3.3895e38): the logits of the decode
+    path's FP32 classifier, infinities with their sign."""
+    cfg = ModelConfig(512, 1280, 1, 8, 8, 300, 64, False)
+    tensors = _tensors(cfg, 27)
+    # a final norm of 0.02: 3.4e38 times an element of x stays finite
+    tensors[L.T_RMS_FINAL] = syn.quant_encode(np.full(cfg.dim, 0.02, dtype=np.float32))
+    wcls = tensors[L.T_WCLS].reshape(cfg.vocab_size, cfg.dim).copy()
+    wcls[3, 7], wcls[130, 500], wcls[200, 64] = np.inf, -np.inf, np.nan
+    wcls[10, 100], wcls[299, 511], wcls[129, 0] = 3.4e38, -3.4e38, 3.39e38
+    tensors[L.T_WCLS] = wcls.reshape(-1)
+    m = _build(cfg, tensors)
+    m.batch_create(5, 8)
+    toks = np.array([3, 50, 99, 150, 299], dtype=np.int32)
+    logits, _ = m.batch_forward(np.arange(5), np.zeros(5, dtype=np.int32), toks)
+    for i, t in enumerate(toks):
+        want = m.forward(int(t), 0)[0]
+        assert np.isinf(want[[3, 130]]).all() and np.isnan(want[200]) and np.isfinite(want[[10, 129, 299]]).all()
+        assert np.array_equal(logits[i][[3, 130]], want[[3, 130]]) and np.isnan(logits[i][200])
+        big = [10, 129, 299]
+        assert np.abs(logits[i][big] / want[big] - 1).max() < LOGIT_TOL
+        rest = np.setdiff1d(np.arange(cfg.vocab_size), big + [3, 130, 200])
+        _check(logits[i][rest], want[rest])
+    assert m.stats().device_status == 0
+    m.close()
+
+
 def test_steps_right_behind_large_new_caches():
     """Caches of several GB are still being cleared when the first step is enqueued: it comes behind the clearing, so the
     rows it writes are there for the second step."""
