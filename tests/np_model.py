@@ -13,6 +13,19 @@ def dequant(groups: np.ndarray, n: int) -> np.ndarray:
     return vals.reshape(-1)[:n]
 
 
+def bf16_pieces(x: np.ndarray, n: int | None) -> np.ndarray:
+    """What n bf16 numbers hold of each FP32 operand (None: the operand as it is)."""
+    if n is None:
+        return x
+    left, held = x.astype(np.float32), np.zeros(x.shape)
+    for _ in range(n):
+        bits = left.view(np.uint32).astype(np.uint64)
+        piece = (((bits + 0x7fff + ((bits >> 16) & 1)) >> 16) << 16).astype(np.uint32).view(np.float32)   # to nearest, ties to even
+        held += piece
+        left = left - piece
+    return held
+
+
 class NumpyModel:
     def __init__(self, cfg, tensors):
         self.cfg = cfg

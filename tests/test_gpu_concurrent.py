@@ -12,6 +12,8 @@ from llama2j_b200 import lib as L
 from llama2j_b200 import synthetic as syn
 from llama2j_b200.model_files import ModelConfig
 from llama2j_b200.transformer import Transformer
+from tests.np_model import bf16_pieces as pieces
+from tests.np_model import dequant
 
 pytestmark = pytest.mark.gpu
 
@@ -131,6 +133,31 @@ def test_classifier_of_a_step(vocab, entries):
         _check(logits[i], m.forward(int(t), 0)[0])
     assert m.stats().device_status == 0
     m.close()
+
+
+@pytest.mark.parametrize("dim, heads", [(768, 12), (4096, 32)])
+def test_classifier_of_a_step_against_float64(dim, heads):
+    """Operands in three bf16 pieces lose nothing that FP32 holds: against float64, with layers that add nothing, the error
+    stays below half of what operands of two pieces would cost (rounded here, on the CPU, to 16 bits)."""
+    cfg = ModelConfig(dim, 256, 1, heads, heads, 1500, 16, False)
+    tensors = syn.synthetic_tensors(cfg, 3)
+    for t in (L.T_WQ, L.T_WK, L.T_WV, L.T_WO, L.T_W1, L.T_W2, L.T_W3):
+        tensors[t] = syn.quant_encode(np.zeros(cfg.tensor_floats(t), dtype=np.float32))
+    wcls = np.random.default_rng(1).normal(0, 6 / np.sqrt(dim), (cfg.vocab_size, dim)).astype(np.float32)
+    tensors[L.T_WCLS] = wcls.reshape(-1)
+    m = _build(cfg, tensors)
+    m.batch_create(64, 8)
+    toks = np.arange(64, dtype=np.int32) * 7 + 3
+    logits, _ = m.batch_forward(np.arange(64), np.zeros(64, dtype=np.int32), toks)
+    assert m.stats().device_status == 0
+    m.close()
+    x = np.asarray(tensors[L.T_TOKEN_EMBEDDING], dtype=np.float64).reshape(cfg.vocab_size, dim)[toks]
+    x = dequant(tensors[L.T_RMS_FINAL], dim) * (x / np.sqrt((x * x).mean(1, keepdims=True) + 1e-5))
+    exact = x @ wcls.astype(np.float64).T
+    two = pieces(x, 2) @ pieces(wcls, 2).T
+    error = lambda y: np.linalg.norm(y - exact) / np.linalg.norm(exact)
+    print(f"error {error(logits):.2e}, with two pieces {error(two):.2e}")
+    assert error(logits) < 0.5 * error(two)
 
 
 def test_classifier_weights_at_the_end_of_the_range():

@@ -14,6 +14,7 @@ from llama2j_b200 import lib as L
 from llama2j_b200 import synthetic as syn
 from llama2j_b200.model_files import ModelConfig
 from llama2j_b200.transformer import Transformer
+from tests.np_model import bf16_pieces, dequant
 
 pytestmark = pytest.mark.gpu
 
@@ -133,6 +134,60 @@ def test_prefill_attention_around_its_tiles(heads, kv_heads, first, more):
     assert pre.stats().device_status == 0
     dec.close()
     pre.close()
+
+
+def _v_behind_attention(cfg, tensors, toks, k, v, rows, pieces=None):
+    """float64: V rows of layer 1, from layer 0's embedded tokens, its attention over the cache rows given and what follows."""
+    d, h, n_l, kv = cfg.dim, cfg.hidden_dim, cfg.n_layers, cfg.kv_dim
+    n, hs, mul = len(toks), cfg.dim // cfg.n_heads, cfg.n_heads // cfg.n_kv_heads
+    mat = lambda t, r, c: dequant(tensors[t], n_l * r * c).reshape(n_l, r, c)
+    rms = lambda x, w: w * (x / np.sqrt((x * x).mean(-1, keepdims=True) + 1e-5))
+    g_att, g_ffn = (dequant(tensors[t], n_l * d).reshape(n_l, d) for t in (L.T_RMS_ATT, L.T_RMS_FFN))
+    x = np.asarray(tensors[L.T_TOKEN_EMBEDDING], dtype=np.float64).reshape(cfg.vocab_size, d)[toks]
+    q = rms(x, g_att[0]) @ mat(L.T_WQ, d, d)[0].T
+    i = np.arange(0, d, 2)
+    angle = np.arange(n)[:, None] / 10000.0 ** ((i % hs) / hs)
+    q[:, 0::2], q[:, 1::2] = (q[:, 0::2] * np.cos(angle) - q[:, 1::2] * np.sin(angle),
+                              q[:, 0::2] * np.sin(angle) + q[:, 1::2] * np.cos(angle))
+    x = x[rows]
+    out = np.zeros((len(rows), d))
+    for head in range(cfg.n_heads):
+        cols, kvc = slice(head * hs, (head + 1) * hs), slice(head // mul * hs, (head // mul + 1) * hs)
+        s = bf16_pieces(q[rows, cols] / np.sqrt(hs), pieces) @ bf16_pieces(k[:, kvc], pieces).T
+        s = np.where(np.arange(n)[None, :] <= np.asarray(rows)[:, None], s, -np.inf)
+        p = np.exp(s - s.max(-1, keepdims=True))
+        out[:, cols] = bf16_pieces(p, pieces) @ bf16_pieces(v[:, kvc], pieces) / p.sum(-1, keepdims=True)
+    x = x + out @ mat(L.T_WO, d, d)[0].T
+    xb = rms(x, g_ffn[0])
+    h1 = xb @ mat(L.T_W1, h, d)[0].T
+    x = x + (h1 / (1 + np.exp(-h1)) * (xb @ mat(L.T_W3, h, d)[0].T)) @ mat(L.T_W2, d, h)[0].T
+    return rms(x, g_att[1]) @ mat(L.T_WV, kv, d)[1].T
+
+
+@pytest.mark.parametrize("heads, kv_heads, cuts", [(4, 2, ()), (8, 4, (200,))])
+@pytest.mark.parametrize("scale", [1, 4])
+def test_prefill_attention_against_float64(heads, kv_heads, cuts, scale):
+    """Operands in three bf16 pieces lose nothing that FP32 holds.  The gate is what the pieces decide: with two of them
+    the error against float64 (computed here, on the CPU) would be at least twice what is allowed.  `scale` sharpens the
+    softmax: scores of about 1 and 16 times that."""
+    cfg = ModelConfig(512, 1280, 2, heads, kv_heads, 1000, 512, True)
+    tensors = _tensors(cfg, 12)
+    rng = np.random.default_rng(13)
+    for t in (L.T_WQ, L.T_WK):
+        tensors[t] = syn.quant_encode(rng.normal(0, 0.02 * scale, cfg.tensor_floats(t)).astype(np.float32))
+    toks = rng.integers(3, cfg.vocab_size, 330).astype(np.int32)
+    m = _build(cfg, tensors)
+    for a, b in zip((0, *cuts), (*cuts, len(toks))):
+        m.prefill(toks[a:b], a)
+    rows = [1, 63, 64, 127, 128, 199, 200, 255, 256, 329]
+    got = np.stack([m.read_buffer(6, cfg.kv_dim, 1, p) for p in rows])
+    k, v = (np.stack([m.read_buffer(which, cfg.kv_dim, 0, p) for p in range(len(toks))]) for which in (5, 6))
+    assert m.stats().device_status == 0
+    m.close()
+    exact, two = (_v_behind_attention(cfg, tensors, toks, k, v, rows, pieces) for pieces in (None, 2))
+    error = lambda x: np.linalg.norm(x - exact) / np.linalg.norm(exact)
+    print(f"error {error(got):.2e}, with two pieces {error(two):.2e}")
+    assert error(got) < 0.5 * error(two)
 
 
 def test_a_smaller_shape_does_not_take_the_larger_ones_shared_memory():
