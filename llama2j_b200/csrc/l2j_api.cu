@@ -2570,10 +2570,13 @@ int status_of(SeqState *dev_state)
 // Large arrays go through pinned staging buffers on several host threads, each with a stream of its own: one thread's
 // copies between pageable and pinned memory move 5 to 10 GB/s and the link more than 50, and the runtime's own staging
 // of a pageable copy is one thread's.  The buffers are those of this call (10 MB pinned, 10 MB on the device).
-// 45 M floats (a W1 matrix of the 7B shape): 28-37 ms in one piece, 20-23 ms this way, of which 4 are the pinned buffers.
+// Host to host, ms, in one piece and this way (medians over boxes of 16 cores; single calls scatter by half): 45 M floats (a
+// W1 matrix of the 7B shape) 28-29 and 19-22, 128 Mi 80-82 and 38-40.
 constexpr int64_t kStagedPiece = (int64_t)kGroup << 10;     // floats per piece: 1 MB
-constexpr int64_t kStagedFloats = (int64_t)kGroup << 14;    // from 4 Mi floats on: making the buffers and threads takes about
-                                                            // as long as the plain path needs for a quarter of that
+constexpr int64_t kStagedFloats = (int64_t)kGroup << 17;    // from 32 Mi floats on (22-24 and 19-25 ms): making buffers and
+                                                            // threads takes about 8 ms, and only then do the fresh pages of the
+                                                            // output slow the plain path (4 Mi floats 2.6 and 11 ms, 16 Mi 8.5
+                                                            // and 14, 24 Mi 12 and 17)
 constexpr int kStagedThreads = 8;
 constexpr int kNotStaged = 1;                                // no such status code
 
@@ -2655,7 +2658,10 @@ extern "C" int l2j_quant_encode(int device, const float *in, int64_t n_floats, v
     int rc = set_device_checked(device);
     if (rc != L2J_OK)
         return rc;
-    if (n_floats >= kStagedFloats) {
+    // (where `out` overlaps `in`, a lane could overwrite what another has still to read; the plain path reads a piece first)
+    const uint8_t *in0 = reinterpret_cast<const uint8_t *>(in), *in1 = reinterpret_cast<const uint8_t *>(in + n_floats);
+    const uint8_t *out0 = static_cast<uint8_t *>(out), *out1 = out0 + (n_floats + kGroup - 1) / kGroup * kGroupBytes;
+    if (n_floats >= kStagedFloats && (out1 <= in0 || in1 <= out0)) {
         rc = quant_encode_staged(device, in, n_floats, static_cast<uint8_t *>(out));
         if (rc != kNotStaged)
             return rc;

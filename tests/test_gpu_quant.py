@@ -58,13 +58,27 @@ def test_synthetic_checkpoint_equals_oracle_checkpoint(oracle, l2j):
         assert np.array_equal(a[t].view(np.uint8), b[t].view(np.uint8)), t
 
 
+@pytest.mark.parametrize("base", [1 << 22, 1 << 25])
 @pytest.mark.parametrize("extra", [0, 1, 257, 262144, 262145 + 256])
-def test_large_arrays_through_the_staging_buffers(extra, l2j):
-    """4 Mi floats and more go through pinned buffers on several threads: the bytes of the same floats sent in parts that
+def test_large_arrays_through_the_staging_buffers(extra, base, l2j):
+    """32 Mi floats and more go through pinned buffers on several threads: the bytes of the same floats sent in parts that
     are too short for that, around the ends of the pieces (262144 floats) and groups (256)."""
-    n = (1 << 22) + extra
+    n = base + extra
     values = np.random.default_rng(extra).normal(0, 0.02, n).astype(np.float32)
     whole = syn.quant_encode(values)
     part = 1 << 20
     pieces = [syn.quant_encode(values[i: i + part]) for i in range(0, n, part)]
     assert np.array_equal(whole, np.concatenate(pieces))
+
+
+@pytest.mark.parametrize("shift", [0, 100, -1000])
+def test_encoding_in_place(shift, l2j):
+    """`out` may lie over `in` (by a shift of so many bytes): the bytes are those of separate arrays."""
+    n = (1 << 25) + 300
+    values = np.random.default_rng(9).normal(0, 0.02, n).astype(np.float32)
+    want = syn.quant_encode(values)
+    room = np.zeros(4 * n + 4096, dtype=np.uint8)
+    room[2048: 2048 + 4 * n] = values.view(np.uint8)
+    at = room.ctypes.data + 2048
+    l2j.check(l2j.load().l2j_quant_encode(0, at, n, at + shift))
+    assert np.array_equal(room[2048 + shift: 2048 + shift + want.size], want)
