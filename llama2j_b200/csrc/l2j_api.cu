@@ -1467,12 +1467,12 @@ static PrefillModel prefill_model(l2j_ctx *c)
 
 // Builds the batched path of a whole-model context on first use; L2J_E_INVALID where the shape is outside it,
 // L2J_E_NOMEM (this call's, the next one tries again) where its workspaces do not fit.
-static int ensure_prefill(l2j_ctx *c, bool required)
+static int ensure_prefill(l2j_ctx *c, bool required, int n)
 {
     if (!c->prefill_tried) {
         const PrefillModel m = prefill_model(c);
         if (prefill_supported(m) && !(c->flags & L2J_F_NO_TENSOR_PREFILL)) {
-            const cudaError_t e = prefill_create(&c->prefill, m, c->stream);
+            const cudaError_t e = prefill_create(&c->prefill, m, c->stream, n);
             if (e == cudaErrorMemoryAllocation) {
                 cudaGetLastError();
                 return fail(c, L2J_E_NOMEM, "no device memory for the workspaces of the batched path");
@@ -1505,7 +1505,7 @@ extern "C" int l2j_prefill(l2j_ctx *c, const int32_t *tokens, int n, int pos0)
         if (n == 0)
             return L2J_OK;
         CK(c, cudaSetDevice(c->device));
-        const int rc = ensure_prefill(c, false);
+        const int rc = ensure_prefill(c, false, n);
         if (rc != L2J_OK && rc != L2J_E_NOMEM)       // without workspaces: through the decode step, this time
             return rc;
         if (c->prefill) {
@@ -1541,7 +1541,7 @@ extern "C" int l2j_batch_create(l2j_ctx *c, int n_seq, int seq_len)
     if (n_seq < 1 || seq_len < 1 || seq_len > c->cfg.seq_len)
         return fail(c, L2J_E_INVALID, "n_seq >= 1 and 1 <= seq_len <= %d", c->cfg.seq_len);
     CK(c, cudaSetDevice(c->device));
-    const int rc = ensure_prefill(c, true);
+    const int rc = ensure_prefill(c, true, kPrefillTokens);
     if (rc != L2J_OK)
         return rc;
     CK(c, cudaStreamSynchronize(c->stream));

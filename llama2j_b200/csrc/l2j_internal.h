@@ -280,7 +280,8 @@ inline bool alloc_fails(int *countdown)
 
 struct Prefill;
 bool prefill_supported(const PrefillModel &m);
-cudaError_t prefill_create(Prefill **out, const PrefillModel &m, cudaStream_t st);   // st: the stream of all later calls
+// st: the stream of all later calls; n: tokens of the call it is made for
+cudaError_t prefill_create(Prefill **out, const PrefillModel &m, cudaStream_t st, int n);
 cudaError_t prefill_run(Prefill *pf, cudaStream_t stream, const int *tokens_host, int n, int pos0);
 cudaError_t prefill_batch_create(Prefill *pf, int n_seq, int seq_len);
 cudaError_t prefill_batch_forward(Prefill *pf, cudaStream_t stream, const int *tokens, const int *pos, const int *seq, int n, float *logits_out,

@@ -31,6 +31,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #define PF_DS_WAIT_TIMEOUT 0x1u   // L2J_DS_WAIT_TIMEOUT of the public header
@@ -1607,18 +1608,24 @@ bool encode_bytes_2d(CUtensorMap *map, const void *base, int rows, int k, int bo
 
 }  // namespace
 
-struct Prefill {
+// What the kernels of one chunk hand to each other.
+struct Workspaces {
+    int blocks = 0;              // blocks of 64 tokens they hold: one, or kTB
+    float *x = nullptr, *qkv = nullptr, *q = nullptr, *h13 = nullptr;
+    float *parts = nullptr;      // [kMaxParts][blocks * 64][dim]: partial row sums of Wo / W2, or the attention's key ranges
+    int8_t *limbs = nullptr;
+    float2 *ux = nullptr;
+    float *ssq = nullptr;        // [blocks][groups / 4][64]
+    CUtensorMap map_b_dim, map_b_hidden;
+    char *mem = nullptr;         // all of them
+};
+
+struct Prefill : Workspaces {
     PrefillModel m;
     cudaStream_t stream = nullptr;   // where all work on the buffers goes, their clearing included
     int kv_dim = 0, qkv_ld = 0, sms = 0;
     std::vector<CUtensorMap> maps;   // [layer][PF_W_COUNT]
-    CUtensorMap map_b_dim, map_b_hidden;
     int *tokens = nullptr;
-    float *x = nullptr, *qkv = nullptr, *q = nullptr, *h13 = nullptr;
-    float *parts = nullptr;      // [kMaxParts][kTB * 64][dim]: partial row sums of Wo / W2, or the attention's key ranges
-    int8_t *limbs = nullptr;
-    float2 *ux = nullptr;
-    float *ssq = nullptr;         // [kTB][groups / 4][64]
     int token_cap = 0;
     size_t gemm_smem_dim = 0, gemm_smem_hidden = 0, attn_smem = 0;
     std::vector<void *> owned;
@@ -1673,6 +1680,16 @@ static cudaError_t pf_alloc(Prefill *pf, T **out, size_t count)
     return cudaMemsetAsync(p, 0, count * sizeof(T), pf->stream);
 }
 
+static void pf_free(Prefill *pf, void *ptr)
+{
+    for (size_t i = 0; i < pf->owned.size(); ++i)
+        if (pf->owned[i] == ptr) {
+            cudaFree(ptr);
+            pf->owned.erase(pf->owned.begin() + (long)i);
+            return;
+        }
+}
+
 template <typename T>
 static cudaError_t pf_host_alloc(Prefill *pf, T **out, size_t count)
 {
@@ -1680,7 +1697,66 @@ static cudaError_t pf_host_alloc(Prefill *pf, T **out, size_t count)
                                          : cudaHostAlloc(reinterpret_cast<void **>(out), count * sizeof(T), cudaHostAllocDefault);
 }
 
-cudaError_t prefill_create(Prefill **out, const PrefillModel &m, cudaStream_t st)
+// Workspaces of `blocks` blocks in the place of those there are, which stay if the new ones do not fit.  A concurrent step
+// and a prompt of at most 64 tokens need one block (35 MB at the 7B shape), the chunks of a longer prompt four (141 MB).
+// The captured steps hold the old addresses: they are captured again when they are next asked for.  First prompt of a
+// 2-layer model of the 7B shape, ms, with eight allocations of four blocks for every caller and with this: 37 tokens 2.6
+// and 0.9, 700 tokens 3.9 and 2.4; 300 tokens behind 37 0.77 and 1.6.
+static cudaError_t make_workspaces(Prefill *pf, int blocks)
+{
+    const PrefillModel &m = pf->m;
+    const size_t kmax = m.dim > m.hidden ? m.dim : m.hidden, tokens = (size_t)blocks * kT;
+    Workspaces w;
+    w.blocks = blocks;
+    // one allocation: the parts are walked once for its size and once for their addresses
+    size_t at = 0;
+    auto take = [&](auto *&part, size_t count) {
+        if (w.mem)
+            part = reinterpret_cast<std::remove_reference_t<decltype(part)>>(w.mem + at);
+        at += (count * sizeof(*part) + 1023) & ~(size_t)1023;
+    };
+    auto walk = [&]() {
+        at = 0;
+        take(w.x, tokens * m.dim);
+        take(w.qkv, tokens * pf->qkv_ld);
+        take(w.q, tokens * m.dim);
+        take(w.h13, kWideParts * tokens * 2 * m.hidden);
+        take(w.parts, kMaxParts * tokens * (m.dim + 2 * m.n_heads));
+        take(w.limbs, (size_t)blocks * kN * kmax);
+        take(w.ux, (kmax / 256) * tokens);
+        take(w.ssq, (kmax / 256) * tokens);
+    };
+    walk();
+    cudaError_t e = pf_alloc(pf, &w.mem, at);
+    if (e != cudaSuccess)
+        return e;
+    walk();
+    if (!encode_bytes_2d(&w.map_b_dim, w.limbs, blocks * kN, m.dim, kN, false) ||
+        !encode_bytes_2d(&w.map_b_hidden, w.limbs, blocks * kN, m.hidden, kN, false))
+        return cudaErrorNotSupported;
+    for (auto &g : pf->step_graphs)
+        cudaGraphExecDestroy(g.second);
+    pf->step_graphs.clear();
+    pf_free(pf, pf->mem);
+    static_cast<Workspaces &>(*pf) = w;
+    return cudaSuccess;
+}
+
+// The workspaces for n tokens.  Where four blocks do not fit, one has to do: chunks of 64 tokens.
+static cudaError_t ensure_workspaces(Prefill *pf, int n)
+{
+    const int want = n > kT ? kTB : 1;
+    if (pf->blocks >= want)
+        return cudaSuccess;
+    cudaError_t e = make_workspaces(pf, want);
+    if (e == cudaErrorMemoryAllocation && want > 1) {
+        cudaGetLastError();
+        e = pf->blocks > 0 ? cudaSuccess : make_workspaces(pf, 1);
+    }
+    return e;
+}
+
+cudaError_t prefill_create(Prefill **out, const PrefillModel &m, cudaStream_t st, int n)
 {
     *out = nullptr;
     if (!prefill_supported(m) || (int)m.layers.size() != m.n_layers)
@@ -1694,15 +1770,8 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m, cudaStream_t st
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&pf->sms, cudaDevAttrMultiProcessorCount, dev);
-    const int kmax = m.dim > m.hidden ? m.dim : m.hidden;
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->x, (size_t)kTB * kT * m.dim);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->qkv, (size_t)kTB * kT * pf->qkv_ld);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->q, (size_t)kTB * kT * m.dim);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->h13, (size_t)kWideParts * kTB * kT * 2 * m.hidden);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->parts, (size_t)kMaxParts * kTB * kT * (m.dim + 2 * m.n_heads));
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->limbs, (size_t)kTB * kN * kmax);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->ux, (size_t)kTB * (kmax / 256) * kT);
-    if (e == cudaSuccess) e = pf_alloc(pf, &pf->ssq, (size_t)kTB * (kmax / 256) * kT);
+    if (e == cudaSuccess)
+        e = ensure_workspaces(pf, n);
     if (e != cudaSuccess) {
         prefill_destroy(pf);
         return e;
@@ -1714,8 +1783,6 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m, cudaStream_t st
     for (int l = 0; l < m.n_layers && ok; ++l)
         for (int w = 0; w < PF_W_COUNT && ok; ++w)
             ok = encode_bytes_2d(&pf->maps[(size_t)l * PF_W_COUNT + w], m.layers[(size_t)l].w[w], rows[w], ks[w], kTileM, true);
-    ok = ok && encode_bytes_2d(&pf->map_b_dim, pf->limbs, kTB * kN, m.dim, kN, false) &&
-         encode_bytes_2d(&pf->map_b_hidden, pf->limbs, kTB * kN, m.hidden, kN, false);
     if (!ok) {
         prefill_destroy(pf);
         return cudaErrorNotSupported;
@@ -1866,9 +1933,10 @@ cudaError_t prefill_run(Prefill *pf, cudaStream_t st, const int *tokens_host, in
         pf->token_cap = n;
     }
     PF_CK(cudaMemcpyAsync(pf->tokens, tokens_host, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st));
-    const int dim = m.dim, hidden = m.hidden, kvd = pf->kv_dim;
-    for (int c0 = 0; c0 < n; c0 += kTB * kT) {
-        const int nv = n - c0 < kTB * kT ? n - c0 : kTB * kT;
+    PF_CK(ensure_workspaces(pf, n));
+    const int dim = m.dim, hidden = m.hidden, kvd = pf->kv_dim, chunk = pf->blocks * kT;
+    for (int c0 = 0; c0 < n; c0 += chunk) {
+        const int nv = n - c0 < chunk ? n - c0 : chunk;
         const int tb = (nv + kT - 1) / kT;
         const Splits ks = splits_for(pf, tb);
         pf_embed_kernel<<<tb * kT, 256, 0, st>>>(pf->tokens + c0, nv, m.emb, dim, m.vocab, pf->x);    // behind a copy or a whole chunk
@@ -1941,20 +2009,12 @@ cudaError_t prefill_batch_create(Prefill *pf, int n_seq, int seq_len)
     if (n_seq < 1 || seq_len < 1 || seq_len > m.seq_len)
         return cudaErrorInvalidValue;
     const size_t per_seq = (size_t)m.n_layers * m.n_kv_heads * seq_len * m.head;
-    auto drop = [&](void *ptr) {
-        for (size_t i = 0; i < pf->owned.size(); ++i)
-            if (pf->owned[i] == ptr) {
-                cudaFree(ptr);
-                pf->owned.erase(pf->owned.begin() + (long)i);
-                return;
-            }
-    };
     for (auto &g : pf->step_graphs)
         cudaGraphExecDestroy(g.second);
     pf->step_graphs.clear();
     if (pf->bkc) {
-        drop(pf->bkc);
-        drop(pf->bvc);
+        pf_free(pf, pf->bkc);
+        pf_free(pf, pf->bvc);
         pf->bkc = pf->bvc = nullptr;
         pf->n_seq = 0;
     }

@@ -231,6 +231,31 @@ def test_short_wait_limit_does_not_count_the_kernels_in_front():
     m.close()
 
 
+def test_workspaces_of_a_step_and_of_a_long_prompt():
+    """A step needs the workspaces of 64 tokens only; a longer prompt replaces them by larger ones, behind which the steps
+    (captured anew) compute the same bits."""
+    import torch
+    cfg = ModelConfig(4096, 11008, 1, 32, 4, 300, 512, True)
+    m = Transformer(cfg)
+    for t in L.QUANT_TENSORS:
+        m.upload_quant(t, syn.synth_quant(cfg.tensor_floats(t), 42, t))
+    m.upload_f32(L.T_TOKEN_EMBEDDING, syn.synth_f32(cfg.tensor_floats(L.T_TOKEN_EMBEDDING), 42, 0))
+    m.finalize()
+    toks = np.random.default_rng(43).integers(3, cfg.vocab_size, 300).astype(np.int32)
+    free = torch.cuda.mem_get_info()[0]
+    m.batch_create(2, 8)
+    before = m.batch_forward([0, 1], [0, 0], toks[:2])[0]
+    one_block = 64 * 4 * (3 * 2 * 11008 + 12 * (4096 + 64) + 2 * 4096 + 5120 + 192 * 11008 // 256)   # h13, parts, x and q, qkv, limbs
+    assert free - torch.cuda.mem_get_info()[0] < 2 * one_block                # (the rest: kernels that are loaded, caches)
+    m.prefill(toks, 0)
+    after = m.batch_forward([0, 1], [0, 0], toks[:2])[0]
+    assert np.array_equal(before, after)
+    m.prefill(toks[:30], 300)
+    assert np.array_equal(before, m.batch_forward([0, 1], [0, 0], toks[:2])[0])
+    assert m.stats().device_status == 0
+    m.close()
+
+
 def test_full_batch_of_64_at_the_110m_shape():
     cfg = syn.SHAPES["stories110M"]
     tensors = _tensors(cfg, 13)

@@ -198,4 +198,4 @@ def test_allocation_that_fails_half_way_can_be_made_again(what):
         assert float(np.abs(got - want).max()) <= (1e-4 * float(want.max() - want.min()) if what == "prefill" else 0.0), nth
         assert m.stats().device_status == 0
         m.close()
-    assert failures >= {"batch": 15, "prefill": 1, "sampler": 6}[what]
+    assert failures >= {"batch": 8, "prefill": 1, "sampler": 6}[what]
