@@ -126,7 +126,7 @@ __device__ int sequential_sum(float *v, int n, float &sum, float limit, bool kee
             if (tid == 0) {
                 float s = sum;
                 int hit = -1;
-                for (int i = i0; i < end && hit < 0 && s == s; i += 4) {
+                for (int i = i0; i < end && hit < 0; i += 4) {
                     float4 x = *reinterpret_cast<const float4 *>(v + i);
                     x.x = __fadd_rn(s, x.x);
                     x.y = i + 1 < n ? __fadd_rn(x.x, x.y) : x.x;
