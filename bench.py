@@ -266,7 +266,7 @@ def long_context_account(cfg, model, tensors, device: int, peak: float) -> dict:
         out["attention"] = {"pos": pos_mid, "us_per_layer": a["us"], "bytes_per_layer": a["bytes"], "gbs": a["gbs"],
                             "frac": a["gbs"] / peak, "where": "attention phase of the persistent kernel, in situ"}
         out["us_per_layer"] = split["us_per_layer"]
-    # the same prompt through l2j_prefill (64 positions per weight sweep on the tensor cores) beside the decode path
+    # the same prompt through l2j_prefill (up to 256 positions per weight sweep on the tensor cores) beside the decode path
     inputs = np.concatenate([[1], prompt[:n_prompt - 1]]).astype(np.int32)   # BOS, then the prompt: what each position is fed
     model.prefill(inputs, 0)
     import torch

@@ -184,7 +184,7 @@ L2J_API int l2j_batch_forward(l2j_ctx *ctx, int n, const int32_t *seq, const int
  * logits the device chooses the token the Java Sampler chooses, and only its id crosses PCIe (call
  * l2j_forward with logits == NULL).  The ProbIndex array the reference keeps across calls (and sorts whole,
  * stale entries included) is kept across calls here too.  temperature == 0 returns the arg-max
- * (Sampler.argmax).  Vocabularies of at most 39,000 tokens (the probabilities live in shared memory). */
+ * (Sampler.argmax).  Vocabularies of at most 39,936 tokens (the probabilities live in shared memory). */
 L2J_API int l2j_sampler_seed(l2j_ctx *ctx, int64_t seed);
 L2J_API int l2j_sample(l2j_ctx *ctx, float temperature, float topp, int *token);
 

@@ -1062,9 +1062,11 @@ static int create_impl(const l2j_config *cfg, int device, int first_layer, int l
         }
         c->use_fused = fused;
     }
-    // The per-step kernels of a shape whose launches give an SM one ring stage or less (64 KB) end together, and waiting for
-    // the kernel in front is cheaper than for 148 bumps of a counter: 303 -> 288 us per token at the 110M shape, 153 -> 148
-    // at 15M.  Where blocks end apart the counters win (7B shape 1862 -> 1853, 20 layers of 13B 1566 -> 1549).
+    // Where the launches of a layer give an SM little to do (on average one ring stage, 64 KB, or less) its blocks end together,
+    // and waiting for the kernel in front is cheaper than for 148 bumps of a counter.  12 layers, us per token with counters
+    // and with waits, by MB of matrices in a layer: 1 (dim 288) 283 / 276, 7 (768) 305 / 291, 20 (1280) 400 / 378, 28 (1536)
+    // 416 / 389; beside the line at 38.8: 39 (1792) 459 / 441; 64 (2304) 508 / 503, 79 (2560) 520 / 529, 113 (3072) 574 / 581.
+    // So the two meet at about 70 MB; the line is on the safe side of that.
     if (tp_size == 1 && c->use_ring && !c->use_fused && !(flags & (L2J_F_STEP_KERNELS | L2J_F_NO_PDL)) && !getenv("L2J_CHAIN")) {
         const int64_t layer = 2 * (int64_t)c->dim * (c->dim + c->kv_dim) + 3 * (int64_t)c->dim * c->hidden;
         if (layer / 4 <= (int64_t)65536 * c->sm_count) {

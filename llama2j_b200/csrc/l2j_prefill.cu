@@ -718,17 +718,17 @@ struct PfAttnParams {
 // 2^-24 of the result are added, the smallest first, into a fresh FP32 accumulator per tile; the running output is
 // kept and rescaled in FP32 registers, so no sum is longer than one tile in the tensor cores' accumulator.
 //
-//   warps 0-3    softmax, the longest of the roles (one warp per scheduler; 1 / sqrt(head size) is applied to Q, masks only
-//                where a tile needs them: 83.7 -> 81.8 ms below): thread = query row; S from tensor memory, online maximum and sum, the three pieces of P back
-//                into tensor memory (the A operand of the second product)
+//   warps 0-3    softmax, one warp per scheduler: thread = query row; S from tensor memory, online maximum and sum, the three
+//                pieces of P back into tensor memory (the A operand of the second product).  1 / sqrt(head size) is applied
+//                to Q, and only tiles that need masks have them
 //   warps 4-11   K and V of the tile from global memory through registers into their pieces in shared memory (V
 //                transposed: both operands K-major, 128-byte swizzle); the output row of the query in registers
-//   warp 12      issue: S(j + 1) = Q K' while the softmax works on tile j, then O(j) = P V
+//   warp 12      issue, the longest of the roles: S(j + 1) = Q K' while the softmax works on tile j, then O(j) = P V
 //
 // Six bf16 products of 128 x 64 x HEAD, twice per tile, are 3072 tensor-core cycles at head size 128; on the FP32 units
 // the same tile takes 16384 cycles at best.  A tile takes 8000, 6900 of them the issue of its 72 instructions (48 wider
-// ones took as long).  3840 tokens through 16 layers of the 7B shape: 144 ms with the FP32 kernel
-// before this one (4 x 4 scores per thread), 88 ms with it.  Error against float64 the same or lower (3.4e-6 against 3.6e-6
+// ones took as long); the softmax warps wait for 3400 of theirs.  3840 tokens through 16 layers of the 7B shape: 144 ms with
+// the FP32 kernel before this one (4 x 4 scores per thread), 88 ms with it; scale and masks as above: 83.7 -> 81.8 ms.  Error against float64 the same or lower (3.4e-6 against 3.6e-6
 // of a row of V behind it, mean over head sizes 64 and 128 and peaked softmaxes).
 constexpr int kAttnQ = 128;      // queries per block: the rows of one accumulator
 constexpr int kAttnKeys = 64;    // keys per tile
@@ -1257,8 +1257,9 @@ __global__ void __launch_bounds__(kBdThreads) bd_attention_kernel(const BdAttnPa
     }
 }
 
-// Key ranges per (head, token): enough blocks for six on every SM, whatever the lengths turn out to be (the captured
-// step serves all of them); ranges that a short sequence leaves empty cost a block that ends at once.
+// Key ranges per (head, token): enough blocks for six on every SM.  The captured step serves all lengths, so the choice knows
+// the number of entries only: ranges that a short sequence leaves empty cost a block that ends at once, and a long sequence
+// among many short ones (from 28 entries at 32 heads on: one range) is scanned by one block per head.
 int bd_splits(int heads, int nv, int sms)
 {
     const int ns = (6 * sms) / (heads * nv);

@@ -125,7 +125,7 @@ class Transformer:
         return x_out
 
     def prefill(self, tokens, pos0: int = 0) -> None:
-        """Positions pos0 .. pos0 + len(tokens) - 1 in batches of 64 on the tensor cores; tokens[i] is the input
+        """Positions pos0 .. pos0 + len(tokens) - 1 in chunks of up to 256 on the tensor cores; tokens[i] is the input
         token of position pos0 + i (BOS, then the prompt: Run.java:614,635-637).  No logits."""
         t = np.ascontiguousarray(tokens, dtype=np.int32).reshape(-1)
         ptr = t.ctypes.data_as(C.POINTER(C.c_int32)) if t.size else None
