@@ -271,7 +271,8 @@ L2J_API int l2j_debug_desync(l2j_ctx *ctx);
 
 /* The same for allocations: the nth device or pinned allocation that the context makes from now on (prompt
  * workspaces, caches of concurrent sequences, sampler: whatever is made on first use) fails as if memory had run
- * out; 0 takes the injection back.  The call answers with an error and may be made again. */
+ * out; 0 takes the injection back.  The call answers with L2J_E_NOMEM and may be made again, or takes a way that
+ * needs less (l2j_prefill: chunks of 64 positions, or the decode step). */
 L2J_API int l2j_debug_fail_alloc(l2j_ctx *ctx, int nth);
 
 L2J_API int l2j_get_stats(l2j_ctx *ctx, l2j_stats *out);

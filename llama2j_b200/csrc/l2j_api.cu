@@ -2572,7 +2572,7 @@ int status_of(SeqState *dev_state)
 // Large arrays go through pinned staging buffers on several host threads, each with a stream of its own: one thread's
 // copies between pageable and pinned memory move 5 to 10 GB/s and the link more than 50, and the runtime's own staging
 // of a pageable copy is one thread's.  The buffers are those of this call (10 MB pinned, 10 MB on the device).
-// Host to host, ms, in one piece and this way (medians over boxes of 16 cores; single calls scatter by half): 45 M floats (a
+// Host to host, ms, in one piece and this way (medians, hosts of 16 cores; single calls scatter by half): 45 M floats (a
 // W1 matrix of the 7B shape) 28-29 and 19-22, 128 Mi 80-82 and 38-40.
 constexpr int64_t kStagedPiece = (int64_t)kGroup << 10;     // floats per piece: 1 MB
 constexpr int64_t kStagedFloats = (int64_t)kGroup << 17;    // from 32 Mi floats on (22-24 and 19-25 ms): making buffers and

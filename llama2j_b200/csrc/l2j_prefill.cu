@@ -728,8 +728,9 @@ struct PfAttnParams {
 // Six bf16 products of 128 x 64 x HEAD, twice per tile, are 3072 tensor-core cycles at head size 128; on the FP32 units
 // the same tile takes 16384 cycles at best.  A tile takes 8000, 6900 of them the issue of its 72 instructions (48 wider
 // ones took as long); the softmax warps wait for 3400 of theirs.  3840 tokens through 16 layers of the 7B shape: 144 ms with
-// the FP32 kernel before this one (4 x 4 scores per thread), 88 ms with it; scale and masks as above: 83.7 -> 81.8 ms.  Error against float64 the same or lower (3.4e-6 against 3.6e-6
-// of a row of V behind it, mean over head sizes 64 and 128 and peaked softmaxes).
+// the FP32 kernel before this one (4 x 4 scores per thread), 88 ms with it; scale and masks as above: 83.7 -> 81.8 ms.
+// Error against float64 the same or lower (3.4e-6 against 3.6e-6 of a row of V behind it, mean over head sizes 64 and 128
+// and peaked softmaxes).
 constexpr int kAttnQ = 128;      // queries per block: the rows of one accumulator
 constexpr int kAttnKeys = 64;    // keys per tile
 constexpr int kAttnSoft = 4, kAttnCvt = 8;              // warps by role
