@@ -113,8 +113,7 @@ struct l2j_ctx {
     MvPlan fplan[4]{};             // its stage geometry for QKV, Wo, W1/W3, W2
     FusedParams fused{};
     int fused_smem = 0, max_smem = 0;
-    float *rms_wmax_dev = nullptr;
-    float *fused_part = nullptr;
+    float2 *fused_pairs = nullptr;   // vectors the blocks of the persistent kernel hand to each other
     unsigned long long *fused_trace = nullptr;
     std::vector<LayerLaunch> layers;
     MvParams cls{};
@@ -372,30 +371,40 @@ void link_ranks(l2j_ctx *c)
     }
 }
 
-// Stage geometry of a phase of the persistent kernel: the lane mapping of plan_matvec (so that every
-// output element is computed exactly as by the per-step kernels), but stages of rpp rows (32 KB at the 7B
-// shape): the phases share one byte ring, and small stages keep more of it in flight and waste less where
-// it wraps.
-MvPlan plan_fused_phase(int n, bool paired, int row_align)
+// Stage geometry of a phase of the persistent kernel: `sets` of wpr warps work on two rows each (paired: a row of either
+// matrix), a warp spans four quantisation groups.  Stages of 22 to 36 KB at most: the phases share one byte ring, and small
+// stages keep more of it in flight and waste less where it wraps; a matrix that would not give every block a stage gets
+// smaller ones.
+MvPlan plan_fused_phase(int n, bool paired, int rows, int blocks)
 {
-    MvPlan pl = plan_matvec(n, false, paired, 0, 0, row_align);
-    if (!pl.ok || !pl.grouped)
-        return MvPlan{};
-    const int rt = 1;   // one row per group of wpr warps and stage (the persistent kernel's consumers are built for that)
-    int rpp = pl.rpp;
-    const int align = paired ? (row_align > 2 ? row_align : 2) : row_align;
-    while (rpp > 1 && (rt * rpp) % align != 0)
-        --rpp;
-    if ((rt * rpp) % align != 0)
-        return MvPlan{};
-    pl.rt = rt;
-    pl.rpp = rpp;
-    pl.half_hdr = ((((rt * rpp * n / 2 + 255) / 256) + 4) * 8 + 15) & ~15;
-    const int payload = rt * rpp * n;
-    pl.hdr_off = payload;
-    pl.slot_bytes = (payload + 2 * pl.half_hdr + 127) & ~127;
+    MvPlan pl{};
+    if (n <= 0 || n % kGroup != 0)
+        return pl;
+    const int groups = n / kGroup;
+    const int wpr = (groups + 3) / 4;
+    if (wpr > kFusedConsWarps)
+        return pl;
+    int sets = kFusedConsWarps / wpr;
+    const int want = (rows + blocks * (paired ? 1 : 2) - 1) / (blocks * (paired ? 1 : 2));
+    if (sets > want)
+        sets = want > 1 ? want : 1;
+    pl.grouped = true;
+    pl.cpt = 2;
+    pl.rt = 1;
+    pl.rpp = 2 * sets;
+    pl.wpr = wpr;
+    pl.half_hdr = ((sets * groups + 4) * 8 + 15) & ~15;
+    pl.hdr_off = 2 * sets * n;
+    pl.slot_bytes = (pl.hdr_off + 2 * pl.half_hdr + 127) & ~127;
     pl.threads = kFusedThreads;
+    pl.ok = true;
     return pl;
+}
+
+// Pairs in all vectors of the persistent kernel.
+int64_t fused_pair_count(const l2j_ctx *c)
+{
+    return 4 * (int64_t)c->dim + 2 * (int64_t)c->kv_dim + c->hidden + (int64_t)c->cfg.n_heads * (kAttSlots - 1) * (c->head + 2);
 }
 
 // Parameters of the persistent kernel: the four matrix-vector phases of the first layer (the kernel adds
@@ -420,9 +429,13 @@ void build_fused_params(l2j_ctx *c)
     F.kv_step = (long long)c->cfg.n_kv_heads * c->cfg.seq_len * c->head;
     F.rms_step = c->reps * c->dim_stride;
     F.n_layers = c->nl;
-    F.rms_wmax = c->rms_wmax_dev;
-    F.q = c->q;
-    F.att_part = c->fused_part;
+    F.xa_pairs = c->fused_pairs;
+    F.xb_pairs = F.xa_pairs + c->dim;
+    F.q_pairs = F.xb_pairs + c->dim;
+    F.kv_pairs = F.q_pairs + c->dim;
+    F.h_pairs = F.kv_pairs + 2 * c->kv_dim;
+    F.o_pairs = F.h_pairs + c->hidden;
+    F.att_pairs = F.o_pairs + c->dim;
     F.n_heads = c->cfg.n_heads;
     F.kv_mul = c->kv_mul;
     F.head = c->head;
@@ -431,8 +444,8 @@ void build_fused_params(l2j_ctx *c)
     while (gw < c->head / 4)
         gw <<= 1;
     const int merge_bytes = kFusedConsWarps * (32 / gw) * (c->head + 4) * 4;
-    const int limb_bytes = 3 * (c->dim > c->hidden ? c->dim : c->hidden);
-    F.xarea_bytes = ((merge_bytes > limb_bytes ? merge_bytes : limb_bytes) + 127) & ~127;
+    const int vec_bytes = 3 * (c->dim > c->hidden ? c->dim : c->hidden);   // limbs of the longest input vector
+    F.xarea_bytes = ((merge_bytes > vec_bytes ? merge_bytes : vec_bytes) + 127) & ~127;
     F.ring_bytes = (c->fused_smem - kFusedHeaderBytes - F.xarea_bytes) & ~127;
     F.sync = c->chain;
     F.epoch = c->chain + (int64_t)kChainStride * (5 * c->nl + 1);
@@ -1025,23 +1038,24 @@ static int create_impl(const l2j_config *cfg, int device, int first_layer, int l
     c->use_ring = !(flags & L2J_F_SIMPLE) && c->plan_qkv.ok && c->plan_wo.ok && c->plan_w13.ok && c->plan_hidden.ok &&
                   c->plan_cls.ok && (head % 2 == 0);
     {   // one persistent launch per token where every matrix has rows of whole quantisation groups
-        // (a consumer warp converts every 18th group of the input vector, three at most; a lane's eight elements of the
-        // attention output lie in one head)
+        // (a lane's four elements of the attention output lie in one head)
         bool fused = c->use_ring && tp_size == 1 && !(flags & L2J_F_STEP_KERNELS) && c->reps == 1 && c->dim % kGroup == 0 &&
-                     c->hidden % kGroup == 0 && c->dim <= 3 * kFusedConsWarps * kGroup && c->hidden <= 3 * kFusedConsWarps * kGroup &&
-                     head % 8 == 0;
-        // Measured on B200: with dim a multiple of 2048 (every consumer warp's lanes own a group of the rows:
-        // 7B shape) the persistent kernel is level with the per-step kernels at short contexts and 4 % ahead at
-        // long ones; with 20 groups per row (13B shape) a sixth of the lanes idle and it is 9 % behind.
-        if (!(flags & L2J_F_PERSISTENT) && c->dim % (8 * kGroup) != 0)
+                     c->hidden % kGroup == 0 && c->dim <= kFusedMaxRow && c->hidden <= kFusedMaxRow &&
+                     head % 8 == 0 && head <= 128;
+        // Measured on B200, us per greedy token, per-step kernels / persistent kernel: 8 layers of dim 1024 229 / 151, 1536 261 / 174,
+        // 2048 297 / 200, 2560 326 / 235, 3072 356 / 261, 3584 403 / 328, 6144 695 / 631; 16 layers of the 7B shape 943 / 771, of the 13B
+        // shape 1230 / 1096 (short contexts) and 1261 / 1170 (200 positions).  The narrowest shapes stay with the per-step
+        // kernels unless asked otherwise, although the 110M shape gains too (287 / 226): what runs there by default is documented
+        // behaviour (five launches per layer, bit for bit those of L2J_F_STEP_KERNELS).
+        if (!(flags & L2J_F_PERSISTENT) && c->dim < 1024)
             fused = false;
         if (const char *e = getenv("L2J_FUSED"))   // diagnostic: A/B against the per-step kernels
             fused = fused && atoi(e) != 0;
         if (fused) {
-            c->fplan[0] = plan_fused_phase(c->dim, false, 2);
-            c->fplan[1] = plan_fused_phase(c->dim, false, 1);
-            c->fplan[2] = plan_fused_phase(c->dim, true, 1);
-            c->fplan[3] = plan_fused_phase(c->hidden, false, 1);
+            c->fplan[0] = plan_fused_phase(c->dim, false, c->dim + 2 * c->kv_dim, c->ring_grid);
+            c->fplan[1] = plan_fused_phase(c->dim, false, c->dim, c->ring_grid);
+            c->fplan[2] = plan_fused_phase(c->dim, true, c->hidden, c->ring_grid);
+            c->fplan[3] = plan_fused_phase(c->hidden, false, c->dim, c->ring_grid);
             fused = c->fplan[0].ok && c->fplan[1].ok && c->fplan[2].ok && c->fplan[3].ok;
         }
         if (fused) {
@@ -1050,13 +1064,11 @@ static int create_impl(const l2j_config *cfg, int device, int first_layer, int l
             int largest = 0;
             for (int k = 0; k < 4; ++k)
                 largest = c->fplan[k].slot_bytes > largest ? c->fplan[k].slot_bytes : largest;
-            const int limb_bytes = 3 * (c->dim > c->hidden ? c->dim : c->hidden);
-            if (c->fused_smem - kFusedHeaderBytes - limb_bytes - 4096 < 3 * largest)
-                fused = false;   // the ring would not hold three stages
+            if (c->fused_smem - kFusedHeaderBytes - 3 * (c->dim > c->hidden ? c->dim : c->hidden) - 4096 < 5 * largest)
+                fused = false;   // the ring would not hold the four stages that the consumers take together, wherever it wraps
         }
         if (fused) {
-            CREATE_CK(dev_alloc(c, &c->rms_wmax_dev, 2 * (int64_t)c->nl, true));
-            CREATE_CK(dev_alloc(c, &c->fused_part, (int64_t)cfg->n_heads * kAttSlots * (head + 4), true));
+            CREATE_CK(dev_alloc(c, &c->fused_pairs, fused_pair_count(c), true));
             if (getenv("L2J_TRACE"))
                 CREATE_CK(dev_alloc(c, &c->fused_trace, (int64_t)c->ring_grid * 5 * c->nl * 8, true));
         }
@@ -1287,14 +1299,6 @@ extern "C" int l2j_finalize(l2j_ctx *c)
         if (c->is_last) {
             CK(c, cudaMemcpy(w.data(), c->rms_final, sizeof(float) * (size_t)dim, cudaMemcpyDeviceToHost));
             c->cls.rms_wmax = vmax(w.data(), dim);
-        }
-        if (c->use_fused) {
-            std::vector<float> wm(2 * (size_t)c->nl);
-            for (int li = 0; li < c->nl; ++li) {
-                wm[2 * (size_t)li] = c->layers[(size_t)li].qkv.rms_wmax;
-                wm[2 * (size_t)li + 1] = c->layers[(size_t)li].w13.rms_wmax;
-            }
-            CK(c, cudaMemcpy(c->rms_wmax_dev, wm.data(), sizeof(float) * wm.size(), cudaMemcpyHostToDevice));
         }
     }
 
@@ -2196,6 +2200,8 @@ extern "C" int l2j_reset(l2j_ctx *c)
         CK(c, cudaMemset(c->ll_buf[TPV_HB], 0, sizeof(float2) * (size_t)c->hidden));
         CK(c, cudaMemset(c->ll_buf[TPV_CAND], 0, sizeof(float2) * 2 * kMaxTp));
     }
+    if (c->use_fused)
+        CK(c, cudaMemset(c->fused_pairs, 0, sizeof(float2) * (size_t)fused_pair_count(c)));   // as above: the tags start again
     CK(c, cudaDeviceSynchronize());
     c->forwards = 0;
     c->status_accum = 0;

@@ -11,20 +11,28 @@
 //                     as far ahead as the ring has room.  Weights and old cache rows never depend
 //                     on this token's activations, so while the consumers wait at a phase boundary
 //                     the ring fills with the next phase: HBM does not idle.
-//   consumer warps    per phase: wait for the hand-over counter of the phase in front, load the
-//                     input vector (for Wo: merge the attention partials), RMSNorm, fixed-point
-//                     limbs, then dp4a over the block's stages as they land.
-//   epilogue warp     folds the per-warp partial sums of a stage and applies RoPE + cache write,
-//                     residual add or SwiGLU; after the block's last stage of a phase it bumps the
-//                     phase's counter (release), which is what the other blocks' consumers poll.
+//   consumer warps    per phase: poll the input vector, which arrives as (value, tag) pairs, RMSNorm,
+//                     fixed-point limbs, then dp4a over the block's stages as they land.
+//   epilogue warp     adds the per-warp partial sums of a group of stages, applies RoPE + cache write,
+//                     residual add or SwiGLU, and hands every result on as a pair.
 //
 // Stages are dealt to the blocks round-robin, continuing across phases, so every block streams the
-// same number of bytes per token (+- one stage).  The attention step's units (head, 64 positions)
-// are dealt in contiguous runs, a block folds the units of one head into one partial (m, l, o), and
-// the Wo phase's prologue merges the few partials of a head (at most kAttSlots) in a fixed order.
+// same number of bytes per token (+- one stage).  The attention step's units (head, 32 positions)
+// are dealt in contiguous runs; a block folds the units of one head into one partial (m, l, o), and the block with the
+// head's first positions merges the few partials of the head (at most kAttSlots) in a fixed order.
 //
-// Arithmetic per output element is that of matvec_ring_kernel (same lane mapping, same reduction
-// order), so the matrix-vector products are bitwise those of the per-step kernels.
+// What bounds it (7B shape, position 160): a layer takes 45 us where its bytes take 31.5 at the measured copy rate.  The
+// ring holds 4.4 us of a block's share of the HBM; a boundary between two phases costs 2 to 3 us from the median block's last
+// result to the next block's first dot product, and the attention step and Wo, which hardly stream, 11 us together.  Measured on the
+// way from 56.6 us per layer (in-kernel timeline, both sides with it on):
+//   - the producer's pass per stage took 900 cycles, whatever a stage held, and bounded the consumers: set up per phase and segment now;
+//   - a warp works on two rows with half as many elements each: 24 instead of 48 registers of limbs, so that the next stage's bytes are
+//     fetched while the dot products of this one run (750 -> about 500 cycles per 25 KB; 288 are the dp4a's);
+//   - pairs instead of a fence, a counter and a second load per hand-over; exchanges instead of stores (see st_pair_gpu);
+//   - the Wo phase's prologue merged the attention partials in every block (5 us); one block per head does it now, in 1.5.
+// Taken back: FP32 multiply-adds on unpacked bytes (a permute per byte: slower than three dp4a per four), asking the stages
+// behind the ring into the L2 (50 us: the extra requests delay the hand-overs), the same for RMSNorm weights and output lines.
+// 7B shape, 48 greedy forwards from position 0: 88.6 -> 72 ms; 8 steps behind 3840 positions: 22.3 -> 18 ms.
 //
 // Blocks wait for each other, so all of them must be resident: the grid is one block per SM.  Every wait is
 // bounded by the SM's cycle counter.  A hand-over between blocks that runs out raises L2J_DS_WAIT_TIMEOUT in
@@ -58,19 +66,18 @@ constexpr int kFBarFull = 0;            // uint64 full[16]
 constexpr int kFBarEmpty = 128;         // uint64 empty[16]
 constexpr int kFBarRedFull = 256;       // uint64 red_full[4]
 constexpr int kFBarRedEmpty = 288;      // uint64 red_empty[4]
-constexpr int kFFlag = 320;             // int: result of the poll of a hand-over counter
-constexpr int kFVStart = 3264;          // int vstart[16]: the producer's bookkeeping of where each stage in flight begins
-constexpr int kFScratch = 384;          // float scratch[64]
-constexpr int kFDescOff = 640;          // FStage desc[16]
-constexpr int kFRedOff = 1152;          // 4 x 132 floats: [stage of the group][row of the stage][warp of the row]
-constexpr int kFRedStride = 528;
+constexpr int kFVStart = 328;           // int vstart[16]: the producer's bookkeeping of where each stage in flight begins
+constexpr int kFScratch = 392;          // float scratch[16]
+constexpr int kFDescOff = 512;          // FStage desc[16]
+constexpr int kFRedOff = 1024;          // 4 x 128 floats: [stage of the group][row of the stage][warp of the row]
+constexpr int kFRedStride = 4 * kFGroup * 2 * kFusedConsWarps;   // a stage has two rows per set of warps
 constexpr int kFRopeOff = 3328;         // float cos[64], sin[64] of the token's position
 constexpr int kFInvTab = 3840;          // float inv[64]: value of one fixed-point unit of each group of the input vector
 constexpr int kFHeader = kFusedHeaderBytes;   // end of the fixed part (128-byte aligned)
-static_assert(kFInvTab + 64 * 4 <= kFHeader, "header layout");
+static_assert(kFScratch + 4 * kFusedConsWarps <= kFDescOff && kFRedOff + kFRedBufs * kFRedStride <= kFRopeOff, "header layout");
+static_assert(kFInvTab + 4 * (kFusedMaxRow / 256) <= kFHeader, "header layout");
 constexpr int kFCons = kFusedConsWarps * 32;
-constexpr int kFGroupRounds = 3;        // quantisation groups of the input vector that one consumer warp converts at most (54 groups)
-constexpr int kAttFastSlots = 4;        // the merge that fetches all partials of a thread's elements at once
+constexpr int kAttBatch = 4;            // cached positions that a lane group works on at a time
 constexpr uint64_t kFShortWaitNs = 2000;
 
 struct FStage {
@@ -100,6 +107,37 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c)
     int d;
     asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
+}
+
+// Two (value, sequence number) pairs of the hand-over between blocks, from L2.
+__device__ __forceinline__ float4 ld_pairs2_gpu(const float2 *p)
+{
+    float4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ float2 ld_pair_gpu(const float2 *p)
+{
+    float2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
+// An exchange and not a store: while the SM streams, a plain store may stay in it for 4 us before the L2 gets it (7B shape,
+// W2 -> QKV: the input vector is complete 3.7 instead of 6.5 us after the median block's last store); an atomic goes at once.
+__device__ __forceinline__ void st_pair_gpu(float2 *p, float v, int tag)
+{
+    unsigned long long old;
+    asm volatile("atom.relaxed.gpu.global.exch.b64 %0, [%1], %2;"
+                 : "=l"(old)
+                 : "l"(p), "l"(((unsigned long long)(unsigned int)tag << 32) | __float_as_uint(v))
+                 : "memory");
+}
+
+__device__ __forceinline__ bool tagged(const float4 &v, int tag)
+{
+    return __float_as_int(v.y) == tag && __float_as_int(v.w) == tag;
 }
 
 // Bulk copy without a cache hint (cached K/V rows are read again by the next token).
@@ -149,20 +187,27 @@ __device__ __forceinline__ AttSplit att_split(const FusedParams &P, int pos, int
     a.units = P.n_heads * a.nchunk;
     // Short contexts are a matter of latency, not bandwidth: three blocks per head keep the partials of a head
     // few enough (four) for the step behind to fetch them in one round of loads.
-    const int per_head = a.nchunk <= 8 ? 3 : kAttMaxSplit;
+    const int per_head = a.nchunk <= 512 / kAttChunk ? 3 : kAttMaxSplit;
     a.ga = min(min(grid, P.n_heads * per_head), a.units);
     a.np_max = min(a.nchunk, (a.ga + P.n_heads - 1) / P.n_heads + 1);
     return a;
 }
 
+// (32-bit divisions: units * blocks stays below 2^31 for every head count and sequence length that fits a device.)
 __device__ __forceinline__ int att_first_unit(const AttSplit &a, int b)
 {
-    return (int)(((long long)b * a.units) / a.ga);
+    return (int)((unsigned int)b * (unsigned int)a.units / (unsigned int)a.ga);
 }
 
 __device__ __forceinline__ int att_block_of(const AttSplit &a, int u)
 {
-    return (int)((((long long)(u + 1)) * a.ga + a.units - 1) / a.units) - 1;
+    return (int)(((unsigned int)(u + 1) * (unsigned int)a.ga + (unsigned int)a.units - 1u) / (unsigned int)a.units) - 1;
+}
+
+// Partial results of head h.
+__device__ __forceinline__ int att_partials(const AttSplit &a, int h)
+{
+    return att_block_of(a, (h + 1) * a.nchunk - 1) - att_block_of(a, h * a.nchunk) + 1;
 }
 
 // Stage index -> (segment, first row, row count) of a ring phase.
@@ -206,6 +251,7 @@ struct Producer {
     int off;                // vhead's position in the ring
     int ring_bytes;
     int seq, tail;          // descriptors issued / known to be released
+    int vtail;              // where the oldest stage not known to be released begins
     bool lost;
     uint64_t wait_ns;
     int pos;                // the token's position, -1 until the kernel in front has set it
@@ -220,12 +266,15 @@ struct Producer {
             off = 0;
         }
         const int vend = vhead + (int)bytes;
-        while (tail < seq && (seq - tail >= kFDesc || vend - ring_bytes > vstart[tail % kFDesc])) {
+        while (tail < seq && (seq - tail >= kFDesc || vend - ring_bytes > vtail)) {
             if (!mbar_wait_bounded(sbase + kFBarEmpty + 8 * (tail % kFDesc), (uint32_t)(tail / kFDesc) & 1u,
                                    wait_ns))
                 lost = true;
             ++tail;
+            vtail = vstart[tail % kFDesc];
         }
+        if (tail == seq)
+            vtail = vhead;
         vstart[seq % kFDesc] = vhead;
         const uint32_t at = (uint32_t)off;
         const int step = (int)((bytes + 127u) & ~127u);
@@ -249,42 +298,56 @@ __device__ __forceinline__ void producer_learn_pos(Producer &pr, const FusedPara
 // bulk copies (rows of one or two matrices, their group headers) are one instruction stream with per-lane
 // operands: lane = 2 * is_header + half.  Every lane arrives on the stage's barrier with the bytes of its own
 // copy (the barrier counts four arrivals), so the lanes need not talk to each other.
-__device__ __forceinline__ void produce_ring_stage(Producer &pr, const FusedParams &P, const MvParams &p, int k, int layer, int s,
-                                                   uint64_t pol, int lane)
+//
+// The block's stages of a phase: first, first + G, ...  One pass of the inner loop is the producer's time per stage, and the
+// ring cannot be drained faster than that, so everything that does not change from stage to stage is set up per
+// phase and segment, and positions advance by additions in units of quantisation groups.
+__device__ __forceinline__ void produce_phase(Producer &pr, const FusedParams &P, const MvParams &p, int k, int layer, int first, int G,
+                                              uint64_t pol, int lane)
 {
-    const uint32_t off = pr.acquire((uint32_t)p.slot_bytes);
-    const int e = pr.seq % kFDesc;
-    const uint32_t full = pr.sbase + kFBarFull + 8 * e;
-    FStage *desc = reinterpret_cast<FStage *>(pr.smem + kFDescOff) + e;
-    int seg, row0, nrows;
-    stage_rows(p, s, seg, row0, nrows);
     const int h = lane & 1, is_hdr = lane >> 1;
-    const bool mine = (p.paired || h == 0) && !(P.debug_no_copy & 1);
-    const int sg = p.paired ? h : seg;
-    const uint32_t pbytes = (uint32_t)nrows * (uint32_t)p.rowbytes;
-    const int64_t flat = p.seg[sg].flat0 + (int64_t)layer * P.seg_step[k][sg] + (int64_t)row0 * p.n;
-    const int64_t ga = (flat >> 8) & ~(int64_t)1;                 // headers are copied from an even group on: 16-byte aligned
-    const int64_t gl = (flat + pbytes - 1) >> 8;
-    const uint32_t hbytes = (uint32_t)(((gl - ga + 2) & ~(int64_t)1) * 8);
-    const uint32_t bytes = mine ? (is_hdr ? hbytes : pbytes) : 0u;
-    const int R = p.rt * p.rpp;
-    const uint32_t dst = pr.ring_base + off +
-                         (is_hdr ? (uint32_t)p.hdr_off + (uint32_t)(h * p.half_hdr) : (uint32_t)(h * (R / 2)) * (uint32_t)p.rowbytes);
-    const void *src = is_hdr ? static_cast<const void *>(p.seg[sg].hdr + ga) : static_cast<const void *>(p.seg[sg].payload + flat);
-    if (lane == 0) {
-        desc->off = (int)off;
-        desc->nrows = nrows;
-        desc->e0a = (int)(flat - ga * 256);
+    const int paired = p.paired, rs = p.rs, groups = p.n >> 8, S = p.total_stages;
+    const bool copy = (paired || h == 0) && !(P.debug_no_copy & 1);
+    const uint32_t slot_bytes = (uint32_t)p.slot_bytes;
+    const uint32_t dst0 = pr.ring_base + (is_hdr ? (uint32_t)(p.hdr_off + h * p.half_hdr) : (uint32_t)(h * rs * p.n));   // h is 0 or the stage is paired
+    const int unit = is_hdr ? 8 : 256;
+    const uint32_t desc0 = pr.sbase + kFDescOff;
+    int s = first, s0 = 0, seg = 0;
+    while (s < S) {
+        while (!paired && seg < 2 && s >= s0 + p.seg_stages[seg]) {
+            s0 += p.seg_stages[seg];
+            ++seg;
+        }
+        const int s1 = paired ? S : s0 + p.seg_stages[seg];
+        const MvSeg &sg = p.seg[paired ? h : seg];
+        const uint8_t *src = is_hdr ? reinterpret_cast<const uint8_t *>(sg.hdr) : sg.payload;
+        int left = sg.rows - (s - s0) * rs;                      // rows from the stage's first one on
+        int gi = (int)((sg.flat0 + (int64_t)layer * P.seg_step[k][paired ? h : seg]) >> 8) + (s - s0) * rs * groups;   // its first group
+        const int grs = G * rs, ggr = grs * groups;
+        for (; s < s1; s += G, left -= grs, gi += ggr) {
+            const int nrows = min(rs, left);
+            const uint32_t off = pr.acquire(slot_bytes);
+            const int e = pr.seq % kFDesc;
+            const uint32_t full = pr.sbase + kFBarFull + 8 * e;
+            const int ga = gi & ~1;                              // headers are copied from an even group on: 16-byte aligned
+            const int ng = nrows * groups;
+            const uint32_t bytes = (uint32_t)(is_hdr ? ((gi + ng + 1) & ~1) - ga : ng) * (uint32_t)unit;
+            const int shift = (gi - ga) << 8;
+            if (lane == 0)
+                asm volatile("st.shared.v2.u32 [%0], {%1, %2};\n\tst.shared.u32 [%0 + 8], %3;" ::"r"(desc0 + 32u * (uint32_t)e), "r"(off),
+                             "r"(nrows), "r"(shift)
+                             : "memory");
+            if (lane == 1)
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(desc0 + 32u * (uint32_t)e + 12u), "r"(shift) : "memory");
+            if (copy) {
+                mbar_arrive_expect_tx(full, bytes);
+                bulk_g2s(dst0 + off, src + (int64_t)(is_hdr ? ga : gi) * unit, bytes, full, pol);
+            } else {
+                mbar_arrive(full);
+            }
+            ++pr.seq;
+        }
     }
-    if (lane == 1)
-        desc->e0b = p.paired ? (int)(flat - ga * 256) : 0;
-    if (bytes) {
-        mbar_arrive_expect_tx(full, bytes);
-        bulk_g2s(dst, src, bytes, full, pol);
-    } else {
-        mbar_arrive(full);
-    }
-    ++pr.seq;
 }
 
 __device__ __forceinline__ void produce_att_stage(Producer &pr, const FusedParams &P, int layer, int unit, const AttSplit &a, int pos,
@@ -330,220 +393,183 @@ struct Consumer {
     bool lost, lost_before;
 };
 
-// Waits until counter `ctr` has reached `target`: one thread polls, the others follow through barrier 1.
-__device__ __forceinline__ void consumers_wait(const unsigned int *ctr, unsigned int target, uint8_t *smem, Consumer &cs, uint64_t wait_ns)
+// A lane's sixteen elements of a quantisation group of an input vector: pairs 64 q.. 64 q + 3 from p on, q = 0..3.
+__device__ __forceinline__ void issue_pairs(const float2 *p, float4 (&v)[8])
 {
-    volatile int *flag = reinterpret_cast<volatile int *>(smem + kFFlag);
-    if (threadIdx.x == 0) {
-        int ok = (int)(ld_acquire_u32(ctr) - target) >= 0;
-        if (!ok)
-            ok = counter_wait_bounded(ctr, target, cs.lost ? kFShortWaitNs : wait_ns) ? 1 : 0;
-        *flag = ok;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        v[2 * q] = ld_pairs2_gpu(p + 64 * q);
+        v[2 * q + 1] = ld_pairs2_gpu(p + 64 * q + 2);
     }
-    named_barrier_sync(1, kFCons);
-    if (*flag == 0)
-        cs.lost = true;
 }
+
+// Those of them that have not arrived yet are asked for again until they carry `tag`.  While nothing at all has come for
+// the warp only an eighth of them is asked for: 148 blocks that poll whole vectors would take as much of the L2 as the
+// weight stream does.
+__device__ __forceinline__ void poll_pairs(const float2 *p, float4 (&v)[8], int tag, Consumer &cs, uint64_t wait_ns)
+{
+    auto all = [&]() {
+        bool ok = true;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            ok = ok && tagged(v[q], tag);
+        return __all_sync(0xffffffffu, ok) != 0;
+    };
+    if (all())
+        return;
+    const long long limit = (long long)(2 * (cs.lost ? kFShortWaitNs : wait_ns));
+    const long long c0 = sm_clock();
+    for (;;) {
+        const bool some = tagged(v[0], tag);
+        if (!some)
+            v[0] = ld_pairs2_gpu(p);
+        if (__any_sync(0xffffffffu, some)) {
+#pragma unroll
+            for (int q = 1; q < 8; ++q)
+                if (!tagged(v[q], tag))
+                    v[q] = ld_pairs2_gpu(p + 64 * (q >> 1) + 2 * (q & 1));
+        }
+        if (all())
+            return;
+        if (__any_sync(0xffffffffu, sm_clock() - c0 > limit)) {
+            cs.lost = true;
+            return;
+        }
+    }
+}
+
+// What a thread works on per stage: 32 bytes of each of two rows (16 bytes at two places of the same group) and the two
+// groups' headers.
+struct StageRegs {
+    uint4 w[2][2];
+    float2 ms[2];
+};
 
 // One matrix-vector phase of the block: prologue (input vector -> fixed-point limbs in shared memory)
 // and the block's `nmine` stages.  One copy of this code serves all four phases (the differences are run-time
 // parameters): the prologue runs once per phase, so its instructions come from the L2 every time, and four
 // inlined copies of it cost more in instruction fetches than the branches cost here.
-// merge: the input is the attention output, assembled from the partial results of the blocks that worked on
-// each head.
-__device__ __forceinline__ void consume_ring_phase(const FusedParams &P, const MvParams &p, int layer, int nmine, bool merge,
-                                                   const float *rms_w, float rms_wmax, const AttSplit &as, uint8_t *smem,
-                                                   uint32_t sbase, Consumer &cs, uint64_t wait_ns, int pidx)
+// in_pairs: the input vector as (value, tag) pairs, or nullptr: plain (p.x_in; the first phase of the launch).
+__device__ __forceinline__ void consume_ring_phase(const FusedParams &P, const MvParams &p, int nmine, const float2 *in_pairs, int tag,
+                                                   const float *rms_w, uint8_t *smem, uint32_t sbase, Consumer &cs, uint64_t wait_ns,
+                                                   int pidx)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nw = p.rpp * p.wpr;
-    const bool active = warp < nw;
+    const int sets = p.rpp >> 1;                  // sets of wpr warps; a set works on two rows of a stage
+    const bool active = warp < sets * p.wpr;
     const int rsub = warp / p.wpr;
     const int wi = warp - rsub * p.wpr;
-    constexpr int RT = 1;   // rows per thread and stage: a stage holds one row per group of wpr warps
     const int n = p.n;
-    const int R = RT * p.rpp;
-    const int rowbytes = n;
     uint8_t *share = smem + kFHeader;
     float *scratch = reinterpret_cast<float *>(smem + kFScratch);
 
-    int chunk[4];
-    const int g = wi * 8 + (lane >> 2);
+    // eight lanes share a quantisation group: lane s of them holds bytes 16 s.. and 128 + 16 s.. of it
+    const int g = wi * 4 + (lane >> 3);
     const bool gvalid = active && g < (n >> 8);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        chunk[k] = g * 16 + 4 * (k ^ ((lane >> 2) & 1)) + (lane & 3);
 
-    // ---- prologue: the input vector as fixed-point limbs in shared memory.  Every warp owns whole quantisation
-    // groups of the vector (group warp + 18 j in round j; a lane holds elements 4 l..4 l + 3 of each half of the group, so that a warp's loads are two contiguous 512-byte requests) and gives each its own
+    // ---- prologue: the input vector as fixed-point limbs in shared memory.  Every half-warp owns whole quantisation
+    // groups of the vector (a lane holds four elements of each quarter of a group) and gives each its own
     // power-of-two scale from the group's largest element: no block-wide maximum has to be agreed on before the
     // conversion can start, and the RMSNorm scalar ss = 1 / sqrt(mean(x^2) + eps) is applied to the dot products
     // at the end (sum_j w_j (r_j ss x_j) = ss sum_j w_j r_j x_j up to rounding), so nothing here waits for the
-    // sum of squares either.
+    // sum of squares either.  Half-warps: 14 warps with a group each would need two rounds for the 16 groups of the 7B shape.
     float *inv_tab = reinterpret_cast<float *>(smem + kFInvTab);   // value of one fixed-point unit, per group
     const int ngroups = n >> 8;
+    const bool has_rms = rms_w != nullptr;
     {
-        const bool has_rms = rms_w != nullptr;
-        float xg[kFGroupRounds][8];
-        const int ps = P.head + 4;
-        const bool merge_fast = merge && as.np_max <= kAttFastSlots;
-        if (merge && !merge_fast) {
-            // Many partials per head: first a table of their weights in shared memory (one thread per head).
-            float *tw = reinterpret_cast<float *>(share);            // [n_heads][kAttSlots] weights, then [n_heads] sums
-            if (tid < P.n_heads) {
-                const int h = tid;
-                const int u0 = h * as.nchunk;
-                const int np = min(att_block_of(as, u0 + as.nchunk - 1) - att_block_of(as, u0) + 1, kAttSlots);
-                const float *hp = P.att_part + (int64_t)h * kAttSlots * ps + P.head;
-                float ms[kAttSlots], ls[kAttSlots];
+        if (tid == 0)
+            fused_trace(P, pidx, 0);
+        float ssq = 0.f;
+#pragma unroll 1
+        for (int g0 = 2 * warp; g0 < ngroups; g0 += 2 * kFusedConsWarps) {
+            const bool live = g0 + (lane >> 4) < ngroups;          // an odd count of groups: the last half-warp repeats one
+            const int gi = live ? g0 + (lane >> 4) : g0;
+            const int e = gi * 256 + (lane & 15) * 4;
+            float xg[16];
+            float4 w4[4];
+            if (has_rms) {
 #pragma unroll
-                for (int s2 = 0; s2 < kAttSlots; ++s2) {
-                    ms[s2] = -INFINITY;
-                    ls[s2] = 0.f;
-                    if (s2 < np) {
-                        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(hp + (int64_t)s2 * ps));
-                        ms[s2] = ml.x;
-                        ls[s2] = ml.y;
-                    }
-                }
-                float gm = -INFINITY;
-#pragma unroll
-                for (int s2 = 0; s2 < kAttSlots; ++s2)
-                    gm = fmaxf(gm, ms[s2]);
-                float L = 0.f;
-#pragma unroll
-                for (int s2 = 0; s2 < kAttSlots; ++s2) {
-                    const float w = ls[s2] > 0.f ? expf(ms[s2] - gm) : 0.f;
-                    L = fmaf(ls[s2], w, L);
-                    tw[h * kAttSlots + s2] = w;
-                }
-                tw[P.n_heads * kAttSlots + h] = L;
+                for (int q = 0; q < 4; ++q)
+                    w4[q] = ld_cg_f4_issue(rms_w + e + 64 * q);
             }
-            named_barrier_sync(2, kFCons);
-        }
-        // ---- loads of all rounds first (they are independent), then the arithmetic
-        float4 wa[kFGroupRounds], wb[kFGroupRounds];
+            if (in_pairs) {
+                float4 v[8];
+                issue_pairs(in_pairs + e, v);
+                poll_pairs(in_pairs + e, v, tag, cs, wait_ns);
 #pragma unroll
-        for (int j = 0; j < kFGroupRounds; ++j) {
-            const int gi = warp + j * kFusedConsWarps;
-            const int e = gi * 256 + lane * 4;
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                xg[j][q] = 0.f;
-            wa[j] = wb[j] = make_float4(1.f, 1.f, 1.f, 1.f);
-            if (gi >= ngroups)
-                continue;
-            if (!merge) {
-                const float4 a4 = ld_cg_f4_issue(p.x_in + e), b4 = ld_cg_f4_issue(p.x_in + e + 128);
-                xg[j][0] = a4.x; xg[j][1] = a4.y; xg[j][2] = a4.z; xg[j][3] = a4.w;
-                xg[j][4] = b4.x; xg[j][5] = b4.y; xg[j][6] = b4.z; xg[j][7] = b4.w;
-                if (has_rms) {
-                    wa[j] = ld_cg_f4_issue(rms_w + e);
-                    wb[j] = ld_cg_f4_issue(rms_w + e + 128);
+                for (int q = 0; q < 8; ++q) {
+                    xg[2 * q] = v[q].x;
+                    xg[2 * q + 1] = v[q].z;
                 }
             } else {
-                // The partials of head h were written by blocks b0..b1 of the attention phase, one slot each, in
-                // block order; merged here in that order, so the result does not depend on which SM ran what.
 #pragma unroll
-                for (int hw = 0; hw < 2; ++hw) {
-                    const int eh = e + 128 * hw;
-                    const int h = eh / P.head, d = eh - h * P.head;
-                    const float *hp = P.att_part + (int64_t)h * kAttSlots * ps;
-                    float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
-                    float L = 0.f;
-                    if (merge_fast) {
-                        const int u0 = h * as.nchunk;
-                        const int np = att_block_of(as, u0 + as.nchunk - 1) - att_block_of(as, u0) + 1;
-                        float4 o4[kAttFastSlots];
-                        float2 ml[kAttFastSlots];
-#pragma unroll
-                        for (int s2 = 0; s2 < kAttFastSlots; ++s2) {
-                            o4[s2] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            ml[s2] = make_float2(-INFINITY, 0.f);
-                            if (s2 < np) {
-                                o4[s2] = ld_cg_f4_issue(hp + (int64_t)s2 * ps + d);
-                                ml[s2] = __ldcg(reinterpret_cast<const float2 *>(hp + (int64_t)s2 * ps + P.head));
-                            }
-                        }
-                        float gm = -INFINITY;
-#pragma unroll
-                        for (int s2 = 0; s2 < kAttFastSlots; ++s2)
-                            gm = fmaxf(gm, ml[s2].x);
-#pragma unroll
-                        for (int s2 = 0; s2 < kAttFastSlots; ++s2) {
-                            if (ml[s2].y > 0.f) {
-                                const float w = expf(ml[s2].x - gm);
-                                L = fmaf(ml[s2].y, w, L);
-                                O.x = fmaf(o4[s2].x, w, O.x);
-                                O.y = fmaf(o4[s2].y, w, O.y);
-                                O.z = fmaf(o4[s2].z, w, O.z);
-                                O.w = fmaf(o4[s2].w, w, O.w);
-                            }
-                        }
-                    } else {
-                        const float *tw = reinterpret_cast<const float *>(share);
-#pragma unroll
-                        for (int s2 = 0; s2 < kAttSlots; ++s2) {
-                            const float w = tw[h * kAttSlots + s2];
-                            if (w > 0.f) {
-                                const float4 o = ld_cg_f4_issue(hp + (int64_t)s2 * ps + d);
-                                O.x = fmaf(o.x, w, O.x);
-                                O.y = fmaf(o.y, w, O.y);
-                                O.z = fmaf(o.z, w, O.z);
-                                O.w = fmaf(o.w, w, O.w);
-                            }
-                        }
-                        L = tw[P.n_heads * kAttSlots + h];
-                    }
-                    // ExpSumNormalize.java:33-37 folded into the weighted sum
-                    xg[j][4 * hw + 0] = __fdiv_rn(O.x, L);
-                    xg[j][4 * hw + 1] = __fdiv_rn(O.y, L);
-                    xg[j][4 * hw + 2] = __fdiv_rn(O.z, L);
-                    xg[j][4 * hw + 3] = __fdiv_rn(O.w, L);
+                for (int q = 0; q < 4; ++q) {
+                    const float4 a4 = ld_cg_f4_issue(p.x_in + e + 64 * q);
+                    xg[4 * q] = a4.x; xg[4 * q + 1] = a4.y; xg[4 * q + 2] = a4.z; xg[4 * q + 3] = a4.w;
                 }
             }
-        }
-        if (merge && !merge_fast)
-            named_barrier_sync(2, kFCons);   // the table's place is taken by the limbs below
-        float ssq = 0.f;
+            if (has_rms) {
 #pragma unroll
-        for (int j = 0; j < kFGroupRounds; ++j) {
-            const int gi = warp + j * kFusedConsWarps;
-            if (gi >= ngroups)   // warp-uniform
-                continue;
-            float amax = 0.f;
-            const float wv[8] = {wa[j].x, wa[j].y, wa[j].z, wa[j].w, wb[j].x, wb[j].y, wb[j].z, wb[j].w};
+                for (int q = 0; q < 16; ++q)
+                    ssq = fmaf(xg[q], live ? xg[q] : 0.f, ssq);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                ssq = fmaf(xg[j][q], xg[j][q], ssq);
-                xg[j][q] = __fmul_rn(wv[q], xg[j][q]);       // RMSNorm weight (1 where the phase has none)
-                amax = fmaxf(amax, fabsf(xg[j][q]));
+                for (int q = 0; q < 4; ++q) {
+                    xg[4 * q] = __fmul_rn(w4[q].x, xg[4 * q]);
+                    xg[4 * q + 1] = __fmul_rn(w4[q].y, xg[4 * q + 1]);
+                    xg[4 * q + 2] = __fmul_rn(w4[q].z, xg[4 * q + 2]);
+                    xg[4 * q + 3] = __fmul_rn(w4[q].w, xg[4 * q + 3]);
+                }
             }
-            amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));   // non-negative floats order like their bits
-            // 24-bit fixed point: one power-of-two scale per group, |x * f| <= 2^22
-            int ex = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 126;   // amax < 2^ex for normal numbers
-            if (!(amax > 0.f) || !(amax < 3.0e38f))
-                ex = 0;
-            ex = max(-90, min(126, ex));
-            const float f = __int_as_float((127 + 22 - ex) << 23);
-            if (lane == 0)
+            uint32_t mbits = 0u;
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+                mbits = max(mbits, __float_as_uint(xg[q]) & 0x7fffffffu);   // non-negative floats order like their bits
+            const uint32_t m_lo = __reduce_max_sync(0xffffffffu, lane < 16 ? mbits : 0u);
+            const uint32_t m_hi = __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : mbits);
+            mbits = lane < 16 ? m_lo : m_hi;
+            // 24-bit fixed point: one power-of-two scale per group, |x * f| <= 2^22, so that adding 1.5 * 2^23 leaves the
+            // rounded integer in the low bits of the sum (the conversion instruction runs at a quarter of that rate)
+            uint32_t z[16];
+            int ex = (int)(mbits >> 23) - 126;   // largest < 2^ex for normal numbers
+            if (max(m_lo, m_hi) < 0x7e800000u) {           // below 2^126
+                if (mbits == 0u)
+                    ex = 0;
+                ex = max(-90, ex);
+                const float f = __int_as_float((127 + 22 - ex) << 23);
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    z[q] = ((uint32_t)__float_as_int(fmaf(xg[q], f, 12582912.0f)) + (0x00008080u - 0x4B400000u)) ^ 0x00008080u;
+            } else {                             // infinities, NaN, the very largest: what the conversion instruction makes of them
+                float amax = 0.f;
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    amax = fmaxf(amax, fabsf(xg[q]));
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1)
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                ex = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 126;
+                if (!(amax > 0.f) || !(amax < 3.0e38f))
+                    ex = 0;
+                ex = max(-90, min(126, ex));
+                const float f = __int_as_float((127 + 22 - ex) << 23);
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    z[q] = ((uint32_t)__float2int_rn(xg[q] * f) + 0x00008080u) ^ 0x00008080u;
+            }
+            if ((lane & 15) == 0)
                 inv_tab[gi] = __int_as_float((127 + ex - 22) << 23);
             // three balanced signed byte limbs: after the add-and-flip, bytes 0..2 of z are l0, l1, l2 in
             // [-128, 127] with X = l0 + 256 l1 + 65536 l2
-            uint32_t z[8];
+            uint32_t *dst = reinterpret_cast<uint32_t *>(share) + gi * 64 + (lane & 15);
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                z[q] = ((uint32_t)__float2int_rn(xg[j][q] * f) + 0x00008080u) ^ 0x00008080u;
-            uint32_t *dst = reinterpret_cast<uint32_t *>(share) + gi * 64 + lane;
-#pragma unroll
-            for (int hw = 0; hw < 2; ++hw) {
-                const uint32_t t0 = __byte_perm(z[4 * hw], z[4 * hw + 1], 0x5140);
-                const uint32_t t2 = __byte_perm(z[4 * hw + 2], z[4 * hw + 3], 0x5140);
-                const uint32_t t1 = __byte_perm(z[4 * hw], z[4 * hw + 1], 0x0062);
-                const uint32_t t3 = __byte_perm(z[4 * hw + 2], z[4 * hw + 3], 0x0062);
-                dst[32 * hw] = __byte_perm(t0, t2, 0x5410);
-                dst[(n >> 2) + 32 * hw] = __byte_perm(t0, t2, 0x7632);
-                dst[(n >> 1) + 32 * hw] = __byte_perm(t1, t3, 0x5410);
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t t0 = __byte_perm(z[4 * q], z[4 * q + 1], 0x5140);
+                const uint32_t t2 = __byte_perm(z[4 * q + 2], z[4 * q + 3], 0x5140);
+                const uint32_t t1 = __byte_perm(z[4 * q], z[4 * q + 1], 0x0062);
+                const uint32_t t3 = __byte_perm(z[4 * q + 2], z[4 * q + 3], 0x0062);
+                dst[16 * q] = __byte_perm(t0, t2, 0x5410);
+                dst[(n >> 2) + 16 * q] = __byte_perm(t0, t2, 0x7632);
+                dst[(n >> 1) + 16 * q] = __byte_perm(t1, t3, 0x5410);
             }
         }
         if (has_rms) {
@@ -554,26 +580,19 @@ __device__ __forceinline__ void consume_ring_phase(const FusedParams &P, const M
     }
     named_barrier_sync(1, kFCons);
 
-    // what a unit of this thread's integer sums is worth: its group's fixed-point unit, times the RMSNorm scalar
-    float unit = gvalid ? inv_tab[g] : 0.f;
-    if (rms_w != nullptr) {
-        const float ssq = warp_sum(lane < kFusedConsWarps ? scratch[lane] : 0.f);   // the same order in every warp and block
-        float tot = __fdiv_rn(ssq, (float)n);
-        tot = __fadd_rn(tot, 1e-5f);
-        unit *= __fdiv_rn(1.0f, __fsqrt_rn(tot));   // RootMeanSquare.java:25-35
-    }
-
-    uint32_t xl[4][4][3];
+    // what a unit of this thread's integer sums is worth: its group's fixed-point unit; the row's sum is multiplied by the
+    // RMSNorm scalar when it is complete
+    const float unit = gvalid ? inv_tab[g] : 0.f;
+    uint32_t xl[2][4][3];
     float xs;
+    const uint32_t in_row = (uint32_t)((gvalid ? g * 256 : 0) + (lane & 7) * 16);
     {
         int s0 = 0, s1 = 0, s2 = 0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < 2; ++k) {
 #pragma unroll
             for (int l = 0; l < 3; ++l) {
-                uint4 t = make_uint4(0u, 0u, 0u, 0u);
-                if (gvalid)
-                    t = *reinterpret_cast<const uint4 *>(share + (size_t)l * n + (size_t)chunk[k] * 16);
+                const uint4 t = *reinterpret_cast<const uint4 *>(share + (size_t)l * n + in_row + 128 * k);
                 xl[k][0][l] = t.x; xl[k][1][l] = t.y; xl[k][2][l] = t.z; xl[k][3][l] = t.w;
             }
 #pragma unroll
@@ -585,83 +604,141 @@ __device__ __forceinline__ void consume_ring_phase(const FusedParams &P, const M
         }
         xs = fmaf((float)s2, 65536.0f, fmaf((float)s1, 256.0f, (float)s0));
     }
+    float rms = 1.0f;
+    if (has_rms) {
+        const float ssq = warp_sum(lane < kFusedConsWarps ? scratch[lane] : 0.f);   // the same order in every warp and block
+        float tot = __fdiv_rn(ssq, (float)n);
+        tot = __fadd_rn(tot, 1e-5f);
+        rms = __fdiv_rn(1.0f, __fsqrt_rn(tot));   // RootMeanSquare.java:25-35
+    }
+    // The limbs, the units and the sums of squares of the next phase take the places of these: a warp may be a whole phase
+    // behind another one from here on.
+    named_barrier_sync(2, kFCons);
     if (tid == 0)
         fused_trace(P, pidx, 1);
 
     // Per-thread constants of the stage loop.  The integer pipe runs at half rate and the dot products live on it,
     // so every address computation in the loop costs as much as a dp4a: offsets inside a stage are fixed per
     // thread and phase, shared memory is addressed with 32-bit window addresses, a stage's descriptor is one
-    // 16-byte load.
-    const int half = (p.paired && rsub >= R / 2) ? 1 : 0;      // second half of a paired stage: the partner matrix
-    const int local = rsub - half * (R / 2);                     // row of this thread inside its half
-    const int par = (lane >> 2) & 1;
+    // 16-byte load.  Rows rsub and rsub + sets of a stage (paired: row rsub of either matrix) are this thread's; rows
+    // beyond the stage's last are computed from what lies there and not used.
+    const int paired = p.paired;
     const uint32_t ring32 = sbase + kFHeader + (uint32_t)P.xarea_bytes;
-    const uint32_t row_off = (uint32_t)(rsub * rowbytes + g * 256 + (lane & 3) * 16);
-    const uint32_t off_a = row_off + 64u * (uint32_t)par;       // chunks 0 and 2 of the thread (+0, +128)
-    const uint32_t off_b = row_off + 64u * (uint32_t)(1 - par); // chunks 1 and 3
-    const uint32_t hdr_off = (uint32_t)(p.hdr_off + half * p.half_hdr + 8 * (local * (n >> 8) + g));
+    const uint32_t row_a = (uint32_t)((active ? rsub : 0) * n) + in_row;
+    const uint32_t row_b = row_a + (uint32_t)(sets * n);
+    const uint32_t hdr_a = (uint32_t)(p.hdr_off + 8 * ((active ? rsub : 0) * (n >> 8) + (gvalid ? g : 0)));
+    const uint32_t hdr_b = hdr_a + (uint32_t)(paired ? p.half_hdr : 8 * sets * (n >> 8));
     const uint32_t desc32 = sbase + kFDescOff;
     uint32_t e = (uint32_t)(cs.seq % kFDesc), parity = (uint32_t)(cs.seq / kFDesc) & 1u;
 
-    // The block's stages are taken in groups of kFGroup: a warp works through the rows of a group one stage after
-    // the other, then folds the group's partial sums with one butterfly and hands them to the epilogue warp in one
-    // go.  A warp's chain of waits, loads, dot products, fold and hand-over is serial; per group instead of per
-    // stage it costs a quarter as much per row, while the ring still moves in stages of rpp rows.
+    auto load = [&](uint32_t at, StageRegs &r) {
+        const uint4 d = lds_v4(desc32 + 32u * at);            // off, nrows, e0a, e0b
+        const uint32_t slot = ring32 + d.x;
+        // rows start on group boundaries: the header of the thread's group is (e0 >> 8) + row * groups per row + g
+        r.ms[0] = lds_f2(slot + hdr_a + ((d.z >> 8) << 3));
+        r.ms[1] = lds_f2(slot + hdr_b + (((paired ? d.w : d.z) >> 8) << 3));
+        r.w[0][0] = lds_v4(slot + row_a);
+        r.w[0][1] = lds_v4(slot + row_a + 128u);
+        r.w[1][0] = lds_v4(slot + row_b);
+        r.w[1][1] = lds_v4(slot + row_b + 128u);
+    };
+
+    auto dot = [&](const StageRegs &r, float &va, float &vb) {
+        float out[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            int a0 = 0, a1 = 0, a2 = 0;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const uint4 w = r.w[q][k];
+                a0 = dp4a_us(w.x, xl[k][0][0], a0);
+                a1 = dp4a_us(w.x, xl[k][0][1], a1);
+                a2 = dp4a_us(w.x, xl[k][0][2], a2);
+                a0 = dp4a_us(w.y, xl[k][1][0], a0);
+                a1 = dp4a_us(w.y, xl[k][1][1], a1);
+                a2 = dp4a_us(w.y, xl[k][1][2], a2);
+                a0 = dp4a_us(w.z, xl[k][2][0], a0);
+                a1 = dp4a_us(w.z, xl[k][2][1], a1);
+                a2 = dp4a_us(w.z, xl[k][2][2], a2);
+                a0 = dp4a_us(w.w, xl[k][3][0], a0);
+                a1 = dp4a_us(w.w, xl[k][3][1], a1);
+                a2 = dp4a_us(w.w, xl[k][3][2], a2);
+            }
+            // |a_l| <= 32 * 255 * 128: the two lower limbs together fit 32 bits
+            const float dsum = fmaf((float)a2, 65536.0f, (float)(a1 * 256 + a0));
+            out[q] = fmaf(r.ms[q].y, dsum, r.ms[q].x * xs);
+        }
+        va = out[0];
+        vb = out[1];
+    };
+
+    auto wait = [&](int t) {
+        const uint32_t at = (e + (uint32_t)t) & (kFDesc - 1);
+        if (!mbar_wait_bounded(sbase + kFBarFull + 8 * at, parity ^ (at < e ? 1u : 0u), wait_ns))
+            cs.lost = true;
+        return at;
+    };
+    auto release = [&](int t) {      // this warp is done with the stage's bytes
+        __syncwarp();
+        if (lane == 0)
+            mbar_arrive(sbase + kFBarEmpty + 8 * ((e + (uint32_t)t) & (kFDesc - 1)));
+    };
+
+    // The block's stages are taken in groups of kFGroup: a warp works through a group's rows in one straight line (the
+    // bytes of a stage are fetched from shared memory while the dot products of the stage in front run), then folds the
+    // partial sums with one butterfly and hands them to the epilogue warp in one go.
     for (int g0 = 0; g0 < nmine; g0 += kFGroup) {
         const int cnt = min(kFGroup, nmine - g0);
-        float v[kFGroup];
-#pragma unroll
-        for (int t = 0; t < kFGroup; ++t) {
-            v[t] = 0.f;
-            if (t >= cnt)
-                continue;
-            if (!mbar_wait_bounded(sbase + kFBarFull + 8 * e, parity, wait_ns))
-                cs.lost = true;
-            if (g0 == 0 && t == 0 && tid == 0)
+        float v[2 * kFGroup];
+        if (cnt == kFGroup && active) {
+            StageRegs a, b;
+            load(wait(0), a);
+            if (g0 == 0 && tid == 0)
                 fused_trace(P, pidx, 4);
-            const uint4 d = lds_v4(desc32 + 32u * e);            // off, nrows, e0a, e0b
-            const uint32_t slot32 = ring32 + d.x;
-            if (gvalid && local < (int)d.y) {
-                // rows start on group boundaries: the header of the thread's group is (e0 >> 8) + local * groups per row + g
-                const float2 ms = lds_f2(slot32 + hdr_off + (((half ? d.w : d.z) >> 8) << 3));
-                const uint32_t sa = slot32 + off_a, sb = slot32 + off_b;
-                int a0 = 0, a1 = 0, a2 = 0;
+            load(wait(1), b);
+            dot(a, v[0], v[1]);
+            release(0);
+            load(wait(2), a);
+            dot(b, v[2], v[3]);
+            release(1);
+            load(wait(3), b);
+            dot(a, v[4], v[5]);
+            release(2);
+            dot(b, v[6], v[7]);
+            release(3);
+        } else {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint4 w = lds_v4(((k & 1) ? sb : sa) + ((k & 2) ? 128u : 0u));
-                    a0 = dp4a_us(w.x, xl[k][0][0], a0);
-                    a1 = dp4a_us(w.x, xl[k][0][1], a1);
-                    a2 = dp4a_us(w.x, xl[k][0][2], a2);
-                    a0 = dp4a_us(w.y, xl[k][1][0], a0);
-                    a1 = dp4a_us(w.y, xl[k][1][1], a1);
-                    a2 = dp4a_us(w.y, xl[k][1][2], a2);
-                    a0 = dp4a_us(w.z, xl[k][2][0], a0);
-                    a1 = dp4a_us(w.z, xl[k][2][1], a1);
-                    a2 = dp4a_us(w.z, xl[k][2][2], a2);
-                    a0 = dp4a_us(w.w, xl[k][3][0], a0);
-                    a1 = dp4a_us(w.w, xl[k][3][1], a1);
-                    a2 = dp4a_us(w.w, xl[k][3][2], a2);
+            for (int t = 0; t < kFGroup; ++t) {
+                v[2 * t] = v[2 * t + 1] = 0.f;
+                if (t < cnt) {
+                    const uint32_t at = wait(t);
+                    if (g0 == 0 && t == 0 && tid == 0)
+                        fused_trace(P, pidx, 4);
+                    if (active) {
+                        StageRegs a;
+                        load(at, a);
+                        dot(a, v[2 * t], v[2 * t + 1]);
+                    }
+                    release(t);
                 }
-                // |a_l| <= 64 * 255 * 128 < 2^24: the conversions are exact
-                const float dsum = fmaf((float)a2, 65536.0f, fmaf((float)a1, 256.0f, (float)a0));
-                v[t] = fmaf(ms.y, dsum, ms.x * xs) * unit;
             }
-            __syncwarp();
-            if (lane == 0)
-                mbar_arrive(sbase + kFBarEmpty + 8 * e);   // this warp is done with the stage's bytes
-            e = (e + 1) & (kFDesc - 1);
-            parity ^= (e == 0);
-            ++cs.seq;
         }
-        const float tot = Fold<kFGroup, 16>::run(v, lane);   // lane t * (32 / kFGroup) holds the sum of stage t
+        const uint32_t en = (e + (uint32_t)cnt) & (kFDesc - 1);
+        parity ^= en < e ? 1u : 0u;
+        e = en;
+        cs.seq += cnt;
+#pragma unroll
+        for (int t = 0; t < 2 * kFGroup; ++t)
+            v[t] = gvalid ? v[t] * unit : 0.f;
+        const float tot = Fold<2 * kFGroup, 16>::run(v, lane) * rms;   // lanes 4 i.. hold the sum of v[i]
         if (cs.rround > 0) {
             if (!mbar_wait_bounded(sbase + kFBarRedEmpty + 8 * cs.rb, (uint32_t)(cs.rround - 1) & 1u, wait_ns))
                 cs.lost = true;
         }
         float *red = reinterpret_cast<float *>(smem + kFRedOff + cs.rb * kFRedStride);
-        if (active && (lane & (32 / kFGroup - 1)) == 0) {
-            const int t = lane / (32 / kFGroup);
-            red[(t * p.rpp + rsub) * p.wpr + wi] = tot;
+        if (active && (lane & 3) == 0) {
+            const int t = lane >> 3, r = (lane >> 2) & 1;
+            red[(t * p.rpp + r * sets + rsub) * p.wpr + wi] = tot;
         }
         __syncwarp();
         if (lane == 0)
@@ -678,7 +755,7 @@ __device__ __forceinline__ void consume_ring_phase(const FusedParams &P, const M
 // The attention step of the block: its run of units, each a stage of cached K and V rows in the ring (the
 // token's own row comes straight from the cache in global memory).  One pass with an online softmax per
 // lane group; the lane groups of the block are merged through shared memory whenever the head changes.
-__device__ __forceinline__ void consume_attention(const FusedParams &P, int layer, const AttSplit &as, int pos, uint8_t *smem,
+__device__ __forceinline__ void consume_attention(const FusedParams &P, int tag, const AttSplit &as, uint8_t *smem,
                                                   uint32_t sbase, Consumer &cs, uint64_t wait_ns)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -697,101 +774,179 @@ __device__ __forceinline__ void consume_attention(const FusedParams &P, int laye
     const int sstride = head + 4;
     float *marea = reinterpret_cast<float *>(smem + kFHeader);
     const float sq = sqrtf((float)head);
-    const float *kc = P.mv[0].k_cache + (int64_t)layer * P.kv_step;
-    const float *vc = P.mv[0].v_cache + (int64_t)layer * P.kv_step;
+    const float2 *kvp = P.kv_pairs;            // the row of this token: keys, then values of all kv heads
+    const int kv_dim = P.mv[0].kv_dim;
 
-    int cur_h = -1;
+    // The lane's four elements of up to three vectors of pairs, waited for together; every lane of the warp takes part.
+    auto get = [&](const float2 *s0, bool want0, float4 &out0, const float2 *s1, const float2 *s2, bool want12, float4 &out1, float4 &out2) {
+        float4 a[6];
+#pragma unroll
+        for (int z = 0; z < 6; ++z)
+            a[z] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const long long c0 = sm_clock();
+        const long long limit = (long long)(2 * (cs.lost ? kFShortWaitNs : wait_ns));
+        for (;;) {
+            if (want0) {
+                a[0] = ld_pairs2_gpu(s0);
+                a[1] = ld_pairs2_gpu(s0 + 2);
+            }
+            if (want12) {
+                a[2] = ld_pairs2_gpu(s1);
+                a[3] = ld_pairs2_gpu(s1 + 2);
+                a[4] = ld_pairs2_gpu(s2);
+                a[5] = ld_pairs2_gpu(s2 + 2);
+            }
+            const bool ok = (!want0 || (tagged(a[0], tag) && tagged(a[1], tag))) &&
+                            (!want12 || (tagged(a[2], tag) && tagged(a[3], tag) && tagged(a[4], tag) && tagged(a[5], tag)));
+            if (__all_sync(0xffffffffu, ok))
+                break;
+            if (__any_sync(0xffffffffu, sm_clock() - c0 > limit)) {
+                cs.lost = true;
+                break;
+            }
+        }
+        if (want0)
+            out0 = make_float4(a[0].x, a[0].z, a[1].x, a[1].z);
+        if (want12) {
+            out1 = make_float4(a[2].x, a[2].z, a[3].x, a[3].z);
+            out2 = make_float4(a[4].x, a[4].z, a[5].x, a[5].z);
+        }
+    };
+    const int batch_log = __ffs(kAttBatch * ppw) - 1;      // positions per warp and batch: a power of two
+
+    int cur_h = -1, kvh = 0, turn = 0;
+    float4 k_own = make_float4(0.f, 0.f, 0.f, 0.f), v_own = k_own;
+    static_assert(kAttChunk / kAttBatch <= kFusedConsWarps, "a warp has one batch of a unit at most");
     float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float m = -INFINITY, l = 0.f;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 
-    auto flush = [&](int h) {
-        // merge the lane groups in slot order and write the block's partial of head h
-        float *mine = marea + slot * sstride;
-        if (act)
-            *reinterpret_cast<float4 *>(mine + 4 * li) = acc;
-        if (li == 0) {
-            mine[head] = m;
-            mine[head + 1] = l;
-        }
-        named_barrier_sync(2, kFCons);
-        if (tid < head) {
-            float M = -INFINITY;
-            for (int s = 0; s < nslots; ++s)
-                M = fmaxf(M, marea[s * sstride + head]);
-            float L = 0.f, O = 0.f;
-            for (int s = 0; s < nslots; ++s) {
-                const float ms = marea[s * sstride + head];
-                const float ls = marea[s * sstride + head + 1];
-                if (ls > 0.f) {
-                    const float w = expf(ms - M);
-                    L = fmaf(ls, w, L);
-                    O = fmaf(marea[s * sstride + tid], w, O);
-                }
-            }
-            const int pslot = b - att_block_of(as, h * as.nchunk);
-            float *part = P.att_part + ((int64_t)h * kAttSlots + pslot) * sstride;
-            __stcg(part + tid, O);
-            if (tid == 0) {
-                __stcg(part + head, M);
-                __stcg(part + head + 1, L);
-            }
-        }
-        named_barrier_sync(2, kFCons);   // the merge area is free again
-    };
-
-    for (int u = u0; u < u1; ++u) {
+    float M = -INFINITY, L = 0.f, O = 0.f;   // the block's result for a head: this thread's element of the output
+    int others = -1;                         // blocks whose results for the head are merged with this block's
+    for (int u = u0;; ++u) {
         const int e = cs.seq % kFDesc;
-        if (!mbar_wait_bounded(sbase + kFBarFull + 8 * e, (uint32_t)(cs.seq / kFDesc) & 1u, wait_ns))
-            cs.lost = true;
-        cs.lost = __any_sync(0xffffffffu, cs.lost) != 0;   // the shuffles below need a warp-uniform decision
-        const FStage d = *(reinterpret_cast<const FStage *>(smem + kFDescOff) + e);
-        const int h = d.seg;
-        if (h != cur_h) {
-            if (cur_h >= 0)
-                flush(cur_h);
+        FStage d{};
+        if (u < u1) {
+            if (!mbar_wait_bounded(sbase + kFBarFull + 8 * e, (uint32_t)(cs.seq / kFDesc) & 1u, wait_ns))
+                cs.lost = true;
+            cs.lost = __any_sync(0xffffffffu, cs.lost) != 0;   // the shuffles below need a warp-uniform decision
+            d = *(reinterpret_cast<const FStage *>(smem + kFDescOff) + e);
+        }
+        const int h = u < u1 ? d.seg : -1;
+        const bool fresh = h != cur_h;
+        if (fresh) {
+            if (cur_h >= 0) {
+                // merge the lane groups in slot order and write the block's partial of head h
+                float *mine = marea + slot * sstride;
+                if (act)
+                    *reinterpret_cast<float4 *>(mine + 4 * li) = acc;
+                if (li == 0) {
+                    mine[head] = m;
+                    mine[head + 1] = l;
+                }
+                named_barrier_sync(2, kFCons);
+                if (tid < ((head + 31) & ~31)) {
+                    // the weights of 32 slots at a time, one per lane and once per warp; then every thread its element
+                    float O2 = 0.f;
+                    M = -INFINITY;
+                    L = O = 0.f;
+                    for (int s = lane; s < nslots; s += 32)
+                        M = fmaxf(M, marea[s * sstride + head]);
+                    M = warp_max(M);
+                    const float *col = marea + (tid < head ? tid : 0);
+                    for (int s0 = 0; s0 < nslots; s0 += 32) {
+                        const int s1 = min(32, nslots - s0);
+                        float w = 0.f;
+                        if (lane < s1) {
+                            const float2 ml = *reinterpret_cast<const float2 *>(marea + (s0 + lane) * sstride + head);
+                            if (ml.y > 0.f)
+                                w = expf(ml.x - M);
+                            L = fmaf(ml.y, w, L);
+                        }
+                        for (int s = 0; s < s1; s += 2) {
+                            O = fmaf(col[(s0 + s) * sstride], __shfl_sync(0xffffffffu, w, s), O);
+                            if (s + 1 < s1)
+                                O2 = fmaf(col[(s0 + s + 1) * sstride], __shfl_sync(0xffffffffu, w, s + 1), O2);
+                        }
+                    }
+                    L = warp_sum(L);
+                    O += O2;
+                    const int pslot = b - att_block_of(as, cur_h * as.nchunk);
+                    others = pslot == 0 ? att_partials(as, cur_h) - 1 : -1;
+                    if (pslot > 0) {
+                        float2 *out = P.att_pairs + ((int64_t)cur_h * (kAttSlots - 1) + pslot - 1) * (head + 2);
+                        if (tid < head)
+                            st_pair_gpu(out + tid, O, tag);
+                        if (tid == 0) {
+                            st_pair_gpu(out + head, M, tag);
+                            st_pair_gpu(out + head + 1, L, tag);
+                        }
+                    } else if (others == 0 && tid < head) {
+                        // ExpSumNormalize.java:33-37 folded into the weighted sum
+                        st_pair_gpu(P.o_pairs + (int64_t)cur_h * head + tid, __fdiv_rn(O, L), tag);
+                    }
+                }
+                named_barrier_sync(2, kFCons);   // the merge area is free again
+            }
+            if (u == u1)
+                break;
             cur_h = h;
             m = -INFINITY;
             l = 0.f;
             acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (act)
-                q4 = __ldcg(reinterpret_cast<const float4 *>(P.q + (int64_t)h * head + 4 * li));
+            kvh = h / P.kv_mul;
         }
-        const bool skip = false;   // a block whose hand-over ran out still works through its stages
+        // the row that this token's QKV phase has just written is the unit's last one, if it is in it at all
+        const bool has_own = d.nrows > d.e0a;
+        if (fresh || has_own)
+            get(P.q_pairs + (int64_t)h * head + 4 * li, fresh && act, q4, kvp + (int64_t)kvh * head + 4 * li,
+                kvp + kv_dim + (int64_t)kvh * head + 4 * li, has_own && act, k_own, v_own);
         const float *ks = reinterpret_cast<const float *>(smem + kFHeader + P.xarea_bytes + (size_t)d.off);
         const float *vs = reinterpret_cast<const float *>(smem + kFHeader + P.xarea_bytes + (size_t)d.off + (size_t)d.aux);
-        const int kvh = h / P.kv_mul;
-        for (int i0 = 0; i0 < d.nrows && !skip; i0 += 2 * nslots) {
-            float4 kk[2], vv[2];
-            float s[2];
+        // A lane group takes kAttBatch positions at a time (independent chains of dot products and shuffles).  A unit is too
+        // small for all warps: the next one starts with the warp behind the last one that had work.
+        const int batches = (d.nrows + (1 << batch_log) - 1) >> batch_log;      // at most kAttChunk / kAttBatch = 8
+        int mine = warp - turn;
+        mine += mine < 0 ? kFusedConsWarps : 0;
+        turn += batches;
+        turn -= turn >= kFusedConsWarps ? kFusedConsWarps : 0;
+        if (mine < batches) {
+            const int first = (mine * ppw + g) * kAttBatch;
+            float4 kk[kAttBatch], vv[kAttBatch];
 #pragma unroll
-            for (int u2 = 0; u2 < 2; ++u2) {
-                const int i = i0 + u2 * nslots + slot;
-                kk[u2] = make_float4(0.f, 0.f, 0.f, 0.f);
-                vv[u2] = kk[u2];
-                if (act && i < d.nrows) {
-                    if (i < d.e0a) {
-                        kk[u2] = *reinterpret_cast<const float4 *>(ks + (size_t)i * head + 4 * li);
-                        vv[u2] = *reinterpret_cast<const float4 *>(vs + (size_t)i * head + 4 * li);
-                    } else {   // the row this token's QKV phase has just written
-                        const int64_t row = ((int64_t)kvh * P.seq_len + d.row0 + i) * head + 4 * li;
-                        kk[u2] = __ldcg(reinterpret_cast<const float4 *>(kc + row));
-                        vv[u2] = __ldcg(reinterpret_cast<const float4 *>(vc + row));
-                    }
+            for (int t = 0; t < kAttBatch; ++t) {
+                kk[t] = vv[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (act && first + t < d.e0a) {
+                    kk[t] = *reinterpret_cast<const float4 *>(ks + (size_t)(first + t) * head + 4 * li);
+                    vv[t] = *reinterpret_cast<const float4 *>(vs + (size_t)(first + t) * head + 4 * li);
                 }
+            }
+            if (has_own) {
+#pragma unroll
+                for (int t = 0; t < kAttBatch; ++t)
+                    if (first + t == d.e0a) {
+                        kk[t] = k_own;
+                        vv[t] = v_own;
+                    }
+            }
+            float s[kAttBatch];
+#pragma unroll
+            for (int t = 0; t < kAttBatch; ++t) {
+                float dd = kk[t].x * q4.x;
+                dd = fmaf(kk[t].y, q4.y, dd);
+                dd = fmaf(kk[t].z, q4.z, dd);
+                s[t] = fmaf(kk[t].w, q4.w, dd);
+            }
+            for (int o = gw >> 1; o > 0; o >>= 1) {
+#pragma unroll
+                for (int t = 0; t < kAttBatch; ++t)
+                    s[t] += __shfl_xor_sync(0xffffffffu, s[t], o);
             }
             float mloc = -INFINITY;
 #pragma unroll
-            for (int u2 = 0; u2 < 2; ++u2) {
-                const int i = i0 + u2 * nslots + slot;
-                float dd = kk[u2].x * q4.x;
-                dd = fmaf(kk[u2].y, q4.y, dd);
-                dd = fmaf(kk[u2].z, q4.z, dd);
-                dd = fmaf(kk[u2].w, q4.w, dd);
-                for (int o = gw >> 1; o > 0; o >>= 1)
-                    dd += __shfl_xor_sync(0xffffffffu, dd, o);
-                s[u2] = i < d.nrows ? __fdiv_rn(dd, sq) : -INFINITY;   // AttentionLoop.java:48
-                mloc = fmaxf(mloc, s[u2]);
+            for (int t = 0; t < kAttBatch; ++t) {
+                s[t] = first + t < d.nrows ? __fdiv_rn(s[t], sq) : -INFINITY;   // AttentionLoop.java:48
+                mloc = fmaxf(mloc, s[t]);
             }
             if (mloc > -INFINITY) {
                 const float mn = fmaxf(m, mloc);
@@ -799,13 +954,13 @@ __device__ __forceinline__ void consume_attention(const FusedParams &P, int laye
                 l *= sc;
                 acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
 #pragma unroll
-                for (int u2 = 0; u2 < 2; ++u2) {
-                    const float pw = expf(s[u2] - mn);
+                for (int t = 0; t < kAttBatch; ++t) {
+                    const float pw = expf(s[t] - mn);
                     l += pw;
-                    acc.x = fmaf(pw, vv[u2].x, acc.x);
-                    acc.y = fmaf(pw, vv[u2].y, acc.y);
-                    acc.z = fmaf(pw, vv[u2].z, acc.z);
-                    acc.w = fmaf(pw, vv[u2].w, acc.w);
+                    acc.x = fmaf(pw, vv[t].x, acc.x);
+                    acc.y = fmaf(pw, vv[t].y, acc.y);
+                    acc.z = fmaf(pw, vv[t].z, acc.z);
+                    acc.w = fmaf(pw, vv[t].w, acc.w);
                 }
                 m = mn;
             }
@@ -815,8 +970,54 @@ __device__ __forceinline__ void consume_attention(const FusedParams &P, int laye
             mbar_arrive(sbase + kFBarEmpty + 8 * e);
         ++cs.seq;
     }
-    if (cur_h >= 0)
-        flush(cur_h);
+    // The block with a head's first positions merges the partial results of the others (the blocks behind it, in block
+    // order) and hands the finished output on.  A head that others work on too is the block's last one, so nobody waits for a
+    // block that waits.
+    if (others > 0 && tid < ((head + 31) & ~31)) {
+        const float2 *parts = P.att_pairs + (int64_t)cur_h * (kAttSlots - 1) * (head + 2);
+        const float2 *src = parts + (tid < head ? tid : 0);
+        const float2 *src_ml = parts + (int64_t)min(lane, others - 1) * (head + 2) + head;   // lane z: maximum and sum of partial z
+        float2 o[kAttSlots - 1];
+        float4 ml = ld_pairs2_gpu(src_ml);
+#pragma unroll
+        for (int z = 0; z < kAttSlots - 1; ++z)
+            if (z < others)
+                o[z] = ld_pair_gpu(src + (int64_t)z * (head + 2));
+        const long long c0 = sm_clock();
+        const long long limit = (long long)(2 * (cs.lost ? kFShortWaitNs : wait_ns));
+        for (;;) {
+            bool ok = tagged(ml, tag);
+#pragma unroll
+            for (int z = 0; z < kAttSlots - 1; ++z)
+                if (z < others)
+                    ok = ok && __float_as_int(o[z].y) == tag;
+            if (__all_sync(0xffffffffu, ok))
+                break;
+            if (__any_sync(0xffffffffu, sm_clock() - c0 > limit)) {
+                cs.lost = true;
+                break;
+            }
+            if (!tagged(ml, tag))
+                ml = ld_pairs2_gpu(src_ml);
+#pragma unroll
+            for (int z = 0; z < kAttSlots - 1; ++z)
+                if (z < others && __float_as_int(o[z].y) != tag)
+                    o[z] = ld_pair_gpu(src + (int64_t)z * (head + 2));
+        }
+        const float gm = fmaxf(M, warp_max(ml.x));
+        const float w0 = L > 0.f ? expf(M - gm) : 0.f;
+        const float w = lane < others && ml.z > 0.f ? expf(ml.x - gm) : 0.f;
+        L = fmaf(L, w0, warp_sum(ml.z * w));
+        O *= w0;
+#pragma unroll
+        for (int z = 0; z < kAttSlots - 1; ++z) {
+            const float wz = __shfl_sync(0xffffffffu, w, z);
+            if (z < others)
+                O = fmaf(o[z].x, wz, O);
+        }
+        if (tid < head)
+            st_pair_gpu(P.o_pairs + (int64_t)cur_h * head + tid, __fdiv_rn(O, L), tag);
+    }
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -828,79 +1029,107 @@ struct Epilogue {
     bool lost, lost_before;
 };
 
+// Results leave as (value, tag) pairs, one store each, which the readers poll: no fence, no counter and no second trip to the
+// L2.  resid: where the old value of a residual element comes from (pairs of `resid_tag`, or the plain vector p.y before the
+// first one).  plain: the last layer, whose query, hidden vector and residual stream stay readable behind the launch.
 __device__ __forceinline__ void epilogue_phase(const FusedParams &P, const MvParams &p, int layer, int first, int nmine, int pos,
-                                               uint8_t *smem, uint32_t sbase, Epilogue &es, uint64_t wait_ns)
+                                               uint8_t *smem, uint32_t sbase, Epilogue &es, uint64_t wait_ns, float2 *out, int tag,
+                                               const float2 *resid, int resid_tag, bool plain)
 {
     const int lane = threadIdx.x & 31;
     const int G = gridDim.x;
-    const int R = p.rt * p.rpp;
-    const int rs = p.rs;                 // output rows (row pairs) per stage: at most 8, so a group fits the 32 lanes
+    const int sets = p.rpp >> 1;
+    const int wpr = p.wpr;
+    const int rs = p.rs;                 // output rows (row pairs) per stage
     const float *rope_c = reinterpret_cast<const float *>(smem + kFRopeOff);
     const float *rope_s = rope_c + 64;
+    const int per = p.epilogue == EPI_QKV_ROPE ? rs >> 1 : rs;   // results (rotated pairs of rows) of a stage
     for (int g0 = 0; g0 < nmine; g0 += kFGroup) {
         const int cnt = min(kFGroup, nmine - g0);
-        if (!mbar_wait_bounded(sbase + kFBarRedFull + 8 * es.rb, (uint32_t)es.rround & 1u, wait_ns))
-            es.lost = true;
         const float *red = reinterpret_cast<const float *>(smem + kFRedOff + es.rb * kFRedStride);
-        const bool skip = false;   // a block whose hand-over ran out still runs its own pipeline to the end
-        if (p.epilogue == EPI_QKV_ROPE) {
-            // a lane owns a pair of rows: (v0, v1) are rotated together (ApplyRope.java:61-92)
-            const int pairs = rs >> 1;
-            const int t = lane / pairs, i = lane - t * pairs;
-            if (t < cnt && !skip) {
-                int seg, row0, nrows;
+        for (int i0 = 0; i0 < cnt * per; i0 += 32) {
+            const int idx = i0 + lane;
+            const int t = idx / per, i = idx - t * per;
+            int seg = 0, row0 = 0, nrows = 0;
+            if (t < cnt)
                 stage_rows(p, first + (g0 + t) * G, seg, row0, nrows);
-                if (2 * i < nrows) {
-                    const float *rt = red + (t * p.rpp) * p.wpr;
-                    float v0 = 0.f, v1 = 0.f;
-                    for (int w = 0; w < p.wpr; ++w) {
-                        v0 += rt[(2 * i) * p.wpr + w];
-                        v1 += rt[(2 * i + 1) * p.wpr + w];
-                    }
-                    const int row = row0 + 2 * i;
-                    if (seg == 2) {
-                        const int kvh = row / p.head, d = row - kvh * p.head;
-                        float *dst = p.v_cache + (int64_t)layer * P.kv_step + ((int64_t)kvh * p.seq_len + pos) * p.head + d;
-                        dst[0] = v0;
-                        dst[1] = v1;
-                    } else {
-                        const int d = row % p.head;
-                        const float c = rope_c[d >> 1], sn = rope_s[d >> 1];
-                        const float r0 = __fsub_rn(__fmul_rn(v0, c), __fmul_rn(v1, sn));
-                        const float r1 = __fadd_rn(__fmul_rn(v0, sn), __fmul_rn(v1, c));
-                        if (seg == 0) {
-                            p.q_out[row] = r0;
-                            p.q_out[row + 1] = r1;
-                        } else {
-                            const int kvh = row / p.head;
-                            float *dst = p.k_cache + (int64_t)layer * P.kv_step + ((int64_t)kvh * p.seq_len + pos) * p.head + d;
-                            dst[0] = r0;
-                            dst[1] = r1;
-                        }
-                    }
+            const int ri = p.epilogue == EPI_QKV_ROPE ? 2 * i : i;
+            const bool mine = t < cnt && ri < nrows;
+            const int row = row0 + ri;
+            float2 old = make_float2(0.f, 0.f);
+            if (p.epilogue == EPI_RESIDUAL && mine) {   // ahead of the sums
+                if (resid)
+                    old = ld_pair_gpu(resid + row);
+                else
+                    old.x = __ldcg(p.y + row);
+            }
+            // everything that does not need the sums is done ahead of them too
+            int kvh = 0, d = 0;
+            float c = 1.f, sn = 0.f;
+            if (p.epilogue == EPI_QKV_ROPE && mine) {
+                kvh = row / p.head;
+                d = row - kvh * p.head;
+                if (seg != 2) {
+                    c = rope_c[d >> 1];
+                    sn = rope_s[d >> 1];
                 }
             }
-        } else {
-            const int t = lane / rs, i = lane - t * rs;
-            if (t < cnt && !skip) {
-                int seg, row0, nrows;
-                stage_rows(p, first + (g0 + t) * G, seg, row0, nrows);
-                if (i < nrows) {
-                    const float *rt = red + (t * p.rpp) * p.wpr;
-                    if (p.epilogue == EPI_SWIGLU) {
-                        float v1 = 0.f, v3 = 0.f;
-                        for (int w = 0; w < p.wpr; ++w) {
-                            v1 += rt[i * p.wpr + w];
-                            v3 += rt[(R / 2 + i) * p.wpr + w];
-                        }
-                        p.y[row0 + i] = __fmul_rn(__fmul_rn(v1, sigmoid_accurate(v1)), v3);   // Silu.java:122-132 order
-                    } else {   // EPI_RESIDUAL
-                        float a = 0.f;
-                        for (int w = 0; w < p.wpr; ++w)
-                            a += rt[i * p.wpr + w];
-                        atomicAdd(p.y + row0 + i, a);   // one add per element and phase: deterministic
-                    }
+            if (i0 == 0) {
+                if (!mbar_wait_bounded(sbase + kFBarRedFull + 8 * es.rb, (uint32_t)es.rround & 1u, wait_ns))
+                    es.lost = true;
+            }
+            if (!mine)
+                continue;
+            const float *ra = red + (t * p.rpp + ri) * wpr;
+            const float *rb = p.epilogue == EPI_SWIGLU ? ra + sets * wpr : ra + wpr;    // partner row: of W3, or the next one
+            const bool two = p.epilogue != EPI_RESIDUAL;
+            float v0 = 0.f, v1 = 0.f;
+#pragma unroll 4
+            for (int w = 0; w < wpr; ++w) {
+                v0 += ra[w];
+                if (two)
+                    v1 += rb[w];
+            }
+            if (p.epilogue == EPI_QKV_ROPE) {
+                // a lane owns a pair of rows: (v0, v1) are rotated together (ApplyRope.java:61-92)
+                float r0 = v0, r1 = v1;
+                if (seg != 2) {
+                    r0 = __fsub_rn(__fmul_rn(v0, c), __fmul_rn(v1, sn));
+                    r1 = __fadd_rn(__fmul_rn(v0, sn), __fmul_rn(v1, c));
                 }
+                float2 *dst = seg == 0 ? out + row : P.kv_pairs + (seg == 2 ? p.kv_dim : 0) + row;
+                st_pair_gpu(dst, r0, tag);
+                st_pair_gpu(dst + 1, r1, tag);
+                if (seg == 0 && plain) {
+                    p.q_out[row] = r0;
+                    p.q_out[row + 1] = r1;
+                }
+                if (seg != 0) {      // the cache is for the tokens behind this one
+                    float *cache = (seg == 2 ? p.v_cache : p.k_cache) + (int64_t)layer * P.kv_step + ((int64_t)kvh * p.seq_len + pos) * p.head + d;
+                    cache[0] = r0;
+                    cache[1] = r1;
+                }
+            } else if (p.epilogue == EPI_SWIGLU) {
+                const float r = __fmul_rn(__fmul_rn(v0, sigmoid_accurate(v0)), v1);   // Silu.java:122-132 order
+                st_pair_gpu(out + row, r, tag);
+                if (plain)
+                    p.y[row] = r;
+            } else {   // EPI_RESIDUAL
+                if (resid && __float_as_int(old.y) != resid_tag) {
+                    const long long c0 = sm_clock();
+                    const long long limit = (long long)(2 * (es.lost ? kFShortWaitNs : wait_ns));
+                    do {
+                        old = ld_pair_gpu(resid + row);
+                        if (sm_clock() - c0 > limit) {
+                            es.lost = true;
+                            break;
+                        }
+                    } while (__float_as_int(old.y) != resid_tag);
+                }
+                const float r = __fadd_rn(old.x, v0);
+                st_pair_gpu(out + row, r, tag);
+                if (plain && resid == P.xa_pairs)
+                    p.y[row] = r;
             }
         }
         __syncwarp();
@@ -951,7 +1180,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
         pr.ring_base = sbase + kFHeader + (uint32_t)P.xarea_bytes;
         pr.vhead = 0;
         pr.ring_bytes = P.ring_bytes;
-        pr.seq = pr.tail = 0;
+        pr.seq = pr.tail = pr.vtail = 0;
         pr.lost = false;
         pr.wait_ns = wait_ns;
         const uint64_t pol = policy_evict_first();
@@ -965,9 +1194,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
                 const MvParams &p = P.mv[k];
                 const int S = p.total_stages;
                 if (!(P.debug_no_copy & 8) && lane == 0) fused_trace(P, layer * 5 + (k == 0 ? 0 : k + 1), 5);
-                for (int s = first_stage_of(b, rot, G); s < S; s += G) {
-                    produce_ring_stage(pr, P, p, k, layer, s, pol, lane);
-                }
+                produce_phase(pr, P, p, k, layer, first_stage_of(b, rot, G), G, pol, lane);
                 if (!(P.debug_no_copy & 8) && lane == 0) fused_trace(P, layer * 5 + (k == 0 ? 0 : k + 1), 6);
                 rot = (rot + S) % G;
                 if (k == 0) {
@@ -996,7 +1223,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
     pdl_wait();
     const int pos = __ldcg(&P.state->cur_pos);
     const AttSplit as = att_split(P, pos, G);
-    const unsigned int target = __ldcg(P.epoch) * (unsigned int)G;
+    const unsigned int epoch = __ldcg(P.epoch);
+    const int tag0 = (int)(epoch * (unsigned int)P.n_layers) + 1;    // tag of layer l: tag0 + l
     const bool lost_at_entry = (__ldcg(&P.state->status) & L2J_DS_WAIT_TIMEOUT) != 0;
 
     // ------------------------------------------------------------------------------ epilogue warp
@@ -1022,14 +1250,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
                 const int first = first_stage_of(b, rot, G);
                 const int nmine = first < S ? (S - first + G - 1) / G : 0;
                 rot = (rot + S) % G;
-                epilogue_phase(P, p, layer, first, nmine, pos, smem, sbase, es, wait_ns);
-                // every result of the block in this phase was written by this warp; the release is cumulative
-                __syncwarp();
-                const int pidx = layer * 5 + (k == 0 ? 0 : k + 1);
-                if (lane == 0) {
-                    red_release_add_u32(P.sync + (int64_t)kSyncStride * pidx, 1u);
-                    fused_trace(P, pidx, 3);
+                const int tag = tag0 + layer;
+                float2 *out = k == 0 ? P.q_pairs : (k == 1 ? P.xa_pairs : (k == 2 ? P.h_pairs : P.xb_pairs));
+                const float2 *resid = k == 1 ? (layer > 0 ? P.xb_pairs : nullptr) : P.xa_pairs;
+                epilogue_phase(P, p, layer, first, nmine, pos, smem, sbase, es, wait_ns, out, tag, resid, k == 1 ? tag - 1 : tag,
+                               layer + 1 == P.n_layers);
+                if (k == 3 && layer + 1 == P.n_layers) {
+                    // the classifier kernel behind polls this counter: every result of the block in this phase was written by
+                    // this warp, the release is cumulative
+                    __syncwarp();
+                    if (lane == 0)
+                        red_release_add_u32(P.sync + (int64_t)kSyncStride * (layer * 5 + 4), 1u);
                 }
+                if (lane == 0)
+                    fused_trace(P, layer * 5 + (k == 0 ? 0 : k + 1), 3);
             }
         }
         if (es.lost && !es.lost_before && lane == 0)
@@ -1055,29 +1289,22 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
             if (nmine > 0) {
                 if (tid == 0)
                     fused_trace(P, pidx, 7);
-                if (pidx > 0)   // the first phase's input came from the kernel in front
-                    consumers_wait(P.sync + (int64_t)kSyncStride * (pidx - 1), target, smem, cs, wait_ns);
-                if (tid == 0)
-                    fused_trace(P, pidx, 0);
                 const float *rms_w = p.rms_w ? p.rms_w + (int64_t)layer * P.rms_step : nullptr;
-                const float wmax = p.rms_w ? __ldg(P.rms_wmax + 2 * layer + (k == 2 ? 1 : 0)) : 1.0f;
-                consume_ring_phase(P, p, layer, nmine, k == 1, rms_w, wmax, as, smem, sbase, cs, wait_ns, pidx);
+                // the first phase's input came from the kernel in front
+                const float2 *in = k == 0 ? (layer > 0 ? P.xb_pairs : nullptr) : (k == 1 ? P.o_pairs : (k == 2 ? P.xa_pairs : P.h_pairs));
+                consume_ring_phase(P, p, nmine, in, k == 0 ? tag0 + layer - 1 : tag0 + layer, rms_w, smem, sbase, cs, wait_ns, pidx);
             }
             if (k == 0) {
                 // attention over positions 0..pos (Run.java:450-478)
                 const int aidx = layer * 5 + 1;
                 if (b < as.ga) {
-                    consumers_wait(P.sync + (int64_t)kSyncStride * (aidx - 1), target, smem, cs, wait_ns);
                     if (tid == 0)
                         fused_trace(P, aidx, 0);
-                    consume_attention(P, layer, as, pos, smem, sbase, cs, wait_ns);
+                    consume_attention(P, tag0 + layer, as, smem, sbase, cs, wait_ns);
                     if (tid == 0)
                         fused_trace(P, aidx, 2);
-                    // flush() ended with a barrier of all consumers: their partials are written
-                }
-                if (tid == 0) {
-                    red_release_add_u32(P.sync + (int64_t)kSyncStride * aidx, 1u);
-                    fused_trace(P, aidx, 3);
+                    if (tid == 0)
+                        fused_trace(P, aidx, 3);
                 }
             }
         }

@@ -200,9 +200,9 @@ struct AttnParams {
 // phases ahead into one shared-memory byte ring while the consumers wait at a phase boundary, and the
 // cached K and V rows of the attention phase travel through the same ring.  The parameters of the
 // first layer are given; those of layer l follow by adding l times a step to the pointers.
-constexpr int kAttSlots = 8;        // partial results per head that the step after the attention phase can merge
+constexpr int kAttSlots = 8;        // partial results per head that can be merged
 constexpr int kAttMaxSplit = 6;     // blocks per head in the attention phase (a head gets at most kAttMaxSplit + 1 partials)
-constexpr int kAttChunk = 64;       // cached positions per ring stage of the attention phase
+constexpr int kAttChunk = 32;       // cached positions per ring stage of the attention phase
 
 struct FusedParams {
     MvParams mv[4];            // QKV, Wo, W1/W3, W2 of the first layer of the context's range
@@ -210,13 +210,19 @@ struct FusedParams {
     long long kv_step;         // floats between the KV caches of consecutive layers
     int rms_step;              // floats between the RMSNorm weight vectors of consecutive layers
     int n_layers;
-    const float *rms_wmax;     // [n_layers][2]: max |w| of the attention and the FFN RMSNorm weights
-    const float *q;            // query vector written by the QKV phase (n_heads * head)
-    float *att_part;           // [n_heads][kAttSlots][head + 4]: o, then m, l
+    // Vectors that the blocks hand to each other, as (value, tag) pairs: a tag is used once per element (forward number times
+    // n_layers, plus the layer, plus one), so whoever finds it knows that the value is the one it waits for.
+    float2 *q_pairs;           // query vector (n_heads * head)
+    float2 *kv_pairs;          // this token's keys, then values (2 * kv_dim)
+    float2 *xa_pairs;          // residual stream behind Wo (dim)
+    float2 *h_pairs;           // hidden vector (hidden)
+    float2 *xb_pairs;          // residual stream behind W2 (dim)
+    float2 *o_pairs;           // attention output (n_heads * head)
+    float2 *att_pairs;         // [n_heads][kAttSlots - 1][head + 2]: partial results on their way to the block that merges a head's: o, m, l
     int n_heads, kv_mul, head, seq_len;
     int xarea_bytes;           // shared memory between the fixed header and the ring: limbs of the input vector / merge area
     int ring_bytes;            // bytes of the ring
-    unsigned int *sync;        // hand-over counters, kSyncStride words apart, five per layer
+    unsigned int *sync;        // hand-over counters, kSyncStride words apart, five per layer, as the per-step kernels have them: the last one is used
     const unsigned int *epoch; // forwards started on this context
     SeqState *state;
     int timeout_us;
@@ -224,8 +230,9 @@ struct FusedParams {
     int debug_no_copy;         // measurement aid: the producer hands out stages without copying (results are garbage)
 };
 constexpr int kSyncStride = 32;     // unsigned ints between two hand-over counters (128 bytes)
-constexpr int kFusedThreads = 640;  // 18 consumer warps, the producer warp, the epilogue warp
-constexpr int kFusedConsWarps = 18;
+constexpr int kFusedThreads = 512;  // 14 consumer warps, the producer warp, the epilogue warp: 128 registers per thread
+constexpr int kFusedConsWarps = 14;
+constexpr int kFusedMaxRow = 4 * kFusedConsWarps * kGroup;   // longest matrix row: a warp spans four groups
 constexpr int kFusedHeaderBytes = 4096;   // barriers, descriptors, reduction buffers in front of the vector area and the ring
 
 cudaError_t prepare_fused(int *max_smem);
