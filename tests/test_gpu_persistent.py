@@ -1,0 +1,75 @@
+"""The persistent kernel at the edges of its mapping, against the per-step kernels.
+
+Both form the same products from the same 24-bit activations and add the FP32 group terms of a row in other orders; a row of g groups
+is then off by at most about g roundings of 2^-24 of its terms, and two layers of them move a logit by a few 1e-6 of the range
+(observed: 1e-6).  The bound is 1e-5."""
+import numpy as np
+import pytest
+
+from llama2j_b200 import lib as L
+from llama2j_b200 import synthetic as syn
+from llama2j_b200.model_files import ModelConfig
+from llama2j_b200.transformer import Transformer
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+def _build(cfg, tensors, flags):
+    m = Transformer(cfg, 0, 0, None, flags)
+    m.upload_all(tensors)
+    m.finalize()
+    assert m.launch_mode()["persistent"] == (flags == L.F_PERSISTENT)
+    return m
+
+
+# dim, hidden, heads, kv heads: one group per row and warps without one; groups that fill a warp and one more; head sizes 8 (more lane
+# groups than lanes in the merge), 32, 64, 128; shared K/V heads; rows of 56 groups (all consumer warps on one set of rows)
+SHAPES = [(256, 512, 32, 32), (512, 1280, 16, 4), (1024, 1280, 8, 8), (1280, 2304, 10, 2), (768, 14336, 12, 12), (4096, 2816, 32, 8)]
+
+
+@pytest.mark.parametrize("dim,hidden,heads,kv", SHAPES)
+def test_against_step_kernels(dim, hidden, heads, kv):
+    cfg = ModelConfig(dim=dim, hidden_dim=hidden, n_layers=2, n_heads=heads, n_kv_heads=kv, vocab_size=500, seq_len=800,
+                      shared_classifier=True)
+    tensors = syn.synthetic_tensors(cfg, 8)
+    rng = np.random.default_rng(9)
+    for t in (L.T_RMS_ATT, L.T_RMS_FFN, L.T_RMS_FINAL):
+        tensors[t] = syn.quant_encode(rng.uniform(0.5, 1.5, cfg.tensor_floats(t)).astype(np.float32))
+    a, b = _build(cfg, tensors, L.F_PERSISTENT), _build(cfg, tensors, L.F_STEP_KERNELS)
+    # ends of attention units (32 positions), of the short regime (512), positions whose partials come from several blocks
+    check = {0, 1, 30, 31, 32, 33, 63, 64, 127, 128, 129, 255, 256, 510, 511, 512, 513, 640, 799}
+    for p in range(800):
+        tok = int(rng.integers(3, cfg.vocab_size))
+        want = p in check
+        x, _ = a.forward(tok, p, want_logits=want)
+        y, _ = b.forward(tok, p, want_logits=want)
+        if want:
+            assert float(np.abs(x - y).max()) <= TOL * float(y.max() - y.min()), p
+    # what the launch leaves behind for readers
+    for which, n in ((0, dim), (2, dim), (3, hidden)):      # x, q, the hidden vector
+        x, y = a.read_buffer(which, n), b.read_buffer(which, n)
+        assert float(np.abs(x - y).max()) <= TOL * float(np.abs(y).max()), which
+    assert a.stats().device_status == 0
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("value", [1e-30, 3e37, np.inf, np.nan])
+def test_embedding_at_the_ends_of_the_range(value):
+    """Tiny and huge activations through the fixed-point conversion: finite where the per-step kernels are, not finite where they are not."""
+    cfg = ModelConfig(dim=512, hidden_dim=1280, n_layers=2, n_heads=4, n_kv_heads=4, vocab_size=300, seq_len=16, shared_classifier=False)
+    tensors = syn.synthetic_tensors(cfg, 10)
+    emb = np.array(tensors[L.T_TOKEN_EMBEDDING], dtype=np.float32).reshape(cfg.vocab_size, cfg.dim)
+    emb[5, 7] = value
+    tensors[L.T_TOKEN_EMBEDDING] = emb.reshape(-1)
+    a, b = _build(cfg, tensors, L.F_PERSISTENT), _build(cfg, tensors, L.F_STEP_KERNELS)
+    x, y = a.forward(5, 0)[0].copy(), b.forward(5, 0)[0].copy()
+    if np.isfinite(y).all():
+        span = max(float(y.max() - y.min()), 1e-30)
+        assert float(np.abs(x - y).max()) <= 1e-4 * span      # one element decides the group's scale
+    else:
+        assert np.array_equal(np.isnan(x), np.isnan(y))
+    a.close()
+    b.close()
