@@ -13,7 +13,7 @@
 //   pf_limbs_kernel     activations -> limbs [3 x 64 rows][K] (the B operand) per block of 64 tokens + per (group,
 //                       token) unit and sum; input is RMSNorm(x) * w, the attention output, or SwiGLU(h1, h3)
 //   pf_gemm_kernel      C[64 tokens][rows] (+)= W[rows][K] x limbs: TMA (cp.async.bulk.tensor) feeds 128-byte-
-//                       swizzled tiles to tcgen05.mma kind::i8 (u8 x s8 -> s32, M 128, N 192, K 32), one
+//                       swizzled tiles to tcgen05.mma kind::i8 (u8 x s8 -> s32, M 128, N 3 x tokens, K 32), one
 //                       accumulator per quantisation group in tensor memory, double-buffered; eight epilogue warps
 //                       read it back (tcgen05.ld), scale in FP32 and keep the row sums in registers
 //   pf_rope_kv_kernel   RoPE on q and k, rows of the K/V cache (ApplyRope.java:61-92, Run.java:443-455)
@@ -49,17 +49,10 @@ constexpr int kN = 3 * kT;                  // columns of the B operand: three l
 constexpr int kTileM = 128;                 // weight rows per tile
 constexpr int kGemmThreads = 384;          // A producer, two issue warps, B producer, eight epilogue warps
 constexpr int kEpiWarps = 8;                // warps 4..11: quarter of tensor memory = warp % 4, half of the tokens = (warp - 4) / 4
-constexpr int kTH = kT / 2;                 // tokens per epilogue thread
-constexpr int kStages = 4;                  // ring depth, a power of two known at compile time: the two single-lane issue
-                                            // loops are on the critical path (a run-time depth, i.e. a division per stage,
-                                            // costs 15 %); one stage = half a quantisation group (K = 128) of A and B
-constexpr int kMaxStages = kStages;
 constexpr int kABytes = kTileM * 128;       // the A part of a stage: 128 rows of 128 bytes
-constexpr int kBBytes = kN * 128;
-constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kMaxParts = 12;               // parts a row sum (or a query's keys) may be dealt into
 constexpr int kWideParts = 3;               // at most this many parts for the wide outputs (W1/W3): their sums are read back
-constexpr int kAccCols = 256;               // column distance of the two accumulators in tensor memory
+constexpr int kAccCols = 256;               // column distance of the two accumulators of the classifier in tensor memory
 constexpr int kTmemCols = 512;
 constexpr int kMaxDim = 16384;              // longest row of a matrix
 
@@ -131,6 +124,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r)
         : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+}
+
 __device__ __forceinline__ void tmem_ld_wait()
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -148,8 +148,30 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr)
     return d;
 }
 
-// c s32, a u8, b s8, both K-major, N 192, M 128
-constexpr uint32_t kIdesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+// The matrix kernel for blocks of TT tokens.  A call of few tokens (a step of a few sequences, a short prompt) takes the
+// smallest that holds them: the tensor cores, the epilogue and the activation tiles cost as much for a token that does not
+// exist, and what they leave free goes into a deeper ring and more accumulators.
+template <int TT>
+struct GemmCfg {
+    static constexpr int kCols = 3 * TT;                       // columns of the B operand
+    static constexpr int kStageBytes = kABytes + kCols * 128;
+    // Ring depth, known at compile time: the two single-lane issue loops are on the critical path (a run-time depth, i.e. a
+    // division per stage, costs 15 %).  One stage = half a quantisation group (K = 128) of A and B.
+    static constexpr int kStages = TT <= 16 ? 8 : 4;
+    static constexpr int kPairs = kStages / 2;                 // groups in the ring
+    static constexpr int kAccs = TT <= 16 ? 8 : (TT <= 32 ? 4 : 2);
+    static constexpr int kAccDist = 512 / kAccs;               // columns between two accumulators in tensor memory
+    static constexpr int kHalf = TT / 2;                       // tokens per epilogue thread
+    static constexpr int kChunk = kHalf % 16 ? 8 : 16;         // of them, taken from tensor memory at a time
+    // c s32, a u8, b s8, both K-major, M 128
+    static constexpr uint32_t kIdesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(kCols >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+    static constexpr size_t smem(int groups) { return (size_t)kStages * kStageBytes + (size_t)groups * TT * sizeof(float2) + 1024; }
+    // The two issue lanes take the groups in turn.  A pair of stages (an accumulator) must always come back to the same lane:
+    // a lane that waits for a phase whose predecessor it has not seen itself may pass on the one before that.
+    static_assert(kPairs % 2 == 0 && kAccs % 2 == 0, "a lane owns its stages and accumulators");
+    static_assert(kCols % 16 == 0 && kCols <= kAccDist && kHalf % kChunk == 0, "shape of the instruction and of its accumulators");
+    static_assert(kStages * kStageBytes + (kMaxDim / 256) * TT * 8 + 1024 <= 227 * 1024, "what a block may have");
+};
 
 // Bounded wait that also ends when another role of the block has given up.
 __device__ __forceinline__ bool pf_wait(uint32_t bar, uint32_t parity, volatile int *give_up, long long limit)
@@ -204,23 +226,26 @@ struct PfGemmParams {
 };
 
 // 512: no more than 128 registers per thread, so that blocks of the kernels in front and behind fit on the SM beside it
+template <int TT>
 __global__ void __launch_bounds__(512, 1)
 pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1,
                const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b, const PfGemmParams p)
 {
     extern __shared__ unsigned char pf_smem_raw[];
-    __shared__ __align__(8) unsigned long long s_bar[2 * kMaxStages + 4 + 2];
+    using C = GemmCfg<TT>;
+    constexpr int kStages = C::kStages, kStageBytes = C::kStageBytes, kAccs = C::kAccs;
+    __shared__ __align__(8) unsigned long long s_bar[2 * kStages + 2 * kAccs + 2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_give_up;
-    __shared__ float s_ss[kT];
+    __shared__ float s_ss[TT];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t base = (smem_u32(pf_smem_raw) + 1023u) & ~1023u;            // swizzled tiles want 1024-byte alignment
     unsigned char *gen = pf_smem_raw + (base - smem_u32(pf_smem_raw));
     float2 *s_ux = reinterpret_cast<float2 *>(gen + (size_t)kStages * kStageBytes);
-    const uint32_t bar_full = smem_u32(&s_bar[0]), bar_empty = smem_u32(&s_bar[kMaxStages]);
-    const uint32_t bar_acc_full = smem_u32(&s_bar[2 * kMaxStages]), bar_acc_empty = smem_u32(&s_bar[2 * kMaxStages + 2]);
-    const uint32_t bar_fin = smem_u32(&s_bar[2 * kMaxStages + 4]);
+    const uint32_t bar_full = smem_u32(&s_bar[0]), bar_empty = smem_u32(&s_bar[kStages]);
+    const uint32_t bar_acc_full = smem_u32(&s_bar[2 * kStages]), bar_acc_empty = smem_u32(&s_bar[2 * kStages + kAccs]);
+    const uint32_t bar_fin = smem_u32(&s_bar[2 * kStages + 2 * kAccs]);
     const long long limit = 2000ll * (long long)p.timeout_us;
 
     int ntiles = 0;
@@ -237,7 +262,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
             mbar_init(bar_full + 8 * s, 2);            // both producers
             mbar_init(bar_empty + 8 * s, 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kAccs; ++b) {
             mbar_init(bar_acc_full + 8 * b, 1);
             mbar_init(bar_acc_empty + 8 * b, kEpiWarps);
         }
@@ -274,7 +299,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         tmem_alloc(smem_u32(&s_tmem), kTmemCols);
         tmem_relinquish();
     }
-    if (tid < kT) {
+    if (tid < TT) {
         // RootMeanSquare.java:25-35: the scalar of the RMSNorm in front multiplies every unit of the token
         float ss = 1.0f;
         if (p.ssq != nullptr) {
@@ -288,9 +313,10 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         s_ss[tid] = ss;
     }
     __syncthreads();
-    for (int i = tid; i < G * kT; i += kGemmThreads) {
-        const float2 u = p.ux[(size_t)tb * G * kT + i];
-        s_ux[i] = make_float2(u.x * s_ss[i & (kT - 1)], u.y);
+    for (int i = tid; i < G * TT; i += kGemmThreads) {
+        const int g = i / TT, t = i - g * TT;
+        const float2 u = p.ux[(size_t)(tb * G + g) * kT + t];
+        s_ux[i] = make_float2(u.x * s_ss[t], u.y);
     }
     tc_fence_before();
     __syncthreads();
@@ -315,11 +341,11 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
                     if (!weights || it >= primed) {
                         if (!pf_wait(bar_empty + 8 * s, ph, give_up, limit))
                             break;
-                        mbar_arrive_expect_tx(bar_full + 8 * s, weights ? kABytes : kBBytes);
+                        mbar_arrive_expect_tx(bar_full + 8 * s, weights ? kABytes : C::kCols * 128);
                         if (weights)
                             tma_load_2d_hint(st, ma, hs * 128, m0, bar_full + 8 * s, pol);
                         else
-                            tma_load_2d(st + kABytes, &map_b, hs * 128, tb * kN, bar_full + 8 * s);
+                            tma_load_2d(st + kABytes, &map_b, hs * 128, tb * C::kCols, bar_full + 8 * s);
                     }
                     if (++s == kStages) {
                         s = 0;
@@ -344,7 +370,6 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         // and two producer lanes 256 tokens through 16 layers of the 7B shape take 3.83 instead of 4.17 ms.
         if (lane == 0) {
             const int b = warp - 1;
-            static_assert(kStages == 4, "a group's two stages are 2 b and 2 b + 1");
             int mine = 0;                        // groups of the block that are this lane's: every second one
             for (int tile = first; tile < ntiles; tile += stride) {
                 const int g0 = (tile % p.ksplit) * gper;
@@ -352,25 +377,36 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
             }
             mine = (mine + 1 - b) / 2;
             bool ok = true;
-            uint32_t ph = 0;
-            const uint32_t d = tmem + (uint32_t)b * kAccCols, ta = base + (uint32_t)(2 * b) * kStageBytes;
-            for (; mine > 0 && ok; --mine, ph ^= 1u) {
-                ok = pf_wait(bar_acc_empty + 8 * b, ph ^ 1u, give_up, limit);
+            int pair = b % C::kPairs, acc = b % kAccs;             // of the lane's next group: two stages of the ring, an accumulator
+            uint32_t ph = (uint32_t)(b / C::kPairs) & 1u, pha = (uint32_t)(b / kAccs) & 1u;
+            for (; mine > 0 && ok; --mine) {
+                const uint32_t d = tmem + (uint32_t)(acc * C::kAccDist), ta = base + (uint32_t)(2 * pair) * kStageBytes;
+                ok = pf_wait(bar_acc_empty + 8 * acc, pha ^ 1u, give_up, limit);
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    ok = ok && pf_wait(bar_full + 8 * (2 * b + half), ph, give_up, limit);
+                    ok = ok && pf_wait(bar_full + 8 * (2 * pair + half), ph, give_up, limit);
                     if (!ok)
                         break;
                     tc_fence_after();
                     const uint32_t t = ta + (uint32_t)half * kStageBytes;
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        umma_i8(d, smem_desc_sw128(t + (uint32_t)kk * 32u), smem_desc_sw128(t + kABytes + (uint32_t)kk * 32u), kIdesc,
+                        umma_i8(d, smem_desc_sw128(t + (uint32_t)kk * 32u), smem_desc_sw128(t + kABytes + (uint32_t)kk * 32u), C::kIdesc,
                                 (half | kk) ? 1u : 0u);
-                    umma_commit(bar_empty + 8 * (2 * b + half));     // the stage may be refilled when these have read it
+                    umma_commit(bar_empty + 8 * (2 * pair + half));  // the stage may be refilled when these have read it
                 }
                 if (ok)
-                    umma_commit(bar_acc_full + 8 * b);               // the group's sums are complete
+                    umma_commit(bar_acc_full + 8 * acc);             // the group's sums are complete
+                pair += 2;
+                if (pair >= C::kPairs) {
+                    pair -= C::kPairs;
+                    ph ^= 1u;
+                }
+                acc += 2;
+                if (acc >= kAccs) {
+                    acc -= kAccs;
+                    pha ^= 1u;
+                }
             }
             if (!ok || *give_up) {
                 umma_commit(bar_fin + 8 * b);
@@ -380,11 +416,12 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
             }
         }
     } else if (warp >= 4) {
-        // ---- epilogue: thread = one row of the tile and half of the tokens, 32 sums in registers
+        // ---- epilogue: thread = one row of the tile and half of the tokens, their sums in registers
+        constexpr int kTH = C::kHalf, kCh = C::kChunk;
         const int q = warp & 3;                               // the quarter of tensor memory this warp may read
         const int th = (warp - 4) >> 2;                       // which half of the tokens
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(th * kTH);
-        long it = 0;
+        unsigned int it = 0;
         bool ok = true;
         for (int tile = first; tile < ntiles && ok; tile += stride) {
             int sg = 0, m0 = (tile / p.ksplit) * kTileM;
@@ -417,38 +454,43 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
                     if (g >= g1 || !ok)
                         continue;
                     const float2 ms = msq[j];
-                    const int b = (int)(it & 1);
-                    const uint32_t pha = (uint32_t)((it >> 1) & 1);
+                    const int b = (int)(it % kAccs);
+                    const uint32_t pha = (uint32_t)((it / kAccs) & 1);
                     // one answer for the warp: the loads below are the whole warp's
                     if (!__all_sync(0xffffffffu, pf_wait(bar_acc_full + 8 * b, pha, give_up, limit))) {
                         ok = false;
                         continue;
                     }
                     tc_fence_after();
-                    const uint32_t tacc = trow + (uint32_t)b * kAccCols;
-                    const float2 *ux = s_ux + g * kT + th * kTH;
-                    // in two halves: registers
+                    const uint32_t tacc = trow + (uint32_t)(b * C::kAccDist);
+                    const float2 *ux = s_ux + g * TT + th * kTH;
+                    // in parts: registers
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        uint32_t s0[16], s1[16], s2[16];
-                        static_assert(kTH == 32, "two 16-column loads per limb");
-                        tmem_ld16(tacc + 16 * half, s0);
-                        tmem_ld16(tacc + kT + 16 * half, s1);
-                        tmem_ld16(tacc + 2 * kT + 16 * half, s2);
+                    for (int c = 0; c < kTH; c += kCh) {
+                        uint32_t s0[kCh], s1[kCh], s2[kCh];
+                        if constexpr (kCh == 16) {
+                            tmem_ld16(tacc + c, s0);
+                            tmem_ld16(tacc + TT + c, s1);
+                            tmem_ld16(tacc + 2 * TT + c, s2);
+                        } else {
+                            tmem_ld8(tacc + c, s0);
+                            tmem_ld8(tacc + TT + c, s1);
+                            tmem_ld8(tacc + 2 * TT + c, s2);
+                        }
                         tmem_ld_wait();
-                        if (half == 1) {
+                        if (c + kCh == kTH) {
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0)
                                 mbar_arrive(bar_acc_empty + 8 * b);
                         }
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) {
+                        for (int k = 0; k < kCh; ++k) {
                             // |s0|, |s1| <= 256 * 255 * 128: the two lower limbs together still fit 32 bits
                             const float low = (float)((int)s1[k] * 256 + (int)s0[k]);
                             const float dsum = fmaf((float)(int)s2[k], 65536.0f, low);
-                            const float2 u = ux[16 * half + k];
-                            acc[16 * half + k] += fmaf(ms.y, dsum, ms.x * u.y) * u.x;
+                            const float2 u = ux[c + k];
+                            acc[c + k] += fmaf(ms.y, dsum, ms.x * u.y) * u.x;
                         }
                     }
                     ++it;
@@ -492,7 +534,9 @@ struct PfLimbParams {
     int lda;
     int n;                 // elements per token (multiple of 256)
     int nvalid;
-    int8_t *limbs;         // [token block][3 * 64][n]
+    int tpad;              // tokens of the chunk, whole blocks of 64 (distance of the parts)
+    int tt;                // tokens of a block of the B operand: 64, or what the matrix kernel of a call of few tokens takes
+    int8_t *limbs;         // [token block][3 * tt][n]
     float2 *ux;            // [token block][n / 256][64]: (value of one fixed-point unit, sum of the fixed-point activations)
     float *ssq;            // NORM: [token block][gridDim.y][64] partial sums of squares of the rows
 };
@@ -506,7 +550,7 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
     // flight at once
     __shared__ float s_ssq[kLimbWarps];
     const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tpad = gridDim.x, tb = t / kT, tl = t % kT;     // tokens of the chunk, whole blocks
+    const int tpad = p.tpad, tb = t / kT, tl = t % kT;
     const int G = p.n >> 8;
     const bool live = t < p.nvalid;
     float ssq = 0.f;
@@ -595,9 +639,9 @@ __global__ void __launch_bounds__(kLimbThreads) pf_limbs_kernel(const PfLimbPara
             const uint32_t t3 = __byte_perm(z[4 * h + 2], z[4 * h + 3], 0x0062);
             const uint32_t l0 = __byte_perm(t0, t2, 0x5410), l1 = __byte_perm(t0, t2, 0x7632), l2 = __byte_perm(t1, t3, 0x5410);
             const size_t e = (size_t)gi * 256 + h * 128 + lane * 4;
-            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)(tb * kN + 0 * kT + tl) * p.n + e) = l0;
-            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)(tb * kN + 1 * kT + tl) * p.n + e) = l1;
-            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)(tb * kN + 2 * kT + tl) * p.n + e) = l2;
+            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)((3 * tb + 0) * p.tt + tl) * p.n + e) = l0;
+            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)((3 * tb + 1) * p.tt + tl) * p.n + e) = l1;
+            *reinterpret_cast<uint32_t *>(p.limbs + (size_t)((3 * tb + 2) * p.tt + tl) * p.n + e) = l2;
             s0 = dp4a_ones(l0, s0);
             s1 = dp4a_ones(l1, s1);
             s2 = dp4a_ones(l2, s2);
@@ -1482,6 +1526,7 @@ __global__ void __launch_bounds__(kClsThreads, 1) bd_classifier_kernel(const __g
         named_barrier_sync(1, 32 * (kClsEpi + 1));
         tc_fence_after();
         const int quarter = warp & 3, th = (warp - kClsCvt) >> 2;
+        constexpr int kTH = kT / 2;           // tokens per thread
         const uint32_t trow = s_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(th * kTH);
         float acc[kTH];
 #pragma unroll
@@ -1610,6 +1655,17 @@ bool encode_bytes_2d(CUtensorMap *map, const void *base, int rows, int k, int bo
 
 }  // namespace
 
+// Token blocks that the matrix kernel is built for, and the one for n tokens in tb blocks of 64.
+constexpr int kTokenBlocks[4] = {16, 32, 48, 64};
+
+static int token_block(int tb, int n)
+{
+    for (int i = 0; tb == 1 && i < 3; ++i)
+        if (n <= kTokenBlocks[i])
+            return i;
+    return 3;
+}
+
 // What the kernels of one chunk hand to each other.
 struct Workspaces {
     int blocks = 0;              // blocks of 64 tokens they hold: one, or kTB
@@ -1618,7 +1674,7 @@ struct Workspaces {
     int8_t *limbs = nullptr;
     float2 *ux = nullptr;
     float *ssq = nullptr;        // [blocks][groups / 4][64]
-    CUtensorMap map_b_dim, map_b_hidden;
+    CUtensorMap map_b_dim[4], map_b_hidden[4];   // by size of the token block: kTokenBlocks
     char *mem = nullptr;         // all of them
 };
 
@@ -1629,7 +1685,7 @@ struct Prefill : Workspaces {
     std::vector<CUtensorMap> maps;   // [layer][PF_W_COUNT]
     int *tokens = nullptr;
     int token_cap = 0;
-    size_t gemm_smem_dim = 0, gemm_smem_hidden = 0, attn_smem = 0;
+    size_t attn_smem = 0;
     std::vector<void *> owned;
     unsigned long long launches = 0;
     // concurrent sequences
@@ -1733,9 +1789,12 @@ static cudaError_t make_workspaces(Prefill *pf, int blocks)
     if (e != cudaSuccess)
         return e;
     walk();
-    if (!encode_bytes_2d(&w.map_b_dim, w.limbs, blocks * kN, m.dim, kN, false) ||
-        !encode_bytes_2d(&w.map_b_hidden, w.limbs, blocks * kN, m.hidden, kN, false))
-        return cudaErrorNotSupported;
+    for (int i = 0; i < 4; ++i) {
+        const int cols = 3 * kTokenBlocks[i], rows = kTokenBlocks[i] == kT ? blocks * cols : cols;
+        if (!encode_bytes_2d(&w.map_b_dim[i], w.limbs, rows, m.dim, cols, false) ||
+            !encode_bytes_2d(&w.map_b_hidden[i], w.limbs, rows, m.hidden, cols, false))
+            return cudaErrorNotSupported;
+    }
     for (auto &g : pf->step_graphs)
         cudaGraphExecDestroy(g.second);
     pf->step_graphs.clear();
@@ -1789,13 +1848,15 @@ cudaError_t prefill_create(Prefill **out, const PrefillModel &m, cudaStream_t st
         prefill_destroy(pf);
         return cudaErrorNotSupported;
     }
-    // ring, unit table (at most 64 groups: 32 KB), alignment slack: below the 227 KB a block may have
-    pf->gemm_smem_dim = (size_t)kStages * kStageBytes + (size_t)(m.dim / 256) * kT * sizeof(float2) + 1024;
-    pf->gemm_smem_hidden = (size_t)kStages * kStageBytes + (size_t)(m.hidden / 256) * kT * sizeof(float2) + 1024;
     // (the limit belongs to the kernel on the device, not to this context: it covers every shape)
-    constexpr size_t gmax = (size_t)kStages * kStageBytes + (size_t)(kMaxDim / 256) * kT * sizeof(float2) + 1024;
-    static_assert(gmax <= 227 * 1024, "what a block may have");
-    e = cudaFuncSetAttribute(pf_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gmax);
+    auto limit = [](auto kernel, size_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+    e = limit(pf_gemm_kernel<16>, GemmCfg<16>::smem(kMaxDim / 256));
+    if (e == cudaSuccess)
+        e = limit(pf_gemm_kernel<32>, GemmCfg<32>::smem(kMaxDim / 256));
+    if (e == cudaSuccess)
+        e = limit(pf_gemm_kernel<48>, GemmCfg<48>::smem(kMaxDim / 256));
+    if (e == cudaSuccess)
+        e = limit(pf_gemm_kernel<64>, GemmCfg<64>::smem(kMaxDim / 256));
     pf->attn_smem = m.head == 128 ? attn_smem_bytes<128>() : attn_smem_bytes<64>();
     if (e == cudaSuccess)
         e = m.head == 128 ? cudaFuncSetAttribute(pf_attention_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf->attn_smem)
@@ -1889,11 +1950,17 @@ cudaError_t launch_gemm(Prefill *pf, cudaStream_t st, int layer, const int *w, i
     p.status = m.status;
     const CUtensorMap *base = &pf->maps[(size_t)layer * PF_W_COUNT];
     const CUtensorMap &a0 = base[w[0]], &a1 = base[w[nw > 1 ? 1 : 0]], &a2 = base[w[nw > 2 ? 2 : 0]];
-    const CUtensorMap &b = k == m.dim ? pf->map_b_dim : pf->map_b_hidden;
-    const size_t smem = k == m.dim ? pf->gemm_smem_dim : pf->gemm_smem_hidden;
+    const int t = token_block(tb, nvalid);
+    const CUtensorMap &b = k == m.dim ? pf->map_b_dim[t] : pf->map_b_hidden[t];
     const int per_block = pf->sms / tb;      // thread blocks per block of tokens
     const int grid = tb * (tiles * ksplit < per_block ? tiles * ksplit : per_block);
-    return launch(pf, st, pf_gemm_kernel, dim3((unsigned)grid), kGemmThreads, smem, a0, a1, a2, b, p);
+    auto go = [&](auto kernel, size_t smem) { return launch(pf, st, kernel, dim3((unsigned)grid), kGemmThreads, smem, a0, a1, a2, b, p); };
+    switch (kTokenBlocks[t]) {
+    case 16: return go(pf_gemm_kernel<16>, GemmCfg<16>::smem(p.groups));
+    case 32: return go(pf_gemm_kernel<32>, GemmCfg<32>::smem(p.groups));
+    case 48: return go(pf_gemm_kernel<48>, GemmCfg<48>::smem(p.groups));
+    default: return go(pf_gemm_kernel<64>, GemmCfg<64>::smem(p.groups));
+    }
 }
 
 template <int MODE>
@@ -1911,7 +1978,9 @@ cudaError_t launch_limbs(Prefill *pf, cudaStream_t st, float *a, const float *b,
     p.limbs = pf->limbs;
     p.ux = pf->ux;
     p.ssq = pf->ssq;
-    const dim3 grid((unsigned)(tb * kT), (unsigned)((n / 256 + kLimbWarps - 1) / kLimbWarps));
+    p.tpad = tb * kT;
+    p.tt = kTokenBlocks[token_block(tb, nvalid)];
+    const dim3 grid((unsigned)(tb > 1 ? tb * kT : p.tt), (unsigned)((n / 256 + kLimbWarps - 1) / kLimbWarps));
     return launch(pf, st, pf_limbs_kernel<MODE>, grid, kLimbThreads, 0, p);
 }
 
