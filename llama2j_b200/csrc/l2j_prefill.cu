@@ -299,25 +299,6 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
         tmem_alloc(smem_u32(&s_tmem), kTmemCols);
         tmem_relinquish();
     }
-    if (tid < TT) {
-        // RootMeanSquare.java:25-35: the scalar of the RMSNorm in front multiplies every unit of the token
-        float ss = 1.0f;
-        if (p.ssq != nullptr) {
-            float tot = 0.f;
-            for (int y = 0; y < p.nssq; ++y)
-                tot += p.ssq[(tb * p.nssq + y) * kT + tid];
-            tot = __fdiv_rn(tot, (float)p.n);
-            tot = __fadd_rn(tot, 1e-5f);
-            ss = __fdiv_rn(1.0f, __fsqrt_rn(tot));
-        }
-        s_ss[tid] = ss;
-    }
-    __syncthreads();
-    for (int i = tid; i < G * TT; i += kGemmThreads) {
-        const int g = i / TT, t = i - g * TT;
-        const float2 u = p.ux[(size_t)(tb * G + g) * kT + t];
-        s_ux[i] = make_float2(u.x * s_ss[t], u.y);
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -418,6 +399,28 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant
     } else if (warp >= 4) {
         // ---- epilogue: thread = one row of the tile and half of the tokens, their sums in registers
         constexpr int kTH = C::kHalf, kCh = C::kChunk;
+        // The table of units is the epilogue's alone: its loads (two trips to the L2) run beside the first tiles' copies and products.
+        const int et = tid - 128;
+        if (et < TT) {
+            // RootMeanSquare.java:25-35: the scalar of the RMSNorm in front multiplies every unit of the token
+            float ss = 1.0f;
+            if (p.ssq != nullptr) {
+                float tot = 0.f;
+                for (int y = 0; y < p.nssq; ++y)
+                    tot += p.ssq[(tb * p.nssq + y) * kT + et];
+                tot = __fdiv_rn(tot, (float)p.n);
+                tot = __fadd_rn(tot, 1e-5f);
+                ss = __fdiv_rn(1.0f, __fsqrt_rn(tot));
+            }
+            s_ss[et] = ss;
+        }
+        named_barrier_sync(1, 32 * kEpiWarps);
+        for (int i = et; i < G * TT; i += 32 * kEpiWarps) {
+            const int g = i / TT, t = i - g * TT;
+            const float2 u = p.ux[(size_t)(tb * G + g) * kT + t];
+            s_ux[i] = make_float2(u.x * s_ss[t], u.y);
+        }
+        named_barrier_sync(1, 32 * kEpiWarps);
         const int q = warp & 3;                               // the quarter of tensor memory this warp may read
         const int th = (warp - 4) >> 2;                       // which half of the tokens
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(th * kTH);
