@@ -32,7 +32,8 @@
 //   - the Wo phase's prologue merged the attention partials in every block (5 us); one block per head does it now, in 1.5.
 // Taken back: FP32 multiply-adds on unpacked bytes (a permute per byte: slower than three dp4a per four), asking the stages
 // behind the ring into the L2 (50 us: the extra requests delay the hand-overs), the same for RMSNorm weights and output lines.
-// 7B shape, 48 greedy forwards from position 0: 88.6 -> 72 ms; 8 steps behind 3840 positions: 22.3 -> 18 ms.
+// 7B shape, 48 greedy forwards from position 0: 88.6 -> 69.7 ms; 8 steps behind 3840 positions: 22.4 -> 17.8 ms; 13B shape, 24
+// forwards (from the per-step kernels): 70.2 -> 63.0 ms.
 //
 // Blocks wait for each other, so all of them must be resident: the grid is one block per SM.  Every wait is
 // bounded by the SM's cycle counter.  A hand-over between blocks that runs out raises L2J_DS_WAIT_TIMEOUT in
@@ -1232,6 +1233,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
         Epilogue es;
         es.rb = es.rround = 0;
         es.lost = es.lost_before = lost_at_entry;
+        // Every forward before this one has bumped the last phase's counter once per block.  If one is missing, the blocks of the
+        // context (or its host) have lost count: reported here too, because a stage of a layer split has no classifier that waits.
+        if (b == 0 && lane == 0 && ld_acquire_u32(P.sync + (int64_t)kSyncStride * (5 * P.n_layers - 1)) != (epoch - 1u) * (unsigned int)G)
+            atomicOr(&P.state->status, L2J_DS_WAIT_TIMEOUT);
         {
             float *rope_c = reinterpret_cast<float *>(smem + kFRopeOff);
             const int half = P.head >> 1;
