@@ -32,8 +32,8 @@
 //   - the Wo phase's prologue merged the attention partials in every block (5 us); one block per head does it now, in 1.5.
 // Taken back: FP32 multiply-adds on unpacked bytes (a permute per byte: slower than three dp4a per four), asking the stages
 // behind the ring into the L2 (50 us: the extra requests delay the hand-overs), the same for RMSNorm weights and output lines.
-// 7B shape, 48 greedy forwards from position 0: 88.6 -> 69.7 ms; 8 steps behind 3840 positions: 22.4 -> 17.8 ms; 13B shape, 24
-// forwards (from the per-step kernels): 70.2 -> 63.0 ms.
+// 7B shape, 48 greedy forwards from position 0: 88.6 -> 69.4 to 72.4 ms; 8 steps behind 3840 positions: 22.4 -> 17.8 to 18.5 ms; 13B shape, 24
+// forwards (from the per-step kernels): 70.2 -> 63.0 to 65.9 ms (by machine and allocation).
 //
 // Blocks wait for each other, so all of them must be resident: the grid is one block per SM.  Every wait is
 // bounded by the SM's cycle counter.  A hand-over between blocks that runs out raises L2J_DS_WAIT_TIMEOUT in
