@@ -1038,8 +1038,10 @@ static int create_impl(const l2j_config *cfg, int device, int first_layer, int l
     c->use_ring = !(flags & L2J_F_SIMPLE) && c->plan_qkv.ok && c->plan_wo.ok && c->plan_w13.ok && c->plan_hidden.ok &&
                   c->plan_cls.ok && (head % 2 == 0);
     {   // one persistent launch per token where every matrix has rows of whole quantisation groups
-        // (a lane's four elements of the attention output lie in one head)
-        bool fused = c->use_ring && tp_size == 1 && !(flags & L2J_F_STEP_KERNELS) && c->reps == 1 && c->dim % kGroup == 0 &&
+        // (a lane's four elements of the attention output lie in one head).  Its tags come from the forward counter, which the begin
+        // kernel keeps for contexts with hand-over counters only, and its blocks wait for each other: all of them must be
+        // resident at once.
+        bool fused = c->use_ring && c->chain_on && tp_size == 1 && !(flags & L2J_F_STEP_KERNELS) && c->reps == 1 && c->dim % kGroup == 0 &&
                      c->hidden % kGroup == 0 && c->dim <= kFusedMaxRow && c->hidden <= kFusedMaxRow &&
                      head % 8 == 0 && head <= 128;
         // Measured on B200, us per greedy token, per-step kernels / persistent kernel: 8 layers of dim 1024 229 / 151, 1536 261 / 174,
@@ -1059,8 +1061,10 @@ static int create_impl(const l2j_config *cfg, int device, int first_layer, int l
             fused = c->fplan[0].ok && c->fplan[1].ok && c->fplan[2].ok && c->fplan[3].ok;
         }
         if (fused) {
-            CREATE_CUDA(prepare_fused(&c->max_smem));
+            int resident = 0;
+            CREATE_CUDA(prepare_fused(232448, &c->max_smem, &resident));
             c->fused_smem = c->max_smem < 232448 ? c->max_smem : 232448;
+            fused = c->ring_grid <= resident;
             int largest = 0;
             for (int k = 0; k < 4; ++k)
                 largest = c->fplan[k].slot_bytes > largest ? c->fplan[k].slot_bytes : largest;

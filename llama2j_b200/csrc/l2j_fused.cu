@@ -1318,19 +1318,26 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
         atomicOr(&P.state->status, L2J_DS_WAIT_TIMEOUT);
 }
 
-cudaError_t prepare_fused(int *max_smem)
+// max_smem: shared memory that a block may have; resident: how many blocks of want_smem bytes (max_smem at most) the device holds at once.
+cudaError_t prepare_fused(int want_smem, int *max_smem, int *resident)
 {
-    int dev = 0, optin = 0;
+    int dev = 0, optin = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess)
         return e;
     if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
         return e;
-    if (max_smem)
-        *max_smem = optin;
+    *max_smem = optin;
     if ((e = cudaFuncSetAttribute(fused_layers_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) != cudaSuccess)
         return e;
-    return cudaFuncSetAttribute(fused_layers_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if ((e = cudaFuncSetAttribute(fused_layers_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess)
+        return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_layers_kernel, kFusedThreads,
+                                                      (size_t)(want_smem < optin ? want_smem : optin));
+    *resident = per_sm * sms;
+    return e;
 }
 
 cudaError_t launch_fused(cudaStream_t stream, bool pdl, int grid, int smem_bytes, const FusedParams &p)

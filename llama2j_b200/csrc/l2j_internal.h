@@ -235,7 +235,7 @@ constexpr int kFusedConsWarps = 14;
 constexpr int kFusedMaxRow = 4 * kFusedConsWarps * kGroup;   // longest matrix row: a warp spans four groups
 constexpr int kFusedHeaderBytes = 4096;   // barriers, descriptors, reduction buffers in front of the vector area and the ring
 
-cudaError_t prepare_fused(int *max_smem);
+cudaError_t prepare_fused(int want_smem, int *max_smem, int *resident);
 cudaError_t launch_fused(cudaStream_t stream, bool pdl, int grid, int smem_bytes, const FusedParams &p);
 
 // Blocks per head of the stand-alone attention kernel: as many as fit on the device at once (two blocks per SM are

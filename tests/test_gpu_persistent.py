@@ -73,3 +73,30 @@ def test_embedding_at_the_ends_of_the_range(value):
         assert np.array_equal(np.isnan(x), np.isnan(y))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("name,value", [("L2J_CHAIN", "0"), ("L2J_BLOCKS_PER_SM", "2")])
+@pytest.mark.parametrize("flags", [0, L.F_PERSISTENT])
+def test_switches_that_take_away_what_the_kernel_needs(monkeypatch, name, value, flags):
+    """No forward counter, or more blocks than are resident at once: the context runs the per-step kernels, with their bits."""
+    cfg = ModelConfig(dim=1280, hidden_dim=2304, n_layers=2, n_heads=10, n_kv_heads=2, vocab_size=500, seq_len=16, shared_classifier=True)
+    tensors = syn.synthetic_tensors(cfg, 11)
+    monkeypatch.setenv(name, value)
+    a, b = (Transformer(cfg, 0, 0, None, f) for f in (flags, L.F_STEP_KERNELS))
+    assert not a.launch_mode()["persistent"]
+    for m in (a, b):
+        m.upload_all(tensors)
+        m.finalize()
+    for p, t in enumerate((1, 17, 400)):
+        assert np.array_equal(a.forward(t, p)[0], b.forward(t, p)[0])
+    assert a.stats().device_status == 0
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("dim,hidden,heads", [(768, 2048, 12), (1024, 2816, 8), (1536, 4096, 12), (2560, 6912, 20)])
+def test_which_kernel_is_the_default(dim, hidden, heads):
+    cfg = ModelConfig(dim=dim, hidden_dim=hidden, n_layers=1, n_heads=heads, n_kv_heads=heads, vocab_size=256, seq_len=8, shared_classifier=True)
+    m = Transformer(cfg, 0)
+    assert m.launch_mode()["persistent"] == (dim >= 1024)
+    m.close()
