@@ -2506,10 +2506,14 @@ extern "C" int l2j_read_buffer(l2j_ctx *c, int which, int layer, int pos, float 
     }
     if (n > len)
         return fail(c, L2J_E_INVALID, "buffer %d holds %d floats", which, len);
-    if (c->tp_size > 1 && (which == 1 || which == 3)) {
-        // these vectors exist only as (value, sequence number) pairs in the receive buffers
+    const float2 *vec = nullptr;   // vectors that exist only as (value, sequence number) pairs
+    if (c->tp_size > 1 && (which == 1 || which == 3))
+        vec = c->ll_buf[which == 1 ? TPV_XB : TPV_HB];
+    else if (c->use_fused && which == 1)
+        vec = c->fused.o_pairs;
+    if (vec) {
         std::vector<float2> pairs((size_t)n);
-        CK(c, cudaMemcpy(pairs.data(), c->ll_buf[which == 1 ? TPV_XB : TPV_HB], sizeof(float2) * (size_t)n, cudaMemcpyDeviceToHost));
+        CK(c, cudaMemcpy(pairs.data(), vec, sizeof(float2) * (size_t)n, cudaMemcpyDeviceToHost));
         for (int i = 0; i < n; ++i)
             out[i] = pairs[(size_t)i].x;
         return L2J_OK;

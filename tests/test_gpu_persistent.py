@@ -48,7 +48,7 @@ def test_against_step_kernels(dim, hidden, heads, kv):
         if want:
             assert float(np.abs(x - y).max()) <= TOL * float(y.max() - y.min()), p
     # what the launch leaves behind for readers
-    for which, n in ((0, dim), (2, dim), (3, hidden)):      # x, q, the hidden vector
+    for which, n in ((0, dim), (1, dim), (2, dim), (3, hidden)):      # x, the attention output, q, the hidden vector
         x, y = a.read_buffer(which, n), b.read_buffer(which, n)
         assert float(np.abs(x - y).max()) <= TOL * float(np.abs(y).max()), which
     assert a.stats().device_status == 0
