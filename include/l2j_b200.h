@@ -83,7 +83,8 @@ enum l2j_tensor {
 #define L2J_F_SIMPLE 0x4      /* plain direct-load matvec kernels (cross-check path, slower) */
 #define L2J_F_STEP_KERNELS 0x8 /* one kernel per step of a layer (5 per layer) instead of one persistent kernel per token */
 #define L2J_F_NO_TENSOR_PREFILL 0x40  /* l2j_prefill pushes the prompt through the decode step (what shapes the tensor-core path does not take get anyway) */
-#define L2J_F_PERSISTENT 0x20  /* the persistent kernel wherever the shape allows it (default: only where it is the faster one) */
+#define L2J_F_PERSISTENT 0x20  /* the persistent kernel wherever the shape allows it (default: dim 1024 to 7168, where it is the faster one; it is
+                                * faster at some narrower widths too, which keep the per-step kernels by default) */
 #define L2J_F_TP_SPLIT_CLASSIFIER 0x10 /* l2j_create_tp: split the classifier's rows over the ranks too (they exchange their best candidates) */
 
 typedef struct l2j_ctx l2j_ctx;

@@ -1044,12 +1044,14 @@ static int create_impl(const l2j_config *cfg, int device, int first_layer, int l
         bool fused = c->use_ring && c->chain_on && tp_size == 1 && !(flags & L2J_F_STEP_KERNELS) && c->reps == 1 && c->dim % kGroup == 0 &&
                      c->hidden % kGroup == 0 && c->dim <= kFusedMaxRow && c->hidden <= kFusedMaxRow &&
                      head % 8 == 0 && head <= 128;
-        // Measured on B200, us per greedy token, per-step kernels / persistent kernel: 8 layers of dim 1024 229 / 151, 1536 261 / 174,
-        // 2048 297 / 200, 2560 326 / 235, 3072 356 / 261, 3584 403 / 328, 6144 695 / 631; 16 layers of the 7B shape 943 / 771, of the 13B
-        // shape 1230 / 1096 (short contexts) and 1261 / 1170 (200 positions).  The narrowest shapes stay with the per-step
-        // kernels unless asked otherwise, although the 110M shape gains too (287 / 226): what runs there by default is documented
-        // behaviour (five launches per layer, bit for bit those of L2J_F_STEP_KERNELS).
-        if (!(flags & L2J_F_PERSISTENT) && c->dim < 1024)
+        // The default lies between two widths.  Measured on B200, per-step kernels / persistent kernel, 10 and 4000 positions: from
+        // dim 1024 up to 7168 the persistent kernel is ahead everywhere (1024 248/186 and 347/312 us, 4096 481/384 and 815/633, 5120
+        // 620/545 and 1002/851, 7168 475/437 and 745/682).  Longer rows take more than half of its consumer warps, so the others
+        // idle: 7424 398/447 and 597/644, 8192 543/569 and 864/856, 9216 484/496 and 744/756 (4 to 8 layers, hidden 2816 to 14336).
+        // Narrower shapes stay with the per-step kernels although the 110M shape would gain (287/226): which kernels run there
+        // is documented.
+        const bool two_sets = (c->dim / kGroup + 3) / 4 <= kFusedConsWarps / 2;
+        if (!(flags & L2J_F_PERSISTENT) && (c->dim < 1024 || !two_sets))
             fused = false;
         if (const char *e = getenv("L2J_FUSED"))   // diagnostic: A/B against the per-step kernels
             fused = fused && atoi(e) != 0;

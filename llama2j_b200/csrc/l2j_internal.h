@@ -94,7 +94,7 @@ struct MvSeg {
 // Tensor-parallel group of up to kMaxTp devices driven by one process.  Every rank computes a block of
 // rows of each matrix from the full input vector and stores its results into every rank's copy of the
 // output vector over the peer links, so each output element is produced by one rank in the same order
-// as on a single device: the ranks' vectors stay bitwise equal, and equal to the single-device ones.
+// as by the per-step kernels of a single device: the ranks' vectors stay bitwise equal, and equal to theirs.
 constexpr int kMaxTp = 8;
 enum TpVector { TPV_X = 0, TPV_XB = 1, TPV_HB = 2, TPV_CAND = 3, TPV_COUNT = 4 };   // CAND: (max, index) of every rank's block of logits
 struct TpTable {

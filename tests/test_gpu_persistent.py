@@ -94,9 +94,12 @@ def test_switches_that_take_away_what_the_kernel_needs(monkeypatch, name, value,
     b.close()
 
 
-@pytest.mark.parametrize("dim,hidden,heads", [(768, 2048, 12), (1024, 2816, 8), (1536, 4096, 12), (2560, 6912, 20)])
-def test_which_kernel_is_the_default(dim, hidden, heads):
-    cfg = ModelConfig(dim=dim, hidden_dim=hidden, n_layers=1, n_heads=heads, n_kv_heads=heads, vocab_size=256, seq_len=8, shared_classifier=True)
-    m = Transformer(cfg, 0)
-    assert m.launch_mode()["persistent"] == (dim >= 1024)
-    m.close()
+@pytest.mark.parametrize("dim,heads,persistent", [(768, 12, False), (1024, 8, True), (1536, 12, True), (2560, 20, True), (7168, 56, True),
+                                                  (7424, 58, False), (8192, 64, False)])
+def test_which_kernel_is_the_default(dim, heads, persistent):
+    """From dim 1024 on, as long as a row leaves room for two sets of consumer warps (28 groups)."""
+    cfg = ModelConfig(dim=dim, hidden_dim=2816, n_layers=1, n_heads=heads, n_kv_heads=heads, vocab_size=256, seq_len=8, shared_classifier=True)
+    for flags, want in ((0, persistent), (L.F_PERSISTENT, True), (L.F_STEP_KERNELS, False)):
+        m = Transformer(cfg, 0, 0, None, flags)
+        assert m.launch_mode()["persistent"] == want
+        m.close()
