@@ -87,6 +87,12 @@ enum l2j_tensor {
                                 * faster at some narrower widths too, which keep the per-step kernels by default) */
 #define L2J_F_TP_SPLIT_CLASSIFIER 0x10 /* l2j_create_tp: split the classifier's rows over the ranks too (they exchange their best candidates) */
 
+/* Contexts may share a device, and be used from a thread each.  The blocks of the persistent kernel wait for each other and
+ * hold every SM; the launch is cooperative, so two contexts' kernels take turns.  A wait is bounded by the context's limit
+ * (l2j_set_wait_limit_us): a kernel of another program that holds some SMs for longer than that while the others already
+ * run the persistent kernel ends the forward with L2J_E_DEVICE.  Where that can happen set a longer limit or
+ * L2J_F_STEP_KERNELS. */
+
 typedef struct l2j_ctx l2j_ctx;
 
 typedef struct l2j_stats {

@@ -35,11 +35,11 @@
 // 7B shape, 48 greedy forwards from position 0: 88.6 -> 69.4 to 72.4 ms; 8 steps behind 3840 positions: 22.4 -> 17.8 to 18.5 ms; 13B shape, 24
 // forwards (from the per-step kernels): 70.2 -> 63.0 to 65.9 ms (by machine and allocation).
 //
-// Blocks wait for each other, so all of them must be resident: the grid is one block per SM.  Every wait is
-// bounded by the SM's cycle counter.  A hand-over between blocks that runs out raises L2J_DS_WAIT_TIMEOUT in
-// the status word, and every later hand-over of the forward gives up after 2 us; the block then still works
-// through all of its stages with the (wrong) inputs it has, so that producer, consumers and epilogue warp stay
-// in step and no bulk copy is in flight when the block ends.
+// Blocks wait for each other, so all of them must be resident: the grid is one block per SM and the launch is
+// cooperative.  Every wait is bounded by the SM's cycle counter.  A hand-over between blocks that runs out raises
+// L2J_DS_WAIT_TIMEOUT in the status word, and every later hand-over of the forward gives up after 2 us; the block then
+// still works through all of its stages with the (wrong) inputs it has, so that producer, consumers and epilogue warp
+// stay in step and no bulk copy is in flight when the block ends.
 //
 // Reference counterparts (paths relative to src/main/java/com/lastbot/llama2j/): the layer body of
 // Run.java:418-508 with kernel/MatMul.java:360-444, RootMeanSquare.java:78-118,
@@ -1347,11 +1347,16 @@ cudaError_t launch_fused(cudaStream_t stream, bool pdl, int grid, int smem_bytes
     cfg.blockDim = dim3(kFusedThreads);
     cfg.dynamicSmemBytes = (size_t)smem_bytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    // Cooperative: the blocks wait for each other, so either all of them get onto the device or none does, also while another
+    // context's persistent kernel wants the same SMs.  Costs nothing that can be measured (4 layers of dim 1280, 400 forwards: 39.5 ms
+    // with and without).
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = pdl ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, fused_layers_kernel, p);
 }
 

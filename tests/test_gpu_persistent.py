@@ -3,6 +3,8 @@
 Both form the same products from the same 24-bit activations and add the FP32 group terms of a row in other orders; a row of g groups
 is then off by at most about g roundings of 2^-24 of its terms, and two layers of them move a logit by a few 1e-6 of the range
 (observed: 1e-6).  The bound is 1e-5."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -102,4 +104,53 @@ def test_which_kernel_is_the_default(dim, heads, persistent):
     for flags, want in ((0, persistent), (L.F_PERSISTENT, True), (L.F_STEP_KERNELS, False)):
         m = Transformer(cfg, 0, 0, None, flags)
         assert m.launch_mode()["persistent"] == want
+        m.close()
+
+
+def test_contexts_that_work_at_the_same_time():
+    """Two persistent kernels want all SMs, a prompt's kernels some of them: everybody gets what they get alone."""
+    cfg = ModelConfig(dim=1280, hidden_dim=2816, n_layers=4, n_heads=10, n_kv_heads=10, vocab_size=2000, seq_len=512, shared_classifier=True)
+    tensors = syn.synthetic_tensors(cfg, 12)
+    prompt = syn.synthetic_prompt(300, 3, cfg.vocab_size)
+
+    def greedy(m):
+        m.reset()
+        return m.generate_greedy(prompt[:8], 300)
+
+    def host_loop(m):
+        m.reset()
+        return np.array([m.forward(int(prompt[p]), p)[0].copy() for p in range(200)])
+
+    def prompts(m):
+        m.reset()
+        m.prefill(prompt, 0)
+        return m.forward(7, prompt.size)[0].copy()
+
+    jobs = [greedy, host_loop, prompts, greedy]
+    models = []
+    for _ in jobs:
+        m = Transformer(cfg, 0)
+        m.upload_all(tensors)
+        m.finalize()
+        models.append(m)
+    assert models[0].launch_mode()["persistent"]
+    alone = [job(m) for job, m in zip(jobs, models)]
+    bad = []
+
+    def work(i):
+        try:
+            for _ in range(4):
+                if not np.array_equal(jobs[i](models[i]), alone[i]):
+                    bad.append((i, "other results"))
+        except L.L2jError as e:
+            bad.append((i, str(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for m in models:
+        assert m.stats().device_status == 0
         m.close()
