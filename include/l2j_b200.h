@@ -276,6 +276,15 @@ L2J_API int l2j_set_wait_limit_us(l2j_ctx *ctx, int limit_us);
  * usable again.  Nothing faults: every wait gives up and the kernels return. */
 L2J_API int l2j_debug_desync(l2j_ctx *ctx);
 
+/* The same for the waits inside the persistent kernel, one kind at a time (a context that runs it; else L2J_E_STATE): from
+ * now on these readers wait for pairs that nobody writes, until l2j_reset.  Partial results exist only where a head's
+ * positions are dealt to several blocks. */
+#define L2J_LATE_INPUT 0x1     /* the input vectors of the matrices */
+#define L2J_LATE_ROWS 0x2      /* the query and this token's key and value in the attention step */
+#define L2J_LATE_PARTIALS 0x4  /* the attention step's partial results */
+#define L2J_LATE_RESIDUAL 0x8  /* old values of the residual stream in the last matrix, in all lanes but a warp's first */
+L2J_API int l2j_debug_late(l2j_ctx *ctx, int readers);
+
 /* The same for allocations: the nth device or pinned allocation that the context makes from now on (prompt
  * workspaces, caches of concurrent sequences, sampler: whatever is made on first use) fails as if memory had run
  * out; 0 takes the injection back.  The call answers with L2J_E_NOMEM and may be made again, or takes a way that

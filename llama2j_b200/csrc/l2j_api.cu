@@ -2287,6 +2287,21 @@ extern "C" int l2j_debug_desync(l2j_ctx *c)
     return L2J_OK;
 }
 
+extern "C" int l2j_debug_late(l2j_ctx *c, int readers)
+{
+    if (!c)
+        return L2J_E_INVALID;
+    std::lock_guard<std::mutex> lock(c->mu);
+    if (readers < 0 || readers > (L2J_LATE_INPUT | L2J_LATE_ROWS | L2J_LATE_PARTIALS | L2J_LATE_RESIDUAL))
+        return fail(c, L2J_E_INVALID, "unknown readers 0x%x", readers);
+    if (!c->finalized || !c->use_fused)
+        return fail(c, L2J_E_STATE, "needs a finalized context that runs the persistent kernel");
+    CK(c, cudaSetDevice(c->device));
+    CK(c, cudaStreamSynchronize(c->stream));
+    CK(c, cudaMemcpy(c->chain + (int64_t)kChainStride * (5 * c->nl + 1) + 1, &readers, sizeof(readers), cudaMemcpyHostToDevice));
+    return L2J_OK;
+}
+
 extern "C" int l2j_debug_fail_alloc(l2j_ctx *c, int nth)
 {
     if (!c || nth < 0)

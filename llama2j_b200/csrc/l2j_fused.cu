@@ -37,8 +37,8 @@
 //
 // Blocks wait for each other, so all of them must be resident: the grid is one block per SM and the launch is
 // cooperative.  Every wait is bounded by the SM's cycle counter.  A hand-over between blocks that runs out raises
-// L2J_DS_WAIT_TIMEOUT in the status word, and every later hand-over of the forward gives up after 2 us; the block then
-// still works through all of its stages with the (wrong) inputs it has, so that producer, consumers and epilogue warp
+// L2J_DS_WAIT_TIMEOUT in the status word, and every hand-over that any warp of the block still waits for gives up after 2 us;
+// the block then still works through all of its stages with the (wrong) inputs it has, so that producer, consumers and epilogue warp
 // stay in step and no bulk copy is in flight when the block ends.
 //
 // Reference counterparts (paths relative to src/main/java/com/lastbot/llama2j/): the layer body of
@@ -53,6 +53,10 @@
 #include <cmath>
 
 #define L2J_DS_WAIT_TIMEOUT 0x1
+#define L2J_LATE_INPUT 0x1
+#define L2J_LATE_ROWS 0x2
+#define L2J_LATE_PARTIALS 0x4
+#define L2J_LATE_RESIDUAL 0x8
 
 namespace l2j {
 
@@ -68,18 +72,21 @@ constexpr int kFBarEmpty = 128;         // uint64 empty[16]
 constexpr int kFBarRedFull = 256;       // uint64 red_full[4]
 constexpr int kFBarRedEmpty = 288;      // uint64 red_empty[4]
 constexpr int kFVStart = 328;           // int vstart[16]: the producer's bookkeeping of where each stage in flight begins
-constexpr int kFScratch = 392;          // float scratch[16]
+constexpr int kFScratch = 392;          // float scratch[14]
+constexpr int kFLost = 448;             // int: a wait of the block has run out, or one of an earlier forward had
+constexpr int kFLate = 452;             // int: the L2J_LATE_* bits
 constexpr int kFDescOff = 512;          // FStage desc[16]
-constexpr int kFRedOff = 1024;          // 4 x 128 floats: [stage of the group][row of the stage][warp of the row]
+constexpr int kFRedOff = 1024;          // 4 x 112 floats: [stage of the group][row of the stage][warp of the row]
 constexpr int kFRedStride = 4 * kFGroup * 2 * kFusedConsWarps;   // a stage has two rows per set of warps
 constexpr int kFRopeOff = 3328;         // float cos[64], sin[64] of the token's position
 constexpr int kFInvTab = 3840;          // float inv[64]: value of one fixed-point unit of each group of the input vector
 constexpr int kFHeader = kFusedHeaderBytes;   // end of the fixed part (128-byte aligned)
-static_assert(kFScratch + 4 * kFusedConsWarps <= kFDescOff && kFRedOff + kFRedBufs * kFRedStride <= kFRopeOff, "header layout");
+static_assert(kFScratch + 4 * kFusedConsWarps <= kFLost && kFLate + 4 <= kFDescOff && kFRedOff + kFRedBufs * kFRedStride <= kFRopeOff, "header layout");
 static_assert(kFInvTab + 4 * (kFusedMaxRow / 256) <= kFHeader, "header layout");
 constexpr int kFCons = kFusedConsWarps * 32;
 constexpr int kAttBatch = 4;            // cached positions that a lane group works on at a time
 constexpr uint64_t kFShortWaitNs = 2000;
+constexpr int kFLateTag = 0x40000000;   // what a reader's tag is off by while l2j_debug_late makes it wait for nothing
 
 struct FStage {
     int off, nrows, e0a, e0b;   // what the consumers of a matrix stage need, in one 16-byte load: byte offset in the
@@ -141,6 +148,33 @@ __device__ __forceinline__ bool tagged(const float4 &v, int tag)
     return __float_as_int(v.y) == tag && __float_as_int(v.w) == tag;
 }
 
+// The block's word for "a wait has run out": whichever warp it was, every hand-over that the block still waits for gives up early.
+__device__ __forceinline__ void set_block_lost(uint32_t sbase)
+{
+    asm volatile("st.volatile.shared.s32 [%0], 1;" ::"r"(sbase + kFLost) : "memory");
+}
+
+// A reader's tag: the one it waits for, or one that nobody writes while l2j_debug_late says so.
+__device__ __forceinline__ int reader_tag(uint32_t sbase, int tag, int reader)
+{
+    int late;
+    asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(late) : "r"(sbase + kFLate) : "memory");
+    return late & reader ? tag ^ kFLateTag : tag;
+}
+
+__device__ __forceinline__ bool block_lost(uint32_t sbase)
+{
+    int v;
+    asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(v) : "r"(sbase + kFLost) : "memory");
+    return v != 0;
+}
+
+// Has a hand-over that the block waits for since c0 run out?
+__device__ __forceinline__ bool hand_over_lost(uint32_t sbase, long long c0, uint64_t wait_ns)
+{
+    return sm_clock() - c0 > (long long)(2 * (block_lost(sbase) ? kFShortWaitNs : wait_ns));
+}
+
 // Bulk copy without a cache hint (cached K/V rows are read again by the next token).
 __device__ __forceinline__ void bulk_g2s_plain(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
 {
@@ -178,7 +212,6 @@ struct Fold {
 // kAttChunk positions), head-major, in contiguous runs over the first `ga` blocks.
 struct AttSplit {
     int nchunk, units, ga;
-    int np_max;   // partial results per head at most
 };
 
 __device__ __forceinline__ AttSplit att_split(const FusedParams &P, int pos, int grid)
@@ -190,7 +223,6 @@ __device__ __forceinline__ AttSplit att_split(const FusedParams &P, int pos, int
     // few enough (four) for the step behind to fetch them in one round of loads.
     const int per_head = a.nchunk <= 512 / kAttChunk ? 3 : kAttMaxSplit;
     a.ga = min(min(grid, P.n_heads * per_head), a.units);
-    a.np_max = min(a.nchunk, (a.ga + P.n_heads - 1) / P.n_heads + 1);
     return a;
 }
 
@@ -253,7 +285,6 @@ struct Producer {
     int ring_bytes;
     int seq, tail;          // descriptors issued / known to be released
     int vtail;              // where the oldest stage not known to be released begins
-    bool lost;
     uint64_t wait_ns;
     int pos;                // the token's position, -1 until the kernel in front has set it
     AttSplit as;
@@ -270,7 +301,7 @@ struct Producer {
         while (tail < seq && (seq - tail >= kFDesc || vend - ring_bytes > vtail)) {
             if (!mbar_wait_bounded(sbase + kFBarEmpty + 8 * (tail % kFDesc), (uint32_t)(tail / kFDesc) & 1u,
                                    wait_ns))
-                lost = true;
+                set_block_lost(sbase);
             ++tail;
             vtail = vstart[tail % kFDesc];
         }
@@ -391,7 +422,6 @@ __device__ __forceinline__ void produce_att_stage(Producer &pr, const FusedParam
 struct Consumer {
     int seq;             // stages consumed so far (descriptor index = seq mod kFDesc)
     int rb, rround;      // position in the ring of reduction buffers
-    bool lost, lost_before;
 };
 
 // A lane's sixteen elements of a quantisation group of an input vector: pairs 64 q.. 64 q + 3 from p on, q = 0..3.
@@ -407,7 +437,7 @@ __device__ __forceinline__ void issue_pairs(const float2 *p, float4 (&v)[8])
 // Those of them that have not arrived yet are asked for again until they carry `tag`.  While nothing at all has come for
 // the warp only an eighth of them is asked for: 148 blocks that poll whole vectors would take as much of the L2 as the
 // weight stream does.
-__device__ __forceinline__ void poll_pairs(const float2 *p, float4 (&v)[8], int tag, Consumer &cs, uint64_t wait_ns)
+__device__ __forceinline__ void poll_pairs(const float2 *p, float4 (&v)[8], int tag, uint32_t sbase, uint64_t wait_ns)
 {
     auto all = [&]() {
         bool ok = true;
@@ -418,7 +448,6 @@ __device__ __forceinline__ void poll_pairs(const float2 *p, float4 (&v)[8], int 
     };
     if (all())
         return;
-    const long long limit = (long long)(2 * (cs.lost ? kFShortWaitNs : wait_ns));
     const long long c0 = sm_clock();
     for (;;) {
         const bool some = tagged(v[0], tag);
@@ -432,8 +461,8 @@ __device__ __forceinline__ void poll_pairs(const float2 *p, float4 (&v)[8], int 
         }
         if (all())
             return;
-        if (__any_sync(0xffffffffu, sm_clock() - c0 > limit)) {
-            cs.lost = true;
+        if (__any_sync(0xffffffffu, hand_over_lost(sbase, c0, wait_ns))) {
+            set_block_lost(sbase);
             return;
         }
     }
@@ -496,7 +525,7 @@ __device__ __forceinline__ void consume_ring_phase(const FusedParams &P, const M
             if (in_pairs) {
                 float4 v[8];
                 issue_pairs(in_pairs + e, v);
-                poll_pairs(in_pairs + e, v, tag, cs, wait_ns);
+                poll_pairs(in_pairs + e, v, tag, sbase, wait_ns);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     xg[2 * q] = v[q].x;
@@ -676,7 +705,7 @@ __device__ __forceinline__ void consume_ring_phase(const FusedParams &P, const M
     auto wait = [&](int t) {
         const uint32_t at = (e + (uint32_t)t) & (kFDesc - 1);
         if (!mbar_wait_bounded(sbase + kFBarFull + 8 * at, parity ^ (at < e ? 1u : 0u), wait_ns))
-            cs.lost = true;
+            set_block_lost(sbase);
         return at;
     };
     auto release = [&](int t) {      // this warp is done with the stage's bytes
@@ -734,7 +763,7 @@ __device__ __forceinline__ void consume_ring_phase(const FusedParams &P, const M
         const float tot = Fold<2 * kFGroup, 16>::run(v, lane) * rms;   // lanes 4 i.. hold the sum of v[i]
         if (cs.rround > 0) {
             if (!mbar_wait_bounded(sbase + kFBarRedEmpty + 8 * cs.rb, (uint32_t)(cs.rround - 1) & 1u, wait_ns))
-                cs.lost = true;
+                set_block_lost(sbase);
         }
         float *red = reinterpret_cast<float *>(smem + kFRedOff + cs.rb * kFRedStride);
         if (active && (lane & 3) == 0) {
@@ -785,7 +814,7 @@ __device__ __forceinline__ void consume_attention(const FusedParams &P, int tag,
         for (int z = 0; z < 6; ++z)
             a[z] = make_float4(0.f, 0.f, 0.f, 0.f);
         const long long c0 = sm_clock();
-        const long long limit = (long long)(2 * (cs.lost ? kFShortWaitNs : wait_ns));
+        const int rtag = reader_tag(sbase, tag, L2J_LATE_ROWS);
         for (;;) {
             if (want0) {
                 a[0] = ld_pairs2_gpu(s0);
@@ -797,12 +826,12 @@ __device__ __forceinline__ void consume_attention(const FusedParams &P, int tag,
                 a[4] = ld_pairs2_gpu(s2);
                 a[5] = ld_pairs2_gpu(s2 + 2);
             }
-            const bool ok = (!want0 || (tagged(a[0], tag) && tagged(a[1], tag))) &&
-                            (!want12 || (tagged(a[2], tag) && tagged(a[3], tag) && tagged(a[4], tag) && tagged(a[5], tag)));
+            const bool ok = (!want0 || (tagged(a[0], rtag) && tagged(a[1], rtag))) &&
+                            (!want12 || (tagged(a[2], rtag) && tagged(a[3], rtag) && tagged(a[4], rtag) && tagged(a[5], rtag)));
             if (__all_sync(0xffffffffu, ok))
                 break;
-            if (__any_sync(0xffffffffu, sm_clock() - c0 > limit)) {
-                cs.lost = true;
+            if (__any_sync(0xffffffffu, hand_over_lost(sbase, c0, wait_ns))) {
+                set_block_lost(sbase);
                 break;
             }
         }
@@ -829,8 +858,8 @@ __device__ __forceinline__ void consume_attention(const FusedParams &P, int tag,
         FStage d{};
         if (u < u1) {
             if (!mbar_wait_bounded(sbase + kFBarFull + 8 * e, (uint32_t)(cs.seq / kFDesc) & 1u, wait_ns))
-                cs.lost = true;
-            cs.lost = __any_sync(0xffffffffu, cs.lost) != 0;   // the shuffles below need a warp-uniform decision
+                set_block_lost(sbase);
+            __syncwarp();     // one descriptor for the whole warp, also behind a wait that ran out in some lanes
             d = *(reinterpret_cast<const FStage *>(smem + kFDescOff) + e);
         }
         const int h = u < u1 ? d.seg : -1;
@@ -985,24 +1014,24 @@ __device__ __forceinline__ void consume_attention(const FusedParams &P, int tag,
             if (z < others)
                 o[z] = ld_pair_gpu(src + (int64_t)z * (head + 2));
         const long long c0 = sm_clock();
-        const long long limit = (long long)(2 * (cs.lost ? kFShortWaitNs : wait_ns));
+        const int ptag = reader_tag(sbase, tag, L2J_LATE_PARTIALS);
         for (;;) {
-            bool ok = tagged(ml, tag);
+            bool ok = tagged(ml, ptag);
 #pragma unroll
             for (int z = 0; z < kAttSlots - 1; ++z)
                 if (z < others)
-                    ok = ok && __float_as_int(o[z].y) == tag;
+                    ok = ok && __float_as_int(o[z].y) == ptag;
             if (__all_sync(0xffffffffu, ok))
                 break;
-            if (__any_sync(0xffffffffu, sm_clock() - c0 > limit)) {
-                cs.lost = true;
+            if (__any_sync(0xffffffffu, hand_over_lost(sbase, c0, wait_ns))) {
+                set_block_lost(sbase);
                 break;
             }
-            if (!tagged(ml, tag))
+            if (!tagged(ml, ptag))
                 ml = ld_pairs2_gpu(src_ml);
 #pragma unroll
             for (int z = 0; z < kAttSlots - 1; ++z)
-                if (z < others && __float_as_int(o[z].y) != tag)
+                if (z < others && __float_as_int(o[z].y) != ptag)
                     o[z] = ld_pair_gpu(src + (int64_t)z * (head + 2));
         }
         const float gm = fmaxf(M, warp_max(ml.x));
@@ -1027,7 +1056,6 @@ __device__ __forceinline__ void consume_attention(const FusedParams &P, int tag,
 
 struct Epilogue {
     int rb, rround;
-    bool lost, lost_before;
 };
 
 // Results leave as (value, tag) pairs, one store each, which the readers poll: no fence, no counter and no second trip to the
@@ -1077,7 +1105,7 @@ __device__ __forceinline__ void epilogue_phase(const FusedParams &P, const MvPar
             }
             if (i0 == 0) {
                 if (!mbar_wait_bounded(sbase + kFBarRedFull + 8 * es.rb, (uint32_t)es.rround & 1u, wait_ns))
-                    es.lost = true;
+                    set_block_lost(sbase);
             }
             if (!mine)
                 continue;
@@ -1118,11 +1146,10 @@ __device__ __forceinline__ void epilogue_phase(const FusedParams &P, const MvPar
             } else {   // EPI_RESIDUAL
                 if (resid && __float_as_int(old.y) != resid_tag) {
                     const long long c0 = sm_clock();
-                    const long long limit = (long long)(2 * (es.lost ? kFShortWaitNs : wait_ns));
                     do {
                         old = ld_pair_gpu(resid + row);
-                        if (sm_clock() - c0 > limit) {
-                            es.lost = true;
+                        if (hand_over_lost(sbase, c0, wait_ns)) {
+                            set_block_lost(sbase);
                             break;
                         }
                     } while (__float_as_int(old.y) != resid_tag);
@@ -1166,6 +1193,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
         mbar_init(sbase + kFBarRedFull + 8 * tid, kFusedConsWarps);
         mbar_init(sbase + kFBarRedEmpty + 8 * tid, 1);
     }
+    if (tid == 0)
+        *reinterpret_cast<volatile int *>(smem + kFLost) = 0;
     if (tid < 32)
         mbar_fence_init();
     __syncthreads();
@@ -1182,7 +1211,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
         pr.vhead = 0;
         pr.ring_bytes = P.ring_bytes;
         pr.seq = pr.tail = pr.vtail = 0;
-        pr.lost = false;
         pr.wait_ns = wait_ns;
         const uint64_t pol = policy_evict_first();
         pr.pos = -1;
@@ -1215,7 +1243,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
         // consumers have waited for every stage, so these waits return at once unless a wait ran out before.
         for (int d = max(pr.tail, pr.seq - kFDesc); d < pr.seq; ++d)
             mbar_wait_bounded(sbase + kFBarFull + 8 * (d % kFDesc), (uint32_t)(d / kFDesc) & 1u, wait_ns);
-        if (pr.lost && lane == 0)
+        __syncwarp(0xfu);
+        if (lane == 0 && block_lost(sbase))
             atomicOr(&P.state->status, L2J_DS_WAIT_TIMEOUT);
         return;
     }
@@ -1226,13 +1255,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
     const AttSplit as = att_split(P, pos, G);
     const unsigned int epoch = __ldcg(P.epoch);
     const int tag0 = (int)(epoch * (unsigned int)P.n_layers) + 1;    // tag of layer l: tag0 + l
-    const bool lost_at_entry = (__ldcg(&P.state->status) & L2J_DS_WAIT_TIMEOUT) != 0;
+    *reinterpret_cast<volatile int *>(smem + kFLate) = (int)__ldcg(P.epoch + 1);    // the same from every thread
+    if ((__ldcg(&P.state->status) & L2J_DS_WAIT_TIMEOUT) != 0)
+        set_block_lost(sbase);
 
     // ------------------------------------------------------------------------------ epilogue warp
     if (warp == kFusedConsWarps + 1) {
         Epilogue es;
         es.rb = es.rround = 0;
-        es.lost = es.lost_before = lost_at_entry;
         // Every forward before this one has bumped the last phase's counter once per block.  If one is missing, the blocks of the
         // context (or its host) have lost count: reported here too, because a stage of a layer split has no classifier that waits.
         if (b == 0 && lane == 0 && ld_acquire_u32(P.sync + (int64_t)kSyncStride * (5 * P.n_layers - 1)) != (epoch - 1u) * (unsigned int)G)
@@ -1258,9 +1288,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
                 const int tag = tag0 + layer;
                 float2 *out = k == 0 ? P.q_pairs : (k == 1 ? P.xa_pairs : (k == 2 ? P.h_pairs : P.xb_pairs));
                 const float2 *resid = k == 1 ? (layer > 0 ? P.xb_pairs : nullptr) : P.xa_pairs;
-                epilogue_phase(P, p, layer, first, nmine, pos, smem, sbase, es, wait_ns, out, tag, resid, k == 1 ? tag - 1 : tag,
-                               layer + 1 == P.n_layers);
-                if (k == 3 && layer + 1 == P.n_layers) {
+                const bool last = layer + 1 == P.n_layers;
+                int rtag = k == 1 ? tag - 1 : tag;
+                if (k == 3 && last && lane > 0)
+                    rtag = reader_tag(sbase, rtag, L2J_LATE_RESIDUAL);
+                epilogue_phase(P, p, layer, first, nmine, pos, smem, sbase, es, wait_ns, out, tag, resid, rtag, last);
+                if (k == 3 && last) {
                     // the classifier kernel behind polls this counter: every result of the block in this phase was written by
                     // this warp, the release is cumulative
                     __syncwarp();
@@ -1271,7 +1304,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
                     fused_trace(P, layer * 5 + (k == 0 ? 0 : k + 1), 3);
             }
         }
-        if (es.lost && !es.lost_before && lane == 0)
+        __syncwarp();
+        if (lane == 0 && block_lost(sbase))
             atomicOr(&P.state->status, L2J_DS_WAIT_TIMEOUT);
         return;
     }
@@ -1280,7 +1314,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
     Consumer cs;
     cs.seq = 0;
     cs.rb = cs.rround = 0;
-    cs.lost = cs.lost_before = lost_at_entry;
     int rot = 0;
     for (int layer = 0; layer < P.n_layers; ++layer) {
 #pragma unroll 1
@@ -1297,7 +1330,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
                 const float *rms_w = p.rms_w ? p.rms_w + (int64_t)layer * P.rms_step : nullptr;
                 // the first phase's input came from the kernel in front
                 const float2 *in = k == 0 ? (layer > 0 ? P.xb_pairs : nullptr) : (k == 1 ? P.o_pairs : (k == 2 ? P.xa_pairs : P.h_pairs));
-                consume_ring_phase(P, p, nmine, in, k == 0 ? tag0 + layer - 1 : tag0 + layer, rms_w, smem, sbase, cs, wait_ns, pidx);
+                const int tag = k == 0 ? tag0 + layer - 1 : tag0 + layer;
+                consume_ring_phase(P, p, nmine, in, reader_tag(sbase, tag, L2J_LATE_INPUT), rms_w, smem, sbase, cs, wait_ns, pidx);
             }
             if (k == 0) {
                 // attention over positions 0..pos (Run.java:450-478)
@@ -1314,7 +1348,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
             }
         }
     }
-    if (cs.lost && !cs.lost_before && lane == 0)
+    __syncwarp();
+    if (lane == 0 && block_lost(sbase))
         atomicOr(&P.state->status, L2J_DS_WAIT_TIMEOUT);
 }
 

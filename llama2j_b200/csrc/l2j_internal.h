@@ -223,7 +223,7 @@ struct FusedParams {
     int xarea_bytes;           // shared memory between the fixed header and the ring: limbs of the input vector / merge area
     int ring_bytes;            // bytes of the ring
     unsigned int *sync;        // hand-over counters, kSyncStride words apart, five per layer, as the per-step kernels have them: the last one is used
-    const unsigned int *epoch; // forwards started on this context
+    const unsigned int *epoch; // forwards started on this context; behind it the L2J_LATE_* bits
     SeqState *state;
     int timeout_us;
     unsigned long long *trace; // optional: [block][5 * n_layers][8] global-timer marks, else nullptr

@@ -15,6 +15,7 @@ E_INVALID, E_CUDA, E_STATE, E_DEVICE, E_NOMEM = -1, -2, -3, -4, -5
 DS_WAIT_TIMEOUT, DS_BAD_POS, DS_BAD_TOKEN, DS_BAD_LINK = 0x1, 0x2, 0x4, 0x8
 F_NO_GRAPH, F_NO_PDL, F_SIMPLE, F_STEP_KERNELS, F_TP_SPLIT_CLASSIFIER, F_PERSISTENT = 0x1, 0x2, 0x4, 0x8, 0x10, 0x20
 F_NO_TENSOR_PREFILL = 0x40
+LATE_INPUT, LATE_ROWS, LATE_PARTIALS, LATE_RESIDUAL = 0x1, 0x2, 0x4, 0x8
 QUANT_GROUP, QUANT_GROUP_BYTES = 256, 264
 
 (T_TOKEN_EMBEDDING, T_RMS_ATT, T_WQ, T_WK, T_WV, T_WO, T_RMS_FFN, T_W1, T_W2, T_W3, T_RMS_FINAL, T_WCLS) = range(12)
@@ -79,6 +80,7 @@ _SIGNATURES = {
     "l2j_pipeline_reset": (C.c_int, [C.POINTER(_P), C.c_int]),
     "l2j_set_wait_limit_us": (C.c_int, [_P, C.c_int]),
     "l2j_debug_desync": (C.c_int, [_P]),
+    "l2j_debug_late": (C.c_int, [_P, C.c_int]),
     "l2j_debug_fail_alloc": (C.c_int, [_P, C.c_int]),
     "l2j_get_stats": (C.c_int, [_P, C.POINTER(Stats)]),
     "l2j_launch_mode": (C.c_int, [_P]),

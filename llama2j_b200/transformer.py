@@ -227,6 +227,10 @@ class Transformer:
         """Host-side failure injection: the next forward waits for hand-overs that never come."""
         _lib.check(self._lib.l2j_debug_desync(self._ctx), self._ctx)
 
+    def debug_late(self, readers: int) -> None:
+        """The readers named by the LATE_* bits wait for pairs that nobody writes (failure injection; ends with reset)."""
+        _lib.check(self._lib.l2j_debug_late(self._ctx, readers), self._ctx)
+
     def debug_fail_alloc(self, nth: int) -> None:
         """Host-side failure injection: the nth allocation from now on fails (0: none)."""
         _lib.check(self._lib.l2j_debug_fail_alloc(self._ctx, int(nth)), self._ctx)

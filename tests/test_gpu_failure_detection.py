@@ -56,6 +56,41 @@ def test_wait_runs_out_is_reported_and_reset_recovers(flags, kernels):
     m.close()
 
 
+@pytest.mark.parametrize("readers", [L.LATE_INPUT, L.LATE_ROWS, L.LATE_PARTIALS, L.LATE_RESIDUAL])
+def test_pairs_that_never_come(readers):
+    """Every kind of wait between the blocks of the persistent kernel runs out: reported, also by lanes that are not a warp's first
+    and without a classifier behind (a stage of a layer split), once per block and not once per wait."""
+    limit = 20000
+    cfg = ModelConfig(dim=512, hidden_dim=1536, n_layers=4, n_heads=8, n_kv_heads=8, vocab_size=512, seq_len=256, shared_classifier=False)
+    m = _build(cfg, syn.synthetic_tensors(cfg, 2), L.F_PERSISTENT, 0, 2, limit_us=limit)
+    pos = 200                                                   # seven units of 32 positions per head on three blocks
+    good = m.forward_stage(5, pos).copy()
+    m.debug_late(readers)
+    t0 = time.perf_counter()
+    with pytest.raises(L.L2jError) as e:
+        m.forward_stage(5, pos)
+    # at least the limit; a block that has lost one wait gives up the others after 2 us (three layers have sixteen waits in a row)
+    assert 1e-6 * limit <= time.perf_counter() - t0 < 4e-6 * limit
+    assert e.value.code == L.E_DEVICE
+    assert m.stats().device_status == L.DS_WAIT_TIMEOUT
+    m.reset()
+    assert np.array_equal(m.forward_stage(5, pos).view(np.uint32), good.view(np.uint32))
+    assert m.stats().device_status == 0
+    with pytest.raises(L.L2jError) as e:
+        m.debug_late(16)
+    assert e.value.code == L.E_INVALID
+    m.close()
+
+
+def test_late_pairs_need_the_persistent_kernel():
+    cfg = ModelConfig(dim=256, hidden_dim=512, n_layers=1, n_heads=4, n_kv_heads=4, vocab_size=256, seq_len=16, shared_classifier=True)
+    m = _build(cfg, syn.synthetic_tensors(cfg, 1), L.F_STEP_KERNELS)
+    with pytest.raises(L.L2jError) as e:
+        m.debug_late(L.LATE_INPUT)
+    assert e.value.code == L.E_STATE
+    m.close()
+
+
 def test_wait_limit_is_fixed_at_finalize():
     cfg = ModelConfig(dim=256, hidden_dim=512, n_layers=1, n_heads=4, n_kv_heads=4, vocab_size=256, seq_len=16,
                       shared_classifier=True)
