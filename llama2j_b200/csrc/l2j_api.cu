@@ -268,7 +268,7 @@ void fill_plan(MvParams &p, const MvPlan &pl)
         p.total_stages = 0;
         const int nseg = p.paired ? 1 : p.nseg;
         for (int i = 0; i < 3; ++i) {
-            p.seg_stages[i] = i < nseg ? (p.seg[i].rows + rs - 1) / rs : 0;
+            p.seg_stages[i] = i < nseg && rs > 0 ? (p.seg[i].rows + rs - 1) / rs : 0;   // no plan: the plain kernels have no stages
             p.total_stages += p.seg_stages[i];
         }
     }

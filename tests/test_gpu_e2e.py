@@ -288,3 +288,12 @@ def test_cli_run_loop_with_checkpoint_and_quant_cache(oracle, tmp_path, monkeypa
     assert second[1] == first[1]
     with pytest.raises(SystemExit):
         cli.main(["--checkpoint", "tiny.bin", "--mode", "CPU"])
+
+
+@pytest.mark.parametrize("dim,hidden,heads,kv", [(72, 200, 6, 3), (9472, 512, 74, 2)])
+def test_shapes_without_ring_kernels(oracle, dim, hidden, heads, kv):
+    """Rows that are no multiple of 16, and rows too long for the classifier's ring kernel: the plain kernels run, which have no stages."""
+    cfg = ModelConfig(dim=dim, hidden_dim=hidden, n_layers=2, n_heads=heads, n_kv_heads=kv, vocab_size=300, seq_len=16, shared_classifier=True)
+    _, worst, _, mode, _ = _compare_run(oracle, cfg, syn.synthetic_tensors(cfg, 0), syn.synthetic_prompt(4, 1, 300), 8)
+    assert not mode["ring"] and not mode["persistent"]
+    assert worst < TOL, worst
