@@ -1,8 +1,9 @@
 """The prompt matrices for few tokens (blocks of 16, 32 and 48 instead of 64) at both sides of every block's end.
 
-The integer sums and the order in which a row's groups are added do not depend on the block a token travels in, so the K/V rows of a
-one-layer model are the same bits as in a block of 64.  With more layers the number of key ranges in the attention depends on the
-length, hence the tolerance of the prompt path (1e-4 of the logit range, tests/test_gpu_prefill.py)."""
+The integer sums, the parts a row's groups are dealt into and the order in which they are added do not depend on the block a token
+travels in, and 64 positions are one key range of the attention, so the K/V rows of both layers of a two-layer model are the
+same bits as in a block of 64: those of the second layer have passed all four matrices of the first.  Against the decode step the
+tolerance is that of the prompt path (1e-4 of the logit range, tests/test_gpu_prefill.py)."""
 import numpy as np
 import pytest
 
@@ -29,18 +30,24 @@ def _config(layers):
 
 
 def test_rows_are_those_of_a_full_block():
-    cfg = _config(1)
+    cfg = _config(2)
     tensors = syn.synthetic_tensors(cfg, 4)
-    toks = np.random.default_rng(5).integers(3, cfg.vocab_size, 64).astype(np.int32)
+    rng = np.random.default_rng(5)
+    toks, other = (rng.integers(3, cfg.vocab_size, 64).astype(np.int32) for _ in range(2))
     m = _build(cfg, tensors)
+
+    def rows():
+        return np.array([[m.read_buffer(w, cfg.kv_dim, layer, p) for layer in range(2) for w in (5, 6)] for p in range(64)])
+
     m.prefill(toks, 0)
-    want = [[m.read_buffer(w, cfg.kv_dim, 0, p).copy() for w in (5, 6)] for p in range(64)]
+    want = rows()
     for n in COUNTS:
-        m.reset()
-        m.prefill(toks[64 - n:], 64 - n)          # the last n positions again, in a block of their own
-        for p in range(64 - n, 64):
-            for w in (5, 6):
-                assert np.array_equal(m.read_buffer(w, cfg.kv_dim, 0, p), want[p][w - 5]), (n, p, w)
+        m.prefill(other, 0)                       # every row is another one before it is written again
+        before = rows()
+        assert all(not np.array_equal(before[p], want[p]) for p in range(64))
+        m.prefill(toks[:64 - n], 0)
+        m.prefill(toks[64 - n:], 64 - n)
+        assert np.array_equal(rows(), want), n
     assert m.stats().device_status == 0
     m.close()
 
