@@ -280,7 +280,7 @@ __device__ __forceinline__ void fused_trace(const FusedParams &P, int phase_inde
 struct Producer {
     uint8_t *smem;
     uint32_t sbase, ring_base;
-    int vhead;              // bytes handed out so far; < 2^31 per token and block
+    int vhead;              // bytes handed out since the last rebase()
     int off;                // vhead's position in the ring
     int ring_bytes;
     int seq, tail;          // descriptors issued / known to be released
@@ -314,7 +314,22 @@ struct Producer {
         off += step;
         return at;
     }
+
+    // Counts from the oldest stage in flight on.  Grouped heads that share a long cache take a block's ring through more than 2^31
+    // bytes in one token.  (48 forwards of 7B: 68.8 ms without it, 69.05 with it, 69.4 with a difference modulo 2^32 in acquire().)
+    __device__ __forceinline__ void rebase(int lane)
+    {
+        int *vstart = reinterpret_cast<int *>(smem + kFVStart);
+        const int base = tail < seq ? vtail : vhead;
+        __syncwarp(0xfu);
+        for (int i = tail + lane; i < seq; i += 4)
+            vstart[i % kFDesc] -= base;
+        __syncwarp(0xfu);
+        vhead -= base;
+        vtail = 0;
+    }
 };
+constexpr int kFRebase = 1 << 30;       // (a phase's matrix rows or a unit of the attention step add far less than as much again)
 
 __device__ __forceinline__ void producer_learn_pos(Producer &pr, const FusedParams &P, int grid)
 {
@@ -1223,6 +1238,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
                 const MvParams &p = P.mv[k];
                 const int S = p.total_stages;
                 if (!(P.debug_no_copy & 8) && lane == 0) fused_trace(P, layer * 5 + (k == 0 ? 0 : k + 1), 5);
+                if (pr.vhead > kFRebase)
+                    pr.rebase(lane);
                 produce_phase(pr, P, p, k, layer, first_stage_of(b, rot, G), G, pol, lane);
                 if (!(P.debug_no_copy & 8) && lane == 0) fused_trace(P, layer * 5 + (k == 0 ? 0 : k + 1), 6);
                 rot = (rot + S) % G;
@@ -1232,6 +1249,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
                         const int u0 = att_first_unit(pr.as, b), u1 = att_first_unit(pr.as, b + 1);
                         if (lane == 0) fused_trace(P, layer * 5 + 1, 5);
                         for (int u = u0; u < u1; ++u) {
+                            if (pr.vhead > kFRebase)
+                                pr.rebase(lane);
                             produce_att_stage(pr, P, layer, u, pr.as, pr.pos, lane);
                         }
                         if (lane == 0) fused_trace(P, layer * 5 + 1, 6);

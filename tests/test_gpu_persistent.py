@@ -154,3 +154,34 @@ def test_contexts_that_work_at_the_same_time():
     for m in models:
         assert m.stats().device_status == 0
         m.close()
+
+
+def test_more_bytes_per_token_than_31_bits_count():
+    """Heads that share one K/V head read a long cache 32 times over: a block's ring takes more than 2^31 bytes in one token.  The keys
+    and values of the last positions differ from zero; the bound is the prompt path's (305,000 FP32 terms per softmax sum)."""
+    last = 305_000
+    cfg = ModelConfig(dim=4096, hidden_dim=256, n_layers=32, n_heads=32, n_kv_heads=1, vocab_size=300, seq_len=last + 8, shared_classifier=True)
+    assert cfg.n_layers * cfg.n_heads * last * 128 * 8 > 148 << 31
+    rng = np.random.default_rng(13)
+    data = {t: syn.synth_quant(cfg.tensor_floats(t) // cfg.n_layers, 14, t) for t in (L.T_WQ, L.T_WK, L.T_WV, L.T_WO, L.T_W1, L.T_W2, L.T_W3)}
+    emb = syn.synth_f32(cfg.tensor_floats(L.T_TOKEN_EMBEDDING), 14, L.T_TOKEN_EMBEDDING)
+    k, v = (rng.normal(0, s, (500, cfg.kv_dim)).astype(np.float32) for s in (1.0, 30.0))
+    logits = []
+    for flags in (L.F_STEP_KERNELS, 0):
+        m = Transformer(cfg, 0, 0, None, flags)
+        assert m.launch_mode()["persistent"] == (flags == 0)
+        for t in L.QUANT_TENSORS:
+            n = cfg.tensor_floats(t)
+            if t not in data:
+                m.upload_quant(t, syn.quant_encode(np.ones(n, dtype=np.float32)))
+                continue
+            for layer in range(cfg.n_layers):
+                m.upload_quant(t, data[t], n // cfg.n_layers, layer * (n // cfg.n_layers))
+        m.upload_f32(L.T_TOKEN_EMBEDDING, emb)
+        m.finalize()
+        for layer in range(cfg.n_layers):
+            m.kv_write(layer, last - 500, k, v)
+        logits.append(np.array([m.forward(7, last + i)[0].copy() for i in range(2)]))
+        assert m.stats().device_status == 0
+        m.close()
+    assert float(np.abs(logits[0] - logits[1]).max()) <= 1e-4 * float(logits[0].max() - logits[0].min())
