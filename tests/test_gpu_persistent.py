@@ -1,6 +1,7 @@
-"""The persistent kernel at the edges of its mapping, against the per-step kernels.
+"""The persistent kernel at the edges of its mapping, against the per-step kernels and a float64 model; when it is chosen; and
+what it does beside other contexts.
 
-Both form the same products from the same 24-bit activations and add the FP32 group terms of a row in other orders; a row of g groups
+Both kernels form the same products from the same 24-bit activations and add the FP32 group terms of a row in other orders; a row of g groups
 is then off by at most about g roundings of 2^-24 of its terms, and two layers of them move a logit by a few 1e-6 of the range
 (observed: 1e-6).  The bound is 1e-5."""
 import threading
@@ -12,6 +13,7 @@ from llama2j_b200 import lib as L
 from llama2j_b200 import synthetic as syn
 from llama2j_b200.model_files import ModelConfig
 from llama2j_b200.transformer import Transformer
+from tests.np_model import NumpyModel
 
 pytestmark = pytest.mark.gpu
 
@@ -56,6 +58,19 @@ def test_against_step_kernels(dim, hidden, heads, kv):
     assert a.stats().device_status == 0
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("dim,hidden,heads,kv", SHAPES[:4])
+def test_against_float64(dim, hidden, heads, kv):
+    """Every position of two attention units and a bit.  An activation is held to 2^-23 of its group's largest element and a row sum
+    adds some ten FP32 terms: a few 1e-7 of the range per matrix, eight of them in a row."""
+    cfg = ModelConfig(dim=dim, hidden_dim=hidden, n_layers=2, n_heads=heads, n_kv_heads=kv, vocab_size=500, seq_len=70, shared_classifier=True)
+    tensors = syn.synthetic_tensors(cfg, 15)
+    m, ref = _build(cfg, tensors, L.F_PERSISTENT), NumpyModel(cfg, tensors)
+    for p, tok in enumerate(syn.synthetic_prompt(70, 16, cfg.vocab_size)):
+        x, y = m.forward(int(tok), p)[0], ref.forward(int(tok), p)
+        assert float(np.abs(x - y).max()) <= TOL * float(y.max() - y.min()), p
+    m.close()
 
 
 @pytest.mark.parametrize("value", [1e-30, 3e37, np.inf, np.nan])
