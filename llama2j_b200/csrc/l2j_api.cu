@@ -372,7 +372,7 @@ void link_ranks(l2j_ctx *c)
 }
 
 // Stage geometry of a phase of the persistent kernel: `sets` of wpr warps work on two rows each (paired: a row of either
-// matrix), a warp spans four quantisation groups.  Stages of 22 to 36 KB at most: the phases share one byte ring, and small
+// matrix), a warp spans four quantisation groups.  Stages of 29 KB at most: the phases share one byte ring, and small
 // stages keep more of it in flight and waste less where it wraps; a matrix that would not give every block a stage gets
 // smaller ones.
 MvPlan plan_fused_phase(int n, bool paired, int rows, int blocks)

@@ -21,19 +21,14 @@
 // are dealt in contiguous runs; a block folds the units of one head into one partial (m, l, o), and the block with the
 // head's first positions merges the few partials of the head (at most kAttSlots) in a fixed order.
 //
-// What bounds it (7B shape, position 160): a layer takes 45 us where its bytes take 31.5 at the measured copy rate.  The
+// What bounds it (7B shape, position 160): a layer takes 44 us where its bytes take 31.5 at the measured copy rate.  The
 // ring holds 4.4 us of a block's share of the HBM; a boundary between two phases costs 2 to 3 us from the median block's last
-// result to the next block's first dot product, and the attention step and Wo, which hardly stream, 11 us together.  Measured on the
-// way from 56.6 us per layer (in-kernel timeline, both sides with it on):
-//   - the producer's pass per stage took 900 cycles, whatever a stage held, and bounded the consumers: set up per phase and segment now;
-//   - a warp works on two rows with half as many elements each: 24 instead of 48 registers of limbs, so that the next stage's bytes are
-//     fetched while the dot products of this one run (750 -> about 500 cycles per 25 KB; 288 are the dp4a's);
-//   - pairs instead of a fence, a counter and a second load per hand-over; exchanges instead of stores (see st_pair_gpu);
-//   - the Wo phase's prologue merged the attention partials in every block (5 us); one block per head does it now, in 1.5.
-// Taken back: FP32 multiply-adds on unpacked bytes (a permute per byte: slower than three dp4a per four), asking the stages
-// behind the ring into the L2 (50 us: the extra requests delay the hand-overs), the same for RMSNorm weights and output lines.
-// 7B shape, 48 greedy forwards from position 0: 88.6 -> 69.4 to 72.4 ms; 8 steps behind 3840 positions: 22.4 -> 17.8 to 18.5 ms; 13B shape, 24
-// forwards (from the per-step kernels): 70.2 -> 63.0 to 65.9 ms (by machine and allocation).
+// result to the next block's first dot product, and the attention step and Wo, which hardly stream, 11 us together.  Two rows per warp
+// with half as many elements each leave registers to fetch the next stage's bytes while the dot products of this one run; 14
+// consumer warps because more than 16 warps would have fewer than 128 registers and spill, which costs more than it saves here.
+// Against counters between the blocks, 18 warps with a row each and a merge of the attention partials in every block: 48 greedy
+// forwards of 7B 88.6 -> 69 to 72 ms (by machine), 8 steps behind 3840 positions 22.4 -> 17.7 to 18.5; 24 forwards of 13B, per-step
+// kernels before, 70.2 -> 62.7 to 65.9.
 //
 // Blocks wait for each other, so all of them must be resident: the grid is one block per SM and the launch is
 // cooperative.  Every wait is bounded by the SM's cycle counter.  A hand-over between blocks that runs out raises
@@ -132,8 +127,8 @@ __device__ __forceinline__ float2 ld_pair_gpu(const float2 *p)
     return v;
 }
 
-// An exchange and not a store: while the SM streams, a plain store may stay in it for 4 us before the L2 gets it (7B shape,
-// W2 -> QKV: the input vector is complete 3.7 instead of 6.5 us after the median block's last store); an atomic goes at once.
+// An exchange and not a store: a plain store waits in the SM behind the stream, an atomic goes at once (7B shape, W2 -> QKV: the
+// input vector is complete 3.7 instead of 6.5 us after the median block's last result).
 __device__ __forceinline__ void st_pair_gpu(float2 *p, float v, int tag)
 {
     unsigned long long old;
