@@ -311,7 +311,8 @@ struct Producer {
     }
 
     // Counts from the oldest stage in flight on.  Grouped heads that share a long cache take a block's ring through more than 2^31
-    // bytes in one token.  (48 forwards of 7B: 68.8 ms without it, 69.05 with it, 69.4 with a difference modulo 2^32 in acquire().)
+    // bytes in one token.  (48 forwards of 7B: 68.65 ms without it, 68.90 with it; with a
+    // difference modulo 2^32 in acquire() 0.5 ms more than without.)
     __device__ __forceinline__ void rebase(int lane)
     {
         int *vstart = reinterpret_cast<int *>(smem + kFVStart);
@@ -324,7 +325,7 @@ struct Producer {
         vtail = 0;
     }
 };
-constexpr int kFRebase = 1 << 30;       // (a phase's matrix rows or a unit of the attention step add far less than as much again)
+constexpr int kFRebase = 1 << 30;       // looked at once per layer and attention unit: neither adds as much again
 
 __device__ __forceinline__ void producer_learn_pos(Producer &pr, const FusedParams &P, int grid)
 {
@@ -1228,13 +1229,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_layers_kernel(const __
         pr.off = 0;
         int rot = 0;
         for (int layer = 0; layer < P.n_layers; ++layer) {
+            if (pr.vhead > kFRebase)
+                pr.rebase(lane);
 #pragma unroll 1
             for (int k = 0; k < 4; ++k) {
                 const MvParams &p = P.mv[k];
                 const int S = p.total_stages;
                 if (!(P.debug_no_copy & 8) && lane == 0) fused_trace(P, layer * 5 + (k == 0 ? 0 : k + 1), 5);
-                if (pr.vhead > kFRebase)
-                    pr.rebase(lane);
                 produce_phase(pr, P, p, k, layer, first_stage_of(b, rot, G), G, pol, lane);
                 if (!(P.debug_no_copy & 8) && lane == 0) fused_trace(P, layer * 5 + (k == 0 ? 0 : k + 1), 6);
                 rot = (rot + S) % G;
