@@ -41,7 +41,7 @@ FALLBACK_HBM_GBS = 6650.0
 # ncu on the same shape with 4 layers (a full-metric capture of 32 layers would hold too much on the device)
 # and scaled by the layer count: the traffic of a launch is the layers' weights, in proportion.  None for
 # other shapes.
-NCU_TRAFFIC_BYTES_PER_LAYER = {"llama2-7b": (835265280 + 23664640) // 4}
+NCU_TRAFFIC_BYTES_PER_LAYER = {"llama2-7b": (856627712 + 3174912) // 4}
 
 
 def bytes_per_token(cfg, pos: int) -> dict:

@@ -1,8 +1,9 @@
 """Failure detection without a GPU fault: a device-side wait that runs out is reported, not hung on.
 
-The failure is injected on the host (l2j_debug_desync advances the context's forward counter as if a
-partner had run a forward that this context missed), so the hand-over counters of the next forward never
-reach their targets.  Every wait in the kernels is bounded: the forward ends by its limit, the call
+The failure is injected on the host.  l2j_debug_desync advances the context's forward counter as if a
+partner had run a forward that this context missed, so the hand-over counters of the next forward never
+reach their targets; the persistent kernel, whose pairs carry tags of that counter and still arrive, compares it with
+its blocks' bumps.  l2j_debug_late makes the readers of those pairs wait for tags that nobody writes.  Every wait in the kernels is bounded: the forward ends by its limit, the call
 returns L2J_E_DEVICE with L2J_DS_WAIT_TIMEOUT in the status word, the status stays raised until
 l2j_reset, and after the reset the context computes the same logits as before.  The reference has no
 counterpart beyond the exception of ContextCUDA.java:296-304."""
