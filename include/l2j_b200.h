@@ -324,8 +324,8 @@ L2J_API int l2j_last_generate_us(l2j_ctx *ctx, double *total_us);
  * classifier+argmax.  Leaves the sequence state undefined: call l2j_reset afterwards. */
 L2J_API int l2j_time_kernels(l2j_ctx *ctx, int pos, int reps, double *us);
 
-/* The same for the persistent kernel that runs all layers of a token in one launch (contexts created
- * without L2J_F_STEP_KERNELS whose matrices have rows of whole quantisation groups): average device time
+/* The same for the persistent kernel that runs all layers of a token in one launch (contexts that run
+ * it: bit 3 of l2j_launch_mode; else L2J_E_STATE): average device time
  * of one launch at position `pos`, CUDA events on the context's stream around the launch alone, each
  * launch after an embedding gather of its own.  Leaves the sequence state undefined: call l2j_reset. */
 L2J_API int l2j_time_layers_kernel(l2j_ctx *ctx, int pos, int reps, double *us_per_launch);
